@@ -45,9 +45,19 @@ cudaError_t launch_momentum(int, const T*, const T*, int, int, double, double, d
 template <typename T>
 cudaError_t launch_measure_static(int, int, int, const T*, const uint8_t*, double*, cudaStream_t);
 template <typename T, typename S>
-cudaError_t launch_phi_batch(const void*, const unsigned short*, int, cudaStream_t);
+cudaError_t launch_phi_batch(const void*, const unsigned short*, int, int, cudaStream_t);
 template <typename T, typename S>
-cudaError_t launch_update_batch(const void*, const unsigned short*, int, bool, cudaStream_t, bool, int);
+cudaError_t launch_update_batch(const void*, const unsigned short*, int, bool, bool, cudaStream_t, int);
+template <typename T, typename S>
+cudaError_t launch_phi_one(const void*, cudaStream_t);
+template <typename T, typename S>
+cudaError_t launch_update_one(const void*, bool, bool, cudaStream_t, bool, int);
+template <typename T, typename S>
+cudaError_t launch_phis_batch(const void*, const unsigned short*, int, cudaStream_t);
+template <typename T, typename S>
+cudaError_t launch_phis_one(const void*, cudaStream_t);
+template <typename T, typename S>
+cudaError_t launch_expand(const Consts<T>&, const State<T, S>&, cudaStream_t);
 template <typename T, typename S>
 cudaError_t launch_mu(const Consts<T>&, const State<T, S>&, cudaStream_t);
 template <typename T, typename S>
@@ -78,7 +88,7 @@ cudaError_t launch_geometry(int, int, int, const uint8_t*, const void*, int, boo
 template <typename T, typename S>
 size_t case_desc_bytes();
 template <typename T, typename S>
-void fill_case_desc(void*, const Consts<T>&, const State<T, S>&, int, int, int, int);
+void fill_case_desc(void*, const Consts<T>&, const State<T, S>&, int, int, int, int, int, const PhiTile&);
 }  // namespace lbm
 
 using namespace lbm;
@@ -104,6 +114,7 @@ static int fail(int code, const std::string& msg) {
       return fail(LBM_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));       \
   } while (0)
 
+constexpr size_t kDescBytes = 4096;  // room for one case descriptor in host memory
 constexpr int kMeasureBlocks = 1024;
 constexpr int kMeasVals = 11;
 
@@ -146,6 +157,8 @@ struct LbmHandle {
   int pc = 0;             // phi buffer holding the latest recovered phi
   bool raw = true;        // current state is the reference state itself (after init)
   bool first = true;      // phi*u of the previous step does not exist yet
+  PhiTile tile{};         // work split of the source form's phi pass (phis_tile of the grid alone)
+  bool sform = false;     // f[cur] holds S (three T per node) instead of the populations (lbm_phis.cuh)
   int c_last = 0;         // cbuf slot of the last step's correction
   int64_t steps = 0;
   bool last_raw_in = true;  // mode of the last step's input (for P read-out)
@@ -156,7 +169,10 @@ struct LbmHandle {
   bool desc_ok = false;
   int desc_cur0 = 0;        // cur when the descriptors were filled (parity 0)
   int phi_per_thread = 16;  // nodes per thread of the phi kernel
-  int upd_block = kBlock;   // threads per block of the (linear-layout) update kernel: 128 or 256
+  // threads per block of the (linear-layout) update kernel: 128 or 256 (the gradient-of-mu modes).  A
+  // block's slot is free again when its last warp is done: 108.8 us per launch at 256, 105.4 at 128 on
+  // the 150x150x107 case (half storage, 384x384x256: 1346 and 1230 us).
+  int upd_block = 128;
 };
 
 namespace {
@@ -201,6 +217,12 @@ Consts<T> make_consts(const LbmHandle& h, const float* ww_lut) {
   k.rho_floor = (T)(0.5 * p.rho_l);
   k.drho = (T)(p.rho_l - p.rho_g);
   k.visc = (T)((0.5 - p.tau_g) / p.tau_g);
+  k.inv_floor = (T)1 / k.rho_floor;
+  k.inv_floor_cs2 = (T)1 / (k.rho_floor * k.cs2);
+  k.drho_cs2 = (T)((p.rho_l - p.rho_g) * cs2);
+  k.visc_drho = (T)((0.5 - p.tau_g) / p.tau_g * (p.rho_l - p.rho_g));
+  k.sharp = (T)(4.0 * cs2 * p.ac_scale / p.xi);
+  k.src_c = (T)(ac_coeff / cs2);
   k.omega_f = (T)(1.0 / tau_f);
   k.omega_g = (T)1 / (T)p.tau_l;
   k.tau_l = (T)p.tau_l;
@@ -560,28 +582,62 @@ bool omega1_of(const LbmHandle* h) {
 // (Pairs of nodes in the paired layout.)
 int64_t units_of(const LbmHandle* h) { return h->paired ? h->N / 2 : h->N; }
 // per_thread counts nodes (a thread of the paired kernel takes per_thread / 2 pairs).
-int phi_blocks_of(const LbmHandle* h, int per_thread) {
+// A grid alone that would not fill the device (608 resident blocks) at that many takes fewer.
+int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
+  if (alone) per_thread = (int)std::max<int64_t>(1, std::min<int64_t>(per_thread, (h->N + 608 * kBlock - 1) / (608 * kBlock)));
   const long long per = (long long)kBlock * (h->paired ? std::max(1, per_thread / 2) : per_thread);
   return (int)std::max<long long>(1, (units_of(h) + per - 1) / per);
 }
+
+// Whether the two-kernel step of a grid leaves f in source form: tau_f == 1, float
+// compute, linear layout.  (float64 keeps the populations: its step is bound by
+// the float64 pipe, and the source form evaluates f again on each tile's halo.)
+bool wants_s(const LbmHandle* h) { return h->prec != LBM_F64 && h->nz > 1 && !h->paired && omega1_of(h); }
+
+// Tiles of the source form's phi pass: the (y, z) split whose blocks (tile plus
+// halo within kPhisThreads nodes) waste the fewest threads, then the planes of
+// x per block (an even number: they are walked in pairs, two more at the ends)
+// that keep the device's slots busy for the shortest time, `share` cases
+// launched together sharing them.
+constexpr int kPhisThreads = 320, kPhisSlots = 304;  // two blocks per SM
+PhiTile phis_tile(const LbmHandle* h, int share) {
+  const int nx = (int)h->nx, ny = (int)h->ny, nz = (int)h->nz;
+  PhiTile best{};
+  double best_eff = -1.0;
+  for (int ntz = 1; ntz <= nz; ++ntz) {
+    const int tz = (nz + ntz - 1) / ntz;
+    if (tz + 2 > kPhisThreads / 3) continue;
+    const int rows = kPhisThreads / (tz + 2) - 2;
+    const int nty = (ny + rows - 1) / rows, ty = (ny + nty - 1) / nty, ntz_ = (nz + tz - 1) / tz;
+    const double eff = (double)ny * nz / ((double)nty * ntz_ * kPhisThreads);
+    if (eff > best_eff * 1.01) {
+      best_eff = eff;
+      best.ty = ty;
+      best.tz = tz;
+      best.nty = nty;
+      best.ntz = ntz_;
+    }
+    if (tz <= 8) break;
+  }
+  const long long tiles = (long long)best.nty * best.ntz * std::max(1, share);
+  long long best_cost = -1;
+  for (int cx = 2; cx <= std::min(nx + (nx & 1), 64); cx += 2) {
+    const int ncx = (nx + cx - 1) / cx;
+    const long long cost = (tiles * ncx + kPhisSlots - 1) / kPhisSlots * (cx + 2);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best.cx = cx;
+      best.ncx = ncx;
+    }
+  }
+  return best;
+}
+
 // upd_block: threads per block of the linear-layout update kernel (the
 // paired update kernel always runs kPairUpdBlock).
 int upd_blocks_of(const LbmHandle* h, int upd_block) {
   const int64_t bs = h->paired ? kPairUpdBlock : upd_block;
   return (int)((units_of(h) + bs - 1) / bs);
-}
-
-// The step kernels of a grid's layout over a case table: the paired kernels
-// or the single-node kernels.
-template <typename T, typename S>
-cudaError_t launch_phi_kernel(bool paired, const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
-  return paired ? launch_phi_pair<T, S>(cases, b2c, blocks, st) : launch_phi_batch<T, S>(cases, b2c, blocks, st);
-}
-template <typename T, typename S>
-cudaError_t launch_update_kernel(bool paired, const void* cases, const unsigned short* b2c, int blocks, bool omega1,
-                                 cudaStream_t st, bool gmu, int upd_block) {
-  return paired ? launch_update_pair<T, S>(cases, b2c, blocks, omega1, st, gmu)
-                : launch_update_batch<T, S>(cases, b2c, blocks, omega1, st, gmu, upd_block);
 }
 
 // The handle's one-case descriptor table for the batched kernels: [0] the
@@ -596,8 +652,8 @@ int fill_desc(LbmHandle* h, cudaStream_t st) {
     State<T, S> s = make_state<T, S>(*h, h->cur ^ par, h->pc ^ par);
     s.c_prev = h->c_last ^ par;
     s.c_cur = h->c_last ^ par ^ 1;
-    fill_case_desc<T, S>(buf.data() + par * db, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread), 0,
-                         upd_blocks_of(h, h->upd_block));
+    fill_case_desc<T, S>(buf.data() + par * db, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread, true), 0,
+                         upd_blocks_of(h, h->upd_block), 0, PhiTile{});
   }
   // earlier steps on `st` may still read the old table
   CUDA_TRY(cudaStreamSynchronize(st));
@@ -615,21 +671,30 @@ int fill_desc(LbmHandle* h, cudaStream_t st) {
 template <typename T, typename S>
 int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid) {
   if (t.tx == 0 && !h->raw && !h->first) {
-    if (!h->desc_ok) {
-      const int rc = fill_desc<T, S>(h, st);
-      if (rc != LBM_OK) return rc;
-    }
-    const int par = (h->cur ^ h->desc_cur0) & 1;
     const bool gmu = h->mu != nullptr;
-    const unsigned char* d = static_cast<const unsigned char*>(h->desc) + par * case_desc_bytes<T, S>();
-    CUDA_TRY((launch_phi_kernel<T, S>(h->paired, d, nullptr, phi_blocks_of(h, h->phi_per_thread), st)));
-    if (mid) CUDA_TRY(cudaEventRecord(mid, st));
-    if (gmu) {
-      State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
-      CUDA_TRY((launch_mu<T, S>(consts_of<T>(*h), s, st)));
+    State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
+    s.c_prev = h->c_last;
+    s.c_cur = h->c_last ^ 1;
+    alignas(16) unsigned char one[kDescBytes];
+    const unsigned char* d = one;
+    if (h->paired) {
+      if (!h->desc_ok) {
+        const int rc = fill_desc<T, S>(h, st);
+        if (rc != LBM_OK) return rc;
+      }
+      d = static_cast<const unsigned char*>(h->desc) + ((h->cur ^ h->desc_cur0) & 1) * case_desc_bytes<T, S>();
+      CUDA_TRY((launch_phi_pair<T, S>(d, nullptr, phi_blocks_of(h, h->phi_per_thread, true), st)));
+    } else {
+      if (case_desc_bytes<T, S>() > kDescBytes) return fail(LBM_E_ARG, "lbm_step: internal error: descriptor size");
+      fill_case_desc<T, S>(one, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread, true), 0,
+                           upd_blocks_of(h, h->upd_block), 0, h->tile);
+      if (h->sform) CUDA_TRY((launch_phis_one<T, S>(d, st)));
+      else CUDA_TRY((launch_phi_one<T, S>(d, st)));
     }
-    CUDA_TRY((launch_update_kernel<T, S>(h->paired, d, nullptr, upd_blocks_of(h, h->upd_block), omega1_of(h), st,
-                                         gmu, h->upd_block)));
+    if (mid) CUDA_TRY(cudaEventRecord(mid, st));
+    if (gmu) CUDA_TRY((launch_mu<T, S>(consts_of<T>(*h), s, st)));
+    if (h->paired) CUDA_TRY((launch_update_pair<T, S>(d, nullptr, upd_blocks_of(h, h->upd_block), omega1_of(h), st, gmu)));
+    else CUDA_TRY((launch_update_one<T, S>(d, omega1_of(h), wants_s(h), st, gmu, h->upd_block)));
     return LBM_OK;
   }
   State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
@@ -639,8 +704,33 @@ int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid)
   return LBM_OK;
 }
 
+// The state's populations, rebuilt from S where the state is in source form: callers that
+// read or save f.  They are evaluated into the buffer the next step would
+// write, which then takes the place of the current one.
+template <typename T, typename S>
+int expand_t(LbmHandle* h, cudaStream_t st) {
+  State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
+  CUDA_TRY((launch_expand<T, S>(consts_of<T>(*h), s, st)));
+  return LBM_OK;
+}
+int ensure_populations(LbmHandle* h, cudaStream_t st) {
+  if (!h->sform) return LBM_OK;
+  const int rc = with_types(h->prec, [&](auto tag) {
+    return expand_t<typename decltype(tag)::T, typename decltype(tag)::S>(h, st);
+  });
+  if (rc != LBM_OK) return rc;
+  std::swap(h->f[0], h->f[1]);
+  h->sform = false;
+  h->desc_ok = false;
+  return LBM_OK;
+}
+
 template <typename T, typename S>
 int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr) {
+  if (nsteps > 0 && h->tiling.tx != 0) {
+    const int rc = ensure_populations(h, st);  // the fused kernel reads f
+    if (rc != LBM_OK) return rc;
+  }
   for (int i = 0; i < nsteps; ++i) {
     if (ev) CUDA_TRY(cudaEventRecord(ev[2 * i], st));
     int rc;
@@ -651,6 +741,7 @@ int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr
       rc = launch_next<T, S>(h, h->tiling, st, ev ? ev[2 * i + 1] : nullptr);
     }
     if (rc != LBM_OK) return rc;
+    h->sform = !h->raw && h->tiling.tx == 0 && wants_s(h);  // the first step writes populations
     h->last_raw_in = h->raw;
     h->obs_init = false;
     h->cur ^= 1;
@@ -760,6 +851,7 @@ int lbm_create(const LbmParams* params, int64_t nx, int64_t ny, int64_t nz, int 
   if (!h) return fail(LBM_E_ARG, "lbm_create: out of host memory");
   h->prm = *params;
   h->prec = precision;
+  if (gmu) h->upd_block = kBlock;
   h->nx = nx;
   h->ny = ny;
   h->nz = nz;
@@ -775,6 +867,7 @@ int lbm_create(const LbmParams* params, int64_t nx, int64_t ny, int64_t nz, int 
   cudaGetDevice(&h->device);
   const size_t T = h->tsize;
   h->tiling = make_tiling(nx, ny, nz, 0, 0, 0, precision);
+  if (nz > 1) h->tile = phis_tile(h, 1);
   const Sizes z = sizes_of(nx, ny, nz, precision);
   cudaError_t e = cudaSuccess;
   auto A = [&](void** p, size_t bytes) {
@@ -1037,6 +1130,7 @@ int lbm_init_fields(LbmHandle* h, const void* phi, const void* u, int src_dtype,
   if (direct) CUDA_TRY(cudaStreamSynchronize(st));
   h->initialized = true;
   h->desc_ok = false;
+  h->sform = false;
   h->raw = true;
   h->first = true;
   h->c_last = 0;
@@ -1139,6 +1233,13 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
   float best_t = 1e30f;
   int rc = LBM_OK;
   for (const Tiling& t : cands) {
+    if (t.tx != 0 && h->sform) {
+      // the fused kernel reads f, which follows from the saved u
+      const cudaError_t e = cudaMemcpyAsync(h->u, u_save, ub, cudaMemcpyDeviceToDevice, st);
+      rc = e == cudaSuccess ? ensure_populations(h, st)
+                            : fail(LBM_E_CUDA, std::string("lbm_autotune: ") + cudaGetErrorString(e));
+      if (rc != LBM_OK) break;
+    }
     // the two-kernel step: also its phi kernel's nodes per thread and the
     // update kernel's threads per block (256 only for the gradient-of-mu modes
     // and the paired layout, whose update kernel has a fixed block)
@@ -1274,6 +1375,10 @@ int lbm_inject_droplet(LbmHandle* h, const double* center3, double radius, doubl
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_inject_droplet: call lbm_init_fields first");
   if (!(radius >= 0.0) || !(xi > 0.0)) return fail(LBM_E_ARG, "lbm_inject_droplet: radius >= 0 and xi > 0 required");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  {
+    const int rc = ensure_populations(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   InjectParams ip;
   std::memset(&ip, 0, sizeof(ip));
   for (int d = 0; d < 3; ++d) {
@@ -1322,6 +1427,7 @@ int lbm_inject_droplet(LbmHandle* h, const double* center3, double radius, doubl
   h->first = true;
   h->obs_init = true;
   h->last_raw_in = true;
+  h->sform = false;
   h->desc_ok = false;
   if (core_nodes) {
     unsigned cnt = 0;
@@ -1336,6 +1442,10 @@ int lbm_get_populations(LbmHandle* h, void* f, void* g, void* stream) {
   if (!h) return fail(LBM_E_ARG, "lbm_get_populations: null handle");
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_get_populations: not initialised");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (f) {
+    const int rc = ensure_populations(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   cudaError_t e;
   // fin = the current state, phi_in = the latest phi, c_prev = its correction
   e = with_types(h->prec, [&](auto tag) {
@@ -1510,6 +1620,10 @@ int lbm_save_state(LbmHandle* h, void* host, int64_t bytes, void* stream) {
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_save_state: call lbm_init_fields first");
   if (bytes != (int64_t)state_bytes(h)) return fail(LBM_E_ARG, "lbm_save_state: buffer size is not lbm_state_bytes");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  {
+    const int rc = ensure_populations(h, st);  // the blob holds populations
+    if (rc != LBM_OK) return rc;
+  }
   StateHeader hd;
   std::memset(&hd, 0, sizeof(hd));
   hd.magic = kStateMagic;
@@ -1583,6 +1697,7 @@ int lbm_load_state(LbmHandle* h, const void* host, int64_t bytes, void* stream) 
   h->obs_init = hd.obs_init != 0;
   h->steps = hd.steps;
   h->initialized = true;
+  h->sform = false;
   h->desc_ok = false;
   return LBM_OK;
 }
@@ -1668,16 +1783,19 @@ struct LbmBatch {
   // with omega_f == 1, 1 linear other, 2 paired layout with omega_f == 1, 3 paired other
   int gstart[5] = {0, 0, 0, 0, 0};
   int phi_per_thread = 16;  // nodes per phi-kernel thread (half as many pairs in the paired layout)
-  int upd_block = kBlock;   // threads per block of the linear-layout update kernel
+  int upd_block = 128;      // threads per block of the linear-layout update kernel
   bool coop = false;        // one cooperative launch per step (k_batch_coop) instead of two launches
   size_t desc = 0;          // bytes of one case descriptor
   void* table[2] = {nullptr, nullptr};  // device descriptors: [0] this step, [1] the next
   unsigned char* staging = nullptr;     // pinned host copy of both tables
   cudaEvent_t staged = nullptr;         // the last copy out of `staging` has run
-  // block -> case: the phi grids of the linear and the paired cases, then the
-  // update grids of the four groups
+  // block -> case: the phi grids of the linear and the paired cases, the
+  // update grids of the four groups, then the source form's phi grid of the linear
+  // cases with omega_f == 1 (float compute)
   unsigned short* b2c = nullptr;
-  int phi_blocks[2] = {0, 0}, upd_blocks[4] = {0, 0, 0, 0};
+  int phi_blocks[2] = {0, 0}, upd_blocks[4] = {0, 0, 0, 0}, phis_blocks = 0;
+  int phi_blocks_om1 = 0;               // linear phi blocks of the omega_f == 1 cases (the first of them)
+  bool graph_s = false;                 // the graph's phi pass reads S
   cudaStream_t cap = nullptr;           // stream used to capture the two-step graph
   cudaGraphExec_t graph = nullptr;
 };
@@ -1693,26 +1811,33 @@ int batch_layout(LbmBatch* b) {
   if (b->b2c) cudaFree(b->b2c);
   b->b2c = nullptr;
   const int n = (int)b->h.size();
-  long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0};
+  long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0, pb_om1 = 0;
   for (int i = 0; i < n; ++i) {
-    pb[b->h[i]->paired ? 1 : 0] += phi_blocks_of(b->h[i], b->phi_per_thread);
-    ub[launch_group(b->h[i])] += upd_blocks_of(b->h[i], b->upd_block);
+    const int phin = phi_blocks_of(b->h[i], b->phi_per_thread), g = launch_group(b->h[i]);
+    pb[b->h[i]->paired ? 1 : 0] += phin;
+    ub[g] += upd_blocks_of(b->h[i], b->upd_block);
+    if (g == 0) pb_om1 += phin;
+    if (wants_s(b->h[i])) jb += phis_tile(b->h[i], n).blocks();
   }
-  const long long tot = pb[0] + pb[1] + ub[0] + ub[1] + ub[2] + ub[3];
+  const long long tot = pb[0] + pb[1] + ub[0] + ub[1] + ub[2] + ub[3] + jb;
   if (tot > 0x7fffffff) return fail(LBM_E_ARG, "lbm_batch: grids too large");
   for (int j = 0; j < 2; ++j) b->phi_blocks[j] = (int)pb[j];
   for (int g = 0; g < 4; ++g) b->upd_blocks[g] = (int)ub[g];
+  b->phis_blocks = (int)jb;
+  b->phi_blocks_om1 = (int)pb_om1;
   std::vector<unsigned short> t((size_t)tot);
-  size_t at[6];
+  size_t at[7];
   at[0] = 0;
   at[1] = (size_t)pb[0];
   at[2] = at[1] + (size_t)pb[1];
-  for (int g = 0; g < 3; ++g) at[3 + g] = at[2 + g] + (size_t)ub[g];
+  for (int g = 0; g < 4; ++g) at[3 + g] = at[2 + g] + (size_t)ub[g];
   for (int i = 0; i < n; ++i) {
     size_t& a = at[b->h[i]->paired ? 1 : 0];
     for (int k = phi_blocks_of(b->h[i], b->phi_per_thread); k > 0; --k) t[a++] = (unsigned short)i;
     size_t& c = at[2 + launch_group(b->h[i])];
     for (int k = upd_blocks_of(b->h[i], b->upd_block); k > 0; --k) t[c++] = (unsigned short)i;
+    if (wants_s(b->h[i]))
+      for (int k = phis_tile(b->h[i], n).blocks(); k > 0; --k) t[at[6]++] = (unsigned short)i;
   }
   CUDA_TRY(cudaMalloc(&b->b2c, t.size() * sizeof(unsigned short)));
   CUDA_TRY(cudaMemcpy(b->b2c, t.data(), t.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
@@ -1723,9 +1848,10 @@ int batch_layout(LbmBatch* b) {
 template <typename T, typename S>
 void batch_fill_t(LbmBatch* b) {
   const int n = (int)b->h.size();
-  int pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0};
+  int pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0;
   for (int i = 0; i < n; ++i) {
     LbmHandle* h = b->h[i];
+    const PhiTile tile = wants_s(h) ? phis_tile(h, n) : PhiTile{};
     const int phin = phi_blocks_of(h, b->phi_per_thread), updn = upd_blocks_of(h, b->upd_block),
               g = launch_group(h);
     int& pbl = pb[h->paired ? 1 : 0];
@@ -1734,10 +1860,11 @@ void batch_fill_t(LbmBatch* b) {
       s.c_prev = h->c_last ^ par;
       s.c_cur = h->c_last ^ par ^ 1;
       fill_case_desc<T, S>(b->staging + ((size_t)par * n + i) * b->desc, consts_of<T>(*h), s, pbl, phin, ub[g],
-                           updn);
+                           updn, jb, tile);
     }
     pbl += phin;
     ub[g] += updn;
+    jb += tile.blocks();
   }
 }
 
@@ -1755,39 +1882,62 @@ int batch_fill(LbmBatch* b, cudaStream_t st) {
   return LBM_OK;
 }
 
-// One batched step reading descriptor table `par`: the phi kernel over every
-// linear-layout case and over every paired case, then the update kernel over
-// each group (layout x omega_f == 1 or not).  Empty launches are skipped.
+// One batched step reading descriptor table `par`: the phi kernels over every
+// linear-layout case (phis_in: the omega_f == 1 ones are in source
+// form and go through that form's kernel) and over every paired case, then the update kernel over each group
+// (layout x omega_f == 1 or not).  Empty launches are skipped.
 template <typename T, typename S>
-cudaError_t batch_launch_t(LbmBatch* b, int par, cudaStream_t st) {
+cudaError_t batch_launch_t(LbmBatch* b, int par, bool phis_in, cudaStream_t st) {
+  const void* tab = b->table[par];
   if (b->coop)
-    return launch_batch_coop<T, S>(b->table[par], b->b2c, b->phi_blocks[0], b->upd_blocks[0], b->upd_blocks[1], st);
+    return launch_batch_coop<T, S>(tab, b->b2c, b->phi_blocks[0], b->upd_blocks[0], b->upd_blocks[1], st);
   const unsigned short* t = b->b2c;
+  const unsigned short* upd = t + b->phi_blocks[0] + b->phi_blocks[1];
+  const unsigned short* tj = upd + b->upd_blocks[0] + b->upd_blocks[1] + b->upd_blocks[2] + b->upd_blocks[3];
+  const bool j = b->phis_blocks > 0;
+  const int skip = j && phis_in ? b->phi_blocks_om1 : 0;  // the omega_f == 1 cases come first
   cudaError_t e = cudaSuccess;
-  for (int j = 0; j < 2 && e == cudaSuccess; ++j) {
-    e = launch_phi_kernel<T, S>(j == 1, b->table[par], t, b->phi_blocks[j], st);
-    t += b->phi_blocks[j];
-  }
+  if (j && phis_in) e = launch_phis_batch<T, S>(tab, tj, b->phis_blocks, st);
+  if (e == cudaSuccess) e = launch_phi_batch<T, S>(tab, t, skip, b->phi_blocks[0] - skip, st);
+  if (e == cudaSuccess) e = launch_phi_pair<T, S>(tab, t + b->phi_blocks[0], b->phi_blocks[1], st);
   for (int g = 0; g < 4 && e == cudaSuccess; ++g) {
-    e = launch_update_kernel<T, S>(g >= 2, b->table[par], t, b->upd_blocks[g], (g & 1) == 0, st, false,
-                                   b->upd_block);
-    t += b->upd_blocks[g];
+    e = g < 2 ? launch_update_batch<T, S>(tab, upd, b->upd_blocks[g], g == 0, j, st, b->upd_block)
+              : launch_update_pair<T, S>(tab, upd, b->upd_blocks[g], g == 2, st, false);
+    upd += b->upd_blocks[g];
   }
   return e;
 }
-cudaError_t batch_launch(LbmBatch* b, int par, cudaStream_t st) {
+cudaError_t batch_launch(LbmBatch* b, int par, bool phis_in, cudaStream_t st) {
   return with_types(b->prec, [&](auto tag) {
-    return batch_launch_t<typename decltype(tag)::T, typename decltype(tag)::S>(b, par, st);
+    return batch_launch_t<typename decltype(tag)::T, typename decltype(tag)::S>(b, par, phis_in, st);
   });
 }
 
+// Makes the form of f the same for all cases that can hold S: true when all of
+// them do, else all hold populations (the cooperative step's form too).
+int batch_form(LbmBatch* b, cudaStream_t st, bool* phis_in) {
+  bool all = !b->coop;
+  for (LbmHandle* h : b->h)
+    if (wants_s(h)) all = all && h->sform;
+  if (!all)
+    for (LbmHandle* h : b->h) {
+      const int rc = ensure_populations(h, st);
+      if (rc != LBM_OK) return rc;
+    }
+  *phis_in = all;
+  return LBM_OK;
+}
+
 // The two-step graph (table 0, then table 1), captured on the batch's own stream.
-int batch_graph(LbmBatch* b) {
-  if (b->graph) return LBM_OK;
+int batch_graph(LbmBatch* b, bool phis_in) {
+  if (b->graph && b->graph_s == phis_in) return LBM_OK;
+  if (b->graph) cudaGraphExecDestroy(b->graph);
+  b->graph = nullptr;
+  b->graph_s = phis_in;
   cudaGraph_t g = nullptr;
   CUDA_TRY(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = batch_launch(b, 0, b->cap);
-  if (e == cudaSuccess) e = batch_launch(b, 1, b->cap);
+  cudaError_t e = batch_launch(b, 0, phis_in, b->cap);
+  if (e == cudaSuccess) e = batch_launch(b, 1, phis_in, b->cap);
   const cudaError_t e2 = cudaStreamEndCapture(b->cap, &g);
   if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
@@ -1807,6 +1957,7 @@ void batch_advance(LbmBatch* b, int nsteps) {
       h->c_last ^= 1;
     }
     h->steps += nsteps;
+    if (nsteps > 0) h->sform = !b->coop && wants_s(h);
     h->last_raw_in = false;
     h->obs_init = false;
   }
@@ -1902,15 +2053,26 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
     --rest;
   }
   if (rest == 0) return LBM_OK;
-  int rc = batch_fill(b, st);
+  bool phis_in = false;
+  int rc = batch_form(b, st, &phis_in);
+  if (rc == LBM_OK) rc = batch_fill(b, st);
   if (rc != LBM_OK) return rc;
+  if (!phis_in && !b->coop && b->phis_blocks > 0) {
+    // from populations to S: one step, then the tables of the other parity
+    CUDA_TRY(batch_launch(b, 0, false, st));
+    batch_advance(b, 1);
+    if (--rest == 0) return LBM_OK;
+    phis_in = true;
+    rc = batch_fill(b, st);
+    if (rc != LBM_OK) return rc;
+  }
   if (rest >= 2) {
-    rc = batch_graph(b);
+    rc = batch_graph(b, phis_in);
     if (rc != LBM_OK) return rc;
     for (int i = 0; i < rest / 2; ++i) CUDA_TRY(cudaGraphLaunch(b->graph, st));
   }
   // after an even number of steps every case is back at the parity of table 0
-  if (rest & 1) CUDA_TRY(batch_launch(b, 0, st));
+  if (rest & 1) CUDA_TRY(batch_launch(b, 0, phis_in, st));
   batch_advance(b, rest);
   return LBM_OK;
 }
@@ -1958,19 +2120,21 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
-  int best = b->phi_per_thread, best_bs = b->upd_block, rc = LBM_OK;
+  bool phis_in = false;
+  int best = b->phi_per_thread, best_bs = b->upd_block, rc = batch_form(b, st, &phis_in);
   float best_t = 1e30f;
   for (int bs : {128, kBlock})
   for (int per : {1, 2, 4, 8, 12, 16, 24, 32}) {
+    if (rc != LBM_OK) break;
     if (b->coop && bs != kBlock) continue;  // the cooperative step runs 256-thread update blocks
     b->phi_per_thread = per;
     b->upd_block = bs;
     rc = batch_layout(b);
     if (rc == LBM_OK) rc = batch_fill(b, st);
     if (rc != LBM_OK) break;
-    cudaError_t e = batch_launch(b, 0, st);  // warm-up
+    cudaError_t e = batch_launch(b, 0, phis_in, st);  // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = batch_launch(b, 0, st);
+    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = batch_launch(b, 0, phis_in, st);
     if (e == cudaSuccess) e = cudaEventRecord(e1, st);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;

@@ -189,6 +189,12 @@ struct Consts {
   // chemical-potential gradient terms of the interface source
   // (lbm/fe_ac_solver.py:457-486): 0 none, kGmuCH Cahn-Hilliard, kGmuDrive mu_drive
   int gmu_mode;
+  // folded products of the constants above
+  T inv_floor, inv_floor_cs2;  // 1 / rho_floor, 1 / (rho_floor cs2)
+  T drho_cs2;   // drho cs2 (pressure force)
+  T visc_drho;  // visc drho (viscous force)
+  T sharp;      // 4 cs2 ac_scale / W (sharpening)
+  T src_c;      // (1 - 1/(2 tau_f)) / cs2 (Allen-Cahn source)
   T mob, guo, mu_drive_a;  // mobility cs2 (tau_f - 1/2), tau_f / (tau_f - 1/2), mu_drive * mobility
 };
 constexpr int kGmuCH = 1;
@@ -230,6 +236,14 @@ struct State {
 struct InjectParams {
   double c[3], radius, xi, u[3];
   int obs_init;
+};
+
+// Work split of the phi pass over a state that holds J (lbm_phij.cuh): a
+// block walks cx planes in x over a ty x tz tile of the (y, z) plane.
+struct PhiTile {
+  int ty, tz, cx;      // tile extents, planes per block
+  int nty, ntz, ncx;   // tiles in y and z, blocks along x
+  __host__ __device__ int blocks() const { return nty * ntz * ncx; }
 };
 
 // Tiling of the fused step kernel: one CTA per tile of TX x TY x TZ nodes

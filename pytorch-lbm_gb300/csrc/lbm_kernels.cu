@@ -16,24 +16,36 @@
 // without c and without relaxation.  Right after init (RAW) the buffers hold
 // the reference state itself.
 //
-// One step = two launches (k_phi_batch, k_update_batch; the first step after
-// init: k_phi, k_update).  k_phi recovers phi of every node (pulling f) into
-// the phi buffer and reduces the grid's sum of phi, an exact fixed-point sum,
-// into the next mass-correction factor; k_update reads the phi stencil from
-// L2 and runs the stencils, wetting, forces, velocity, Allen-Cahn source and
-// both BGK collisions of every node (pulling g).  The batched kernels serve
-// many grids per launch through a case table and single grids through a
-// one-entry table.  An alternative fused kernel (k_step) does a whole step in
-// one launch per tile of nodes, recomputing phi on a one-node halo in shared
-// memory.  Arithmetic follows the reference's operation order where it
-// matters for parity; the isotropic gradient is accumulated without FMA
-// contraction.  (Measured and dropped for k_phi: runs of four consecutive
-// nodes per thread -- 43 -> 58 us, the per-thread runs break coalescing.)
+// One step = a phi pass and an update (k_phi_one / k_phis_one and
+// k_update_one; batches: the _batch forms; the first step after init: k_phi,
+// k_update).  The phi pass recovers phi of every node into the phi buffer and
+// reduces the grid's sum of phi, an exact fixed-point sum, into the next
+// mass-correction factor; the update reads the phi stencil from L2 and runs the
+// stencils, wetting, forces, velocity, Allen-Cahn source and both BGK collisions
+// of every node (pulling g).
+//
+// Source form.  With tau_f == 1 (float compute, linear layout) the update stores
+// the interface source S in the place of f's 19 populations, and the phi pass
+// evaluates them again from phi, u and S (lbm_phis.cuh): 197 + 33 bytes per node
+// and step (float) instead of 257 + 81.  Whatever reads f gets it back with
+// k_expand.  Measured with the block-uniform addressing below on the 150x150x107
+// case: 171.9 -> 144.4 us per step, 256x256x192 909 -> 702 us, 384x384x256 in
+// half storage 2288 -> 1849 us, 80x80x65 44.5 -> 31.0 us.
+//
+// A grid alone gets its descriptor as a kernel parameter; the batched kernels
+// serve many grids per launch through a case table in device memory.  An
+// alternative fused kernel (k_step) does a whole step in one launch per tile of
+// nodes, recomputing phi on a one-node halo in shared memory.  Arithmetic
+// follows the reference's operation order where it matters for parity; the
+// isotropic gradient is accumulated without FMA contraction.  (Measured and
+// dropped for k_phi: runs of four consecutive nodes per thread -- 43 -> 58 us,
+// the per-thread runs break coalescing.)
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
@@ -126,10 +138,10 @@ template <>
 struct PopIO<float, __half> {
   static constexpr bool kDev = true;
   __device__ __forceinline__ static float ld_f(__half raw, int q, float ref, const Consts<float>& k) {
-    return Lat<float>::w(q) * (__half2float(raw) + ref);
+    return __fmul_rn(Lat<float>::w(q), __fadd_rn(__half2float(raw), ref));
   }
   __device__ __forceinline__ static __half st_f(float v, int q, float ref, const Consts<float>& k) {
-    return __float2half_rn(v * Lat<float>::inv_w(q) - ref);
+    return __float2half_rn(__fmaf_rn(v, Lat<float>::inv_w(q), -ref));
   }
   __device__ __forceinline__ static float ld_g(__half raw, int q, const Consts<float>& k) {
     return Lat<float>::w(q) * __half2float(raw);
@@ -163,11 +175,19 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float rcp(float a) { return 1.0f / a; }
+__device__ __forceinline__ double rcp(double a) { return 1.0 / a; }
+__device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
+__device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
+__device__ __forceinline__ float sqrt_rn(float a) { return __fsqrt_rn(a); }
+__device__ __forceinline__ double sqrt_rn(double a) { return __dsqrt_rn(a); }
+__device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 // Fused multiply-add, written out where the step relies on it.
 template <typename T>
 __device__ __forceinline__ T fma_(T a, T b, T c) { return fma(a, b, c); }
-__device__ __forceinline__ double rcp(double a) { return 1.0 / a; }
 
 // q = floor(t / d) for 0 <= t < 2^22 via a float reciprocal: the relative
 // error of (t + 1/2) * (1/d) is below 2^-23, inside the 1/(2d) margin.
@@ -267,14 +287,15 @@ __device__ __forceinline__ void fetch_pop(T (&v)[Q], const Consts<T>& k, const S
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = ld(q, q * Nu + I(nb.at(n, -ex(q), -ey(q), -ez(q))), ref_self);
     if (c & kPartial) {
-      const T one_m = T(1) - eps;
+      const T one_m = sub_rn(T(1), eps);
 #pragma unroll
-      for (int q = 0; q < Q; ++q) v[q] = one_m * v[q] + eps * ld(opp(q), opp(q) * Nu + nu, ref_nb(q));
+      for (int q = 0; q < Q; ++q)
+        v[q] = fma_(one_m, v[q], mul_rn(eps, ld(opp(q), opp(q) * Nu + nu, ref_nb(q))));
     }
   }
   if (WITH_C) {
 #pragma unroll
-    for (int q = 0; q < Q; ++q) v[q] = v[q] * corr;
+    for (int q = 0; q < Q; ++q) v[q] = mul_rn(v[q], corr);
   }
 }
 
@@ -309,7 +330,7 @@ __device__ __forceinline__ T relax_target(const Consts<T>& k, const T* __restric
       target = clamp01((cubic[2] + sqrt(disc)) / cubic[3]);
     }
   }
-  return clamp01(pb + k.relax_r * (target - pb));
+  return clamp01(fma_(k.relax_r, sub_rn(target, pb), pb));
 }
 
 // Relaxation scale of lbm/fe_ac_solver.py:626-629.
@@ -332,12 +353,64 @@ __device__ __forceinline__ void fetch_f(T (&v)[Q], const Consts<T>& k, const Sta
     if (r >= T(0)) {
       const T sc = relax_scale(r, seqsum(v));
 #pragma unroll
-      for (int q = 0; q < Q; ++q) v[q] = v[q] * sc;
+      for (int q = 0; q < Q; ++q) v[q] = mul_rn(v[q], sc);
     }
   }
 }
 
-// Lattice constants as the step kernels read them: compile-time immediates
+// phi of fluid node n from its populations v (pulled, bounced back and blended):
+// the last step's mass correction, boundary-phi relaxation, their sum in
+// velocity order (lbm/fe_ac_solver.py:385-389, 582-636).  float64 fuses the
+// correction into the sum (19 operations on the slow float64 pipe instead of
+// 37: phi pass of a 96^3 grid 132 -> 85 us).
+template <typename T, typename S, bool MAP>
+__device__ __forceinline__ T phi_of(const Consts<T>& k, const State<T, S>& s, int n, uint8_t c, T (&v)[Q], T corr,
+                                    T phi_prev) {
+  T sum;
+  if constexpr (sizeof(T) == 8) {
+    sum = mul_rn(v[0], corr);
+#pragma unroll
+    for (int q = 1; q < Q; ++q) sum = fma_(v[q], corr, sum);
+  } else {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = mul_rn(v[q], corr);
+    sum = seqsum(v);
+  }
+  if (k.relax_on && (c & kTop)) {
+    const T r = relax_target<T, MAP>(k, s.phi_in, s.nsw, s.cubic, n, phi_prev, corr);
+    if (r >= T(0)) {
+      const T sc = relax_scale(r, sum);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) v[q] = mul_rn(sizeof(T) == 8 ? mul_rn(v[q], corr) : v[q], sc);
+      sum = seqsum(v);
+    }
+  }
+  return clamp01(sum);
+}
+
+// phi of fluid node n from stored populations.
+template <typename T, typename S, bool RAW, bool MAP>
+__device__ __forceinline__ T phi_value(const Consts<T>& k, const State<T, S>& s, int n, uint8_t c, const Nbr& nb,
+                                       unsigned long long pol) {
+  const T eps = (c & kPartial) ? s.eps[n] : T(0);
+  T v[Q];
+  if constexpr (RAW && PopIO<T, S>::kDev) {
+    // the first step of the half form: deviation plus reference, weighted into the sum by fused multiply-adds
+    const unsigned e = MAP ? sidx(k, n) : (unsigned)n;
+    const T ref = ldg(s.phi_in + e);
+    auto h = [&](int q) { return add_rn(__half2float(ld_pol(s.fin + (q * (unsigned)k.Np + e), pol)), ref); };
+    T sum = fma_(Lat<T>::w(0), h(0), mul_rn(Lat<T>::w(1), h(1)));
+#pragma unroll
+    for (int q = 2; q < Q; ++q) sum = fma_(Lat<T>::w(q), h(q), sum);
+    return clamp01(sum);
+  }
+  fetch_pop<T, S, RAW, false, true, true, MAP>(v, k, s.fin, s.phi_in, n, (size_t)k.N, nb, c, eps, T(1), pol);
+  if (RAW) return clamp01(seqsum(v));
+  return phi_of<T, S, MAP>(k, s, n, c, v, s.cbuf[s.c_prev],
+                           (k.relax_on && (c & kTop)) ? ldg(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)) : T(0));
+}
+
+// Lattice constants as the paired step kernels read them: compile-time immediates
 // (IMM) or the grid's constant table.  Both hold the same values (the table is
 // checked against the immediates when it is built); which is faster depends
 // on the kernel's register allocation (measured on the 150x150x107 case:
@@ -354,58 +427,78 @@ struct LatK {
   __device__ __forceinline__ T inv_two_cs2() const { return IMM ? Lat<T>::inv_two_cs2() : k.inv_two_cs2; }
 };
 
+// First population of each opposite pair (q, opp q) of D3Q19.
+__host__ __device__ constexpr int pair_first(int i) {
+  return i == 0 ? 1 : i == 1 ? 3 : i == 2 ? 5 : i == 3 ? 7 : i == 4 ? 8 : i == 5 ? 11 : i == 6 ? 12 : i == 7 ? 15 : 16;
+}
+
+// e_q . (a0, a1, a2) with the reference's exact two-term sums.
+template <typename T>
+__device__ __forceinline__ T edot(int q, T a0, T a1, T a2) {
+  T r = T(0);
+  bool any = false;
+  if (ex(q) != 0) { r = ex(q) > 0 ? a0 : -a0; any = true; }
+  if (ey(q) != 0) { const T t = ey(q) > 0 ? a1 : -a1; r = any ? r + t : t; any = true; }
+  if (ez(q) != 0) { const T t = ez(q) > 0 ? a2 : -a2; r = any ? r + t : t; }
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // Isotropic gradient / laplacian with the ghost-node wetting correction
 // (lbm/fe_ac_solver.py:296-320 fused, :282-294 unfused; fe_wetting.py:418-446).
 // ps[q] holds phi(x + e_q); nsolid(q) tells whether that neighbour is solid.
 // ---------------------------------------------------------------------------
-// PAIR: the gradient from opposite-pair differences t_q = (w_q / cs2)
-// (phi(x + e_q) - phi(x - e_q)), nine products instead of thirty, with
-// mirror partners summed first so that a mirror-symmetric phi still gives
-// an exactly zero component (the sharpening normal grad / |grad| depends on
-// it where the gradient vanishes).
-template <typename T, bool FUSED, typename St, typename SolidFn, bool PAIR = false, bool IMM = false>
+// FUSED is the step's form, every operation explicitly rounded, so that each
+// kernel that uses it gives the same bits: the gradient from opposite-pair
+// differences t_q = (w_q / cs2)(phi(x + e_q) - phi(x - e_q)), mirror partners
+// summed first so that a mirror-symmetric phi gives an exactly zero component
+// (the sharpening normal grad / |grad| depends on it where the gradient
+// vanishes).  float64 takes the laplacian from opposite-pair sums and applies
+// its weights once per weight class (27 operations on the slow float64 pipe
+// instead of 36).
+template <typename T, bool FUSED, typename St, typename SolidFn>
 __device__ __forceinline__ void grad_lap(const Consts<T>& k, const St& s, int n, uint8_t c, T phi,
                                          T (&ps)[Q], SolidFn nsolid, T& gx, T& gy, T& gz, T& lap) {
-  const LatK<T, IMM> L{k};
   if (k.wetting && (c & kBoundary)) {
     const size_t N = (size_t)k.N;
     const float n0 = s.wn[n], n1 = s.wn[N + n], n2 = s.wn[2 * N + n];
 #pragma unroll
     for (int q = 1; q < Q; ++q) {
       if (nsolid(q)) {
-        float nde = 0.0f;
-        nde = __fadd_rn(nde, __fmul_rn(n0, (float)ex(q)));
-        nde = __fadd_rn(nde, __fmul_rn(n1, (float)ey(q)));
-        nde = __fadd_rn(nde, __fmul_rn(n2, (float)ez(q)));
+        const float nde = edot(q, n0, n1, n2);
         if (k.linear) {
-          ps[q] = phi - (T)__fmul_rn(nde, k.h_over_kappa_f);
+          ps[q] = sub_rn(phi, (T)__fmul_rn(nde, k.h_over_kappa_f));
         } else {
-          ps[q] = phi + (T)__fmul_rn(nde, k.pcok_f) * phi * (T(1) - phi);
+          ps[q] = fma_(mul_rn((T)__fmul_rn(nde, k.pcok_f), phi), sub_rn(T(1), phi), phi);
         }
       }
     }
   }
-  gx = gy = gz = lap = T(0);
-  if constexpr (PAIR) {
-    auto t = [&](int q) { return mul_rn(L.wc(q), ps[q] - ps[opp(q)]); };
+  if constexpr (FUSED) {
+    auto t = [&](int q) { return mul_rn(Lat<T>::wc(q), sub_rn(ps[q], ps[opp(q)])); };
     const T t1 = t(1), t3 = t(3), t5 = t(5), t7 = t(7), t8 = t(8), t11 = t(11), t12 = t(12), t15 = t(15),
             t16 = t(16);
-    gx = add_rn(add_rn(t1, t7 - t8), t11 - t12);  // e_x: q 1, 7, -8, 11, -12 (and their opposites)
-    gy = add_rn(add_rn(t3, t7 + t8), t15 - t16);  // e_y: q 3, 7, 8, 15, -16
-    gz = add_rn(add_rn(t5, t11 + t12), t15 + t16);  // e_z: q 5, 11, 12, 15, 16
-  }
-#pragma unroll
-  for (int q = 1; q < Q; ++q) {
-    if (!PAIR) {
-      if (ex(q) != 0) gx = add_rn(gx, mul_rn(ex(q) > 0 ? L.wc(q) : -L.wc(q), ps[q]));
-      if (ey(q) != 0) gy = add_rn(gy, mul_rn(ey(q) > 0 ? L.wc(q) : -L.wc(q), ps[q]));
-      if (ez(q) != 0) gz = add_rn(gz, mul_rn(ez(q) > 0 ? L.wc(q) : -L.wc(q), ps[q]));
-    }
-    if (FUSED) {
-      lap = fma_(L.w2c(q), ps[q] - phi, lap);
+    gx = add_rn(add_rn(t1, sub_rn(t7, t8)), sub_rn(t11, t12));  // e_x: q 1, 7, -8, 11, -12 (and their opposites)
+    gy = add_rn(add_rn(t3, add_rn(t7, t8)), sub_rn(t15, t16));  // e_y: q 3, 7, 8, 15, -16
+    gz = add_rn(add_rn(t5, add_rn(t11, t12)), add_rn(t15, t16));  // e_z: q 5, 11, 12, 15, 16
+    if constexpr (sizeof(T) == 8) {
+      auto d = [&](int q) { return fma_(T(-2), phi, add_rn(ps[q], ps[opp(q)])); };
+      const T la = add_rn(add_rn(d(1), d(3)), d(5));
+      const T ld = add_rn(add_rn(add_rn(d(7), d(8)), add_rn(d(11), d(12))), add_rn(d(15), d(16)));
+      lap = fma_(Lat<T>::w2c(7), ld, mul_rn(Lat<T>::w2c(1), la));
     } else {
-      lap = lap + (T(2) * L.w(q)) * (ps[q] - phi) / L.cs2();
+      lap = T(0);
+#pragma unroll
+      for (int q = 1; q < Q; ++q) lap = fma_(Lat<T>::w2c(q), sub_rn(ps[q], phi), lap);
+    }
+  } else {
+    gx = gy = gz = lap = T(0);
+#pragma unroll
+    for (int q = 1; q < Q; ++q) {
+      if (ex(q) != 0) gx = add_rn(gx, mul_rn(ex(q) > 0 ? k.wc[q] : -k.wc[q], ps[q]));
+      if (ey(q) != 0) gy = add_rn(gy, mul_rn(ey(q) > 0 ? k.wc[q] : -k.wc[q], ps[q]));
+      if (ez(q) != 0) gz = add_rn(gz, mul_rn(ez(q) > 0 ? k.wc[q] : -k.wc[q], ps[q]));
+      lap = lap + (T(2) * k.w[q]) * (ps[q] - phi) / k.cs2;
     }
   }
 }
@@ -413,10 +506,10 @@ __device__ __forceinline__ void grad_lap(const Consts<T>& k, const St& s, int n,
 // Chemical potential (lbm/fe_ac_solver.py:326-340).
 template <typename T>
 __device__ __forceinline__ T chem_pot(const Consts<T>& k, uint8_t c, T phi, T lap) {
-  T mu = fma_(-k.kappa, lap, k.beta4 * phi * (phi - T(1)) * (phi - T(0.5)));
+  T mu = fma_(-k.kappa, lap, mul_rn(mul_rn(mul_rn(k.beta4, phi), sub_rn(phi, T(1))), sub_rn(phi, T(0.5))));
   if (k.wetting && (c & kBoundary)) {
-    if (k.linear) mu = mu + k.mu_wall_add;
-    else mu = mu + k.phi_c * phi * (T(1) - phi);
+    if (k.linear) mu = add_rn(mu, k.mu_wall_add);
+    else mu = fma_(mul_rn(k.phi_c, phi), sub_rn(T(1), phi), mu);
   }
   return mu;
 }
@@ -457,31 +550,8 @@ __device__ __forceinline__ void grad_mu(const Consts<T>& k, const St& s, int n, 
   }
 }
 
-// e_q . (a0, a1, a2) with the reference's exact two-term sums.
-template <typename T>
-__device__ __forceinline__ T edot(int q, T a0, T a1, T a2) {
-  T r = T(0);
-  bool any = false;
-  if (ex(q) != 0) { r = ex(q) > 0 ? a0 : -a0; any = true; }
-  if (ey(q) != 0) { const T t = ey(q) > 0 ? a1 : -a1; r = any ? r + t : t; any = true; }
-  if (ez(q) != 0) { const T t = ez(q) > 0 ? a2 : -a2; r = any ? r + t : t; }
-  return r;
-}
 
-// ---------------------------------------------------------------------------
-// The update of one node (lbm/fe_ac_solver.py:392-530): stencils, chemical
-// potential, wetting, pressure, stress, forces, velocity, Allen-Cahn source
-// and both BGK collisions; writes fout, gout, u, phi_out.
-// ---------------------------------------------------------------------------
-// First population of each opposite pair (q, opp q) of D3Q19.
-__host__ __device__ constexpr int pair_first(int i) {
-  return i == 0 ? 1 : i == 1 ? 3 : i == 2 ? 5 : i == 3 ? 7 : i == 4 ? 8 : i == 5 ? 11 : i == 6 ? 12 : i == 7 ? 15 : 16;
-}
 
-// OMEGA1: tau_f == 1 (the reference's default tau_h = 1.0), where the
-// phase-field BGK collision f - (f - f_eq) + src is f_eq + src and the
-// pre-collision f is not read.  PhiAt(q) gives phi(x + e_q) of this step,
-// SolidAt(q) whether x + e_q is solid.
 // Words of one node's staging slot: the 19 streamed g, u of the last step, phi
 // of the last step.
 constexpr int kStage = Q + 4;
@@ -507,67 +577,216 @@ __device__ __forceinline__ void stage_node(const Consts<T>& k, const State<T, T>
   if (!FIRST) cp_async(st + (Q + 3) * kBlock, s.phi_in + nu, pol);
 }
 
-// STAGED: g, u and the previous phi come from the node's cp.async staging
-// slot `st` (word j at st[j * kBlock]); otherwise they are loaded here.
-template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1, bool STAGED, bool STORE_PHI, bool GMU,
-          bool MAP, typename PhiAt, typename SolidAt, typename RefAt>
-__device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S>& s, int n, const Nbr& nb,
-                                            uint8_t c, T phi, PhiAt phi_at, SolidAt solid_at, RefAt ref_at,
-                                            const Pol& pol, const T* st) {
+__device__ __forceinline__ void decode(const FastDiv& dz, const FastDiv& dy, int n, int nz, int ny, int& ix,
+                                       int& iy, int& iz) {
+  const int t = (int)dz.div((unsigned)n);
+  iz = n - t * nz;
+  ix = (int)dy.div((unsigned)t);
+  iy = t - ix * ny;
+}
+
+// How the update of a node reaches the grid's arrays.  Each accessor gives the
+// phi stencil of this step (phi_at), the solid test of a neighbour, the
+// reconstructed g and f, u and phi of the last step, and the stores.
+//
+// NodeAt: any node, through its Nbr offsets (MAP: the storage element map of k).
+template <typename T, typename S, bool RAW, bool MAP>
+struct NodeAt {
   using IO = PopIO<T, S>;
-  constexpr bool IMM = IO::kDev;
-  const LatK<T, IMM> L{k};
+  const Consts<T>& k;
+  const State<T, S>& s;
+  const Pol& pol;
+  const Nbr nb;
+  const int n;
+  const unsigned Np, e;  // component stride; the node's storage element (f, g, u, phi)
+  __device__ __forceinline__ NodeAt(const Consts<T>& k_, const State<T, S>& s_, const Pol& p_, const Nbr& nb_, int n_)
+      : k(k_), s(s_), pol(p_), nb(nb_), n(n_), Np((unsigned)k_.Np), e(MAP ? sidx(k_, n_) : (unsigned)n_) {}
+  __device__ __forceinline__ int nbr(int q) const { return nb.at(n, ex(q), ey(q), ez(q)); }
+  __device__ __forceinline__ unsigned el(int m) const { return MAP ? sidx(k, m) : (unsigned)m; }
+  __device__ __forceinline__ T phi_at(int q) const { return ld_pol(s.phi_out + el(nbr(q)), pol.keep); }
+  __device__ __forceinline__ bool solid_at(int q) const { return (s.cls[nbr(q)] & kSolid) != 0; }
+  __device__ __forceinline__ void load_g(T (&g)[Q], uint8_t c, T eps) const {
+    fetch_pop<T, S, RAW, false, false, true, MAP>(g, k, s.gin, s.phi_in, n, (size_t)k.N, nb, c, eps, T(1), pol.once);
+  }
+  __device__ __forceinline__ void load_f(T (&f)[Q], uint8_t c, T eps) const {
+    fetch_f<T, S, RAW, true, MAP>(f, k, s, n, (size_t)k.N, nb, c, eps, pol.same);
+  }
+  __device__ __forceinline__ T u_old(int d) const { return ld_pol(s.u + (d * Np + e), pol.once); }
+  __device__ __forceinline__ T phi_old() const { return ld_pol(s.phi_in + e, pol.once); }
+  __device__ __forceinline__ T ref_at(int q) const { return phi_at(q); }
+  __device__ __forceinline__ void st_g(int q, T v) const { st_pol(s.gout + (q * Np + e), IO::st_g(v, q, k), pol.once); }
+  __device__ __forceinline__ void st_f(int q, T v) const {
+    st_pol(s.fout + (q * Np + e), IO::st_f(v, q, IO::kDev ? ref_at(q) : T(0), k), pol.once);
+  }
+  __device__ __forceinline__ void st_u(int d, T v) const { st_pol(s.u + (d * Np + e), v, pol.once); }
+  __device__ __forceinline__ void st_s(int d, T v) const {
+    st_pol(reinterpret_cast<T*>(s.fout) + (d * Np + e), v, pol.once);
+  }
+};
+
+// NodeIn: a node with 1 <= x <= nx - 2 of a grid in the linear layout, one or
+// more per thread block with the whole block inside that range.  The plane
+// shift of a step in x is then +-ny nz for every thread, so the arrays'
+// component and plane bases are the same for the block and the nine in-plane
+// neighbours (periodic in y and z) are nine 32-bit offsets of the thread,
+// shared by every population and stencil load: one address register and no
+// address arithmetic per load.  (19 N < 2^31 elements, so the byte offsets
+// of one component stay below 2^32.)
+template <typename T, typename S>
+struct NodeIn {
+  using IO = PopIO<T, S>;
+  const Consts<T>& k;
+  const State<T, S>& s;
+  const Pol& pol;
+  const int n;
+  const unsigned Np, P;  // component stride, nodes of a plane
+  unsigned o[3][3];       // in-plane neighbour (dy, dz) of the node
+  __device__ __forceinline__ NodeIn(const Consts<T>& k_, const State<T, S>& s_, const Pol& p_, int n_, int iy, int iz)
+      : k(k_), s(s_), pol(p_), n(n_), Np((unsigned)k_.Np), P((unsigned)(k_.ny * k_.nz)) {
+    const int row[3] = {iy == 0 ? n + (k.ny - 1) * k.nz : n - k.nz, n, iy == k.ny - 1 ? n - (k.ny - 1) * k.nz : n + k.nz};
+    const int dz[3] = {iz == 0 ? k.nz - 1 : -1, 0, iz == k.nz - 1 ? 1 - k.nz : 1};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) o[a][b] = (unsigned)(row[a] + dz[b]);
+  }
+  __device__ __forceinline__ T phi_at(int q) const {
+    return ld_pol(s.phi_out + (ex(q) * P + o[ey(q) + 1][ez(q) + 1]), pol.keep);
+  }
+  __device__ __forceinline__ bool solid_at(int q) const {
+    return (s.cls[ex(q) * P + o[ey(q) + 1][ez(q) + 1]] & kSolid) != 0;
+  }
+  __device__ __forceinline__ T own_g(int q) const {
+    return IO::ld_g(ld_pol(s.gin + (q * Np + o[1][1]), pol.once), q, k);
+  }
+  __device__ __forceinline__ void load_g(T (&g)[Q], uint8_t c, T eps) const {
+    if (c & kSolid) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) g[q] = own_g(opp(q));
+      return;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      g[q] = IO::ld_g(ld_pol(s.gin + (q * Np - ex(q) * P + o[1 - ey(q)][1 - ez(q)]), pol.once), q, k);
+    if (c & kPartial) {
+      const T one_m = sub_rn(T(1), eps);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) g[q] = fma_(one_m, g[q], mul_rn(eps, own_g(opp(q))));
+    }
+  }
+  __device__ __forceinline__ void load_f(T (&f)[Q], uint8_t c, T eps) const {
+    int ix, iy, iz;
+    decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+    const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
+    fetch_f<T, S, false, true, false>(f, k, s, n, (size_t)k.N, nb, c, eps, pol.same);
+  }
+  __device__ __forceinline__ T u_old(int d) const { return ld_pol(s.u + (d * Np + o[1][1]), pol.once); }
+  __device__ __forceinline__ T phi_old() const { return ld_pol(s.phi_in + o[1][1], pol.once); }
+  __device__ __forceinline__ void st_g(int q, T v) const {
+    st_pol(s.gout + (q * Np + o[1][1]), IO::st_g(v, q, k), pol.once);
+  }
+  __device__ __forceinline__ void st_f(int q, T v) const {
+    st_pol(s.fout + (q * Np + o[1][1]), IO::st_f(v, q, IO::kDev ? phi_at(q) : T(0), k), pol.once);
+  }
+  __device__ __forceinline__ void st_u(int d, T v) const { st_pol(s.u + (d * Np + o[1][1]), v, pol.once); }
+  __device__ __forceinline__ void st_s(int d, T v) const {
+    st_pol(reinterpret_cast<T*>(s.fout) + (d * Np + o[1][1]), v, pol.once);
+  }
+};
+
+// f_eq and interface source of the phase-field collision, one opposite pair
+// (q, opp q) at a time:
+//   w_q p (1 - u.u / (2 cs2) + ec^2 / 2) + w_q p ec + w_q c e_q.S,   ec = e_q.u / cs2,
+// with p = omega_f phi, S the interface source and c = (1 - 1 / (2 tau_f)) / cs2: all of
+// the post-collision populations when tau_f == 1.  ob = 1 - u.u / (2 cs2).
+// Explicitly rounded: every kernel that evaluates it gives the same bits.
+// (float64 folds p u / cs2 and c S into one vector and the weight into the last
+// operations.)
+template <typename T>
+struct FEval {
+  T wa_A, wd_A, wa_H, wd_H, wa_p, wd_p, f0, ca, cd, sx, sy, sz;
+  // p, u / cs2, ob, S
+  __device__ __forceinline__ FEval(const Consts<T>& k, T p, T ux, T uy, T uz, T ob, T s0, T s1, T s2) {
+    constexpr T w0 = Lat<T>::w(0), wa = Lat<T>::w(1), wd = Lat<T>::w(7);
+    wa_p = mul_rn(p, wa);
+    wd_p = mul_rn(p, wd);
+    f0 = mul_rn(mul_rn(p, w0), ob);
+    wa_H = mul_rn(T(0.5), wa_p);
+    wd_H = mul_rn(T(0.5), wd_p);
+    wa_A = mul_rn(wa_p, ob);
+    wd_A = mul_rn(wd_p, ob);
+    if constexpr (sizeof(T) == 8) {
+      sx = fma_(p, ux, mul_rn(k.src_c, s0));
+      sy = fma_(p, uy, mul_rn(k.src_c, s1));
+      sz = fma_(p, uz, mul_rn(k.src_c, s2));
+    } else {
+      ca = k.wac3[1];
+      cd = k.wac3[7];
+      sx = s0;
+      sy = s1;
+      sz = s2;
+    }
+  }
+  // the pair (q, opp q), ec = e_q.u / cs2
+  __device__ __forceinline__ void pair(int q, T ec, T& fq, T& fp) const {
+    const bool ax = q <= 6;
+    const T es = edot(q, sx, sy, sz);
+    const T e = fma_(mul_rn(ax ? wa_H : wd_H, ec), ec, ax ? wa_A : wd_A);
+    if constexpr (sizeof(T) == 8) {
+      const T w = Lat<T>::w(q);
+      fq = fma_(w, es, e);
+      fp = fma_(-w, es, e);
+    } else {
+      const T o = fma_(ax ? wa_p : wd_p, ec, mul_rn(ax ? ca : cd, es));
+      fq = add_rn(e, o);
+      fp = sub_rn(e, o);
+    }
+  }
+};
+
+// The update of one node (lbm/fe_ac_solver.py:392-530): stencils, chemical
+// potential, wetting, pressure, stress, forces, velocity, Allen-Cahn source
+// and both BGK collisions; writes f, g, u.  c, phi: the node's class and its
+// phi of this step.  Every operation is explicitly rounded, with the fused
+// multiply-adds written out, so that all kernels that step a node (alone, in a
+// batch, tiled, whatever their addressing) give the same bits.  In float32 and
+// half storage the places of the fused operations are fixed: FB (the first
+// step, and every step of the half form) fuses u.u / (2 cs2) into P - b and
+// 1 - b.  float64 has freer ones with fewer operations (LEAN).
+// OMEGA1: tau_f == 1 (the reference's default tau_h = 1.0), where the
+// phase-field BGK collision f - (f - f_eq) + src is f_eq + src and the
+// pre-collision f is not read.  SOUT (with OMEGA1): f is not written either, but
+// the source vector S from which, with phi and u, FEval gives it back.
+template <typename T, typename S, bool FIRST, bool OMEGA1, bool GMU, bool SOUT, typename Node>
+__device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S>& s, const Node& a, uint8_t c, T phi) {
+  constexpr bool LEAN = sizeof(T) == 8;
+  constexpr bool HALF = PopIO<T, S>::kDev;
+  constexpr bool FB = FIRST || HALF;
+  using L = Lat<T>;
+  const int n = a.n;
   const size_t N = (size_t)k.N;
-  // nu: the node's storage element (f, g, u, phi); nn: its node index (node-order arrays)
-  const unsigned Nu = (unsigned)k.Np, nu = MAP ? sidx(k, n) : (unsigned)n, nn = (unsigned)n;
 
   // 2. first the stencil: gradient and laplacian with the ghost-node wetting values
   T ps[Q];
 #pragma unroll
-  for (int q = 1; q < Q; ++q) ps[q] = phi_at(q);
+  for (int q = 1; q < Q; ++q) ps[q] = a.phi_at(q);
   T gx, gy, gz, lap;
-  grad_lap<T, true, State<T, S>, SolidAt, true, IMM>(k, s, n, c, phi, ps, solid_at, gx, gy, gz, lap);
+  grad_lap<T, true>(k, s, n, c, phi, ps, [&](int q) { return a.solid_at(q); }, gx, gy, gz, lap);
 
   // then g (pulled), u and phi of the last step.  Loading them after the
   // stencil keeps the 18 stencil values and the 19 populations from being
-  // live at once (fewer registers, no spills; measured 157 -> 137 us per
-  // update launch on the 150x150x107 case; moving the density, chemical
-  // potential and wall correction ahead of these loads as well measured 143).
+  // live at once (fewer registers, no spills).
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T g[Q];
-  T uo0, uo1, uo2, pp;
-  if constexpr (STAGED) {
-    const T* gin = reinterpret_cast<const T*>(s.gin);
-    if (!RAW && (c & kSolid)) {
-      // bounce-back: the node's own opposite values, not the staged pulled ones
-#pragma unroll
-      for (int q = 0; q < Q; ++q) g[q] = ldg(gin + (opp(q) * Nu + nu));
-    } else {
-#pragma unroll
-      for (int q = 0; q < Q; ++q) g[q] = st[q * kBlock];
-    }
-    if (!RAW && (c & kPartial)) {
-      const T one_m = T(1) - eps;
-#pragma unroll
-      for (int q = 0; q < Q; ++q) g[q] = one_m * g[q] + eps * ldg(gin + (opp(q) * Nu + nu));
-    }
-    uo0 = st[Q * kBlock];
-    uo1 = st[(Q + 1) * kBlock];
-    uo2 = st[(Q + 2) * kBlock];
-    pp = FIRST ? T(0) : st[(Q + 3) * kBlock];
-  } else {
-    fetch_pop<T, S, RAW, false, false, true, MAP>(g, k, s.gin, s.phi_in, n, N, nb, c, eps, T(1), pol.once);
-    uo0 = ld_pol(s.u + nu, pol.once);
-    uo1 = ld_pol(s.u + (Nu + nu), pol.once);
-    uo2 = ld_pol(s.u + (2 * Nu + nu), pol.once);
-    pp = FIRST ? T(0) : ld_pol(s.phi_in + nu, pol.once);
-  }
+  a.load_g(g, c, eps);
+  const T uo0 = a.u_old(0), uo1 = a.u_old(1), uo2 = a.u_old(2);
+  const T pp = FIRST ? T(0) : a.phi_old();
 
-  const T rho = fma_(phi, k.rho_l, (T(1) - phi) * k.rho_g);
-  const T rho_eff = rho < k.rho_floor ? k.rho_floor : rho;
+  const T omphi = sub_rn(T(1), phi);
+  const T rho = fma_(phi, k.rho_l, mul_rn(omphi, k.rho_g));
   // with a chemical-potential gradient term, mu of every node comes from k_mu
   // (the same arithmetic), so that the node's own mu and its neighbours' agree
-  const T mu = GMU ? ld_pol(s.mu + n, pol.keep) : chem_pot(k, c, phi, lap);
+  const T mu = GMU ? ld_pol(s.mu + n, a.pol.keep) : chem_pot(k, c, phi, lap);
 
   // geometric contact-angle gradient correction (fe_wetting.py:448-539).  The
   // wall normal is zero away from boundary nodes, where the correction is the
@@ -575,25 +794,26 @@ __device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S
   if (k.geometric && (c & kBoundary)) {
     const T n0 = (T)s.wn[n], n1 = (T)s.wn[N + n], n2 = (T)s.wn[2 * N + n];
     const T gn = add_rn(add_rn(mul_rn(n0, gx), mul_rn(n1, gy)), mul_rn(n2, gz));
-    const T tx = gx - mul_rn(gn, n0), ty = gy - mul_rn(gn, n1), tz = gz - mul_rn(gn, n2);
-    T tm = sqrt_mag<IMM>(add_rn(add_rn(mul_rn(tx, tx), mul_rn(ty, ty)), mul_rn(tz, tz)));
+    const T tx = sub_rn(gx, mul_rn(gn, n0)), ty = sub_rn(gy, mul_rn(gn, n1)), tz = sub_rn(gz, mul_rn(gn, n2));
+    T tm = sqrt_rn(add_rn(add_rn(mul_rn(tx, tx), mul_rn(ty, ty)), mul_rn(tz, tz)));
     tm = tm < T(1e-10) ? T(1e-10) : tm;
-    T gd = mul_rn(-tm, k.cos_t) / k.sin_t;
+    T gd = div_rn(mul_rn(-tm, k.cos_t), k.sin_t);
     // scalar amplification, or a per-node field active where alpha > 1 (fe_wetting.py:503-512)
-    T a = k.amp;
+    T al = k.amp;
     bool amp_on = k.amp_active;
     if (s.amp) {
-      a = s.amp[n];
-      amp_on = a > T(1);
+      al = s.amp[n];
+      amp_on = al > T(1);
     }
-    if (amp_on) gd = add_rn(gn, mul_rn(gd - gn, a));
+    if (amp_on) gd = add_rn(gn, mul_rn(sub_rn(gd, gn), al));
     const T cx = add_rn(tx, mul_rn(gd, n0)), cy = add_rn(ty, mul_rn(gd, n1)), cz = add_rn(tz, mul_rn(gd, n2));
-    const T gm = sqrt_mag<IMM>(add_rn(add_rn(mul_rn(gx, gx), mul_rn(gy, gy)), mul_rn(gz, gz)));
-    if (gm > T(1e-6)) {
+    // |grad| > 1e-6, without the square root: the largest value whose rounded root is at most 1e-6
+    constexpr T g2_min = sizeof(T) == 8 ? T(0x1.19799812dea11p-40) : T(0x1.19799ap-40);
+    if (add_rn(add_rn(mul_rn(gx, gx), mul_rn(gy, gy)), mul_rn(gz, gz)) > g2_min) {
       const T bl = k.ww[c >> kWwShift];
-      gx = add_rn(gx, mul_rn(bl, cx - gx));
-      gy = add_rn(gy, mul_rn(bl, cy - gy));
-      gz = add_rn(gz, mul_rn(bl, cz - gz));
+      gx = add_rn(gx, mul_rn(bl, sub_rn(cx, gx)));
+      gy = add_rn(gy, mul_rn(bl, sub_rn(cy, gy)));
+      gz = add_rn(gz, mul_rn(bl, sub_rn(cz, gz)));
     }
   }
 
@@ -607,35 +827,51 @@ __device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S
   T sp[9], dp[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
-    sp[i] = g[pair_first(i)] + g[opp(pair_first(i))];
-    dp[i] = g[pair_first(i)] - g[opp(pair_first(i))];
+    sp[i] = add_rn(g[pair_first(i)], g[opp(pair_first(i))]);
+    dp[i] = sub_rn(g[pair_first(i)], g[opp(pair_first(i))]);
   }
-  T P = g[0];
+  const T sxy_ = add_rn(sp[3], sp[4]), sxz_ = add_rn(sp[5], sp[6]), syz_ = add_rn(sp[7], sp[8]);
+  T P;
+  if constexpr (LEAN) {
+    P = add_rn(add_rn(g[0], add_rn(add_rn(sp[0], sp[1]), sp[2])), add_rn(add_rn(sxy_, sxz_), syz_));
+  } else {
+    P = g[0];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) P = P + sp[i];
-  T sxx, syy, szz, sxy, sxz, syz;
-  {
-    const T pc = P * L.cs2();
-    sxx = fma_(-uo0, uo0, (sp[0] + (sp[3] + sp[4]) + (sp[5] + sp[6])) - pc);
-    syy = fma_(-uo1, uo1, (sp[1] + (sp[3] + sp[4]) + (sp[7] + sp[8])) - pc);
-    szz = fma_(-uo2, uo2, (sp[2] + (sp[5] + sp[6]) + (sp[7] + sp[8])) - pc);
-    sxy = fma_(-uo0, uo1, sp[3] - sp[4]);
-    sxz = fma_(-uo0, uo2, sp[5] - sp[6]);
-    syz = fma_(-uo1, uo2, sp[7] - sp[8]);
+    for (int i = 0; i < 9; ++i) P = add_rn(P, sp[i]);
   }
 
   // 5. forces (Fakhari 2017, :416-439)
-  T F0 = mu * gx, F1 = mu * gy, F2 = mu * gz;
-  if (k.stab_mode <= 1) {
-    const T fp = ((-P) * k.drho) * L.cs2();
-    F0 = fma_(fp, gx, F0);
-    F1 = fma_(fp, gy, F1);
-    F2 = fma_(fp, gz, F2);
+  T F0, F1, F2;
+  if constexpr (LEAN) {
+    const T m = k.stab_mode <= 1 ? fma_(-P, k.drho_cs2, mu) : mu;
+    F0 = mul_rn(m, gx);
+    F1 = mul_rn(m, gy);
+    F2 = mul_rn(m, gz);
+  } else {
+    F0 = mul_rn(mu, gx);
+    F1 = mul_rn(mu, gy);
+    F2 = mul_rn(mu, gz);
+    if (k.stab_mode <= 1) {
+      const T fp = mul_rn(mul_rn(-P, k.drho), L::cs2());
+      F0 = fma_(fp, gx, F0);
+      F1 = fma_(fp, gy, F1);
+      F2 = fma_(fp, gz, F2);
+    }
   }
   if (k.stab_mode == 0) {
-    F0 = fma_(k.visc * fma_(sxz, gz, fma_(sxy, gy, sxx * gx)), k.drho, F0);
-    F1 = fma_(k.visc * fma_(syz, gz, fma_(syy, gy, sxy * gx)), k.drho, F1);
-    F2 = fma_(k.visc * fma_(szz, gz, fma_(syz, gy, sxz * gx)), k.drho, F2);
+    auto diag = [&](T u, T sum) { return fma_(-u, u, fma_(-P, L::cs2(), sum)); };
+    const T sxx = diag(uo0, LEAN ? add_rn(sp[0], add_rn(sxy_, sxz_)) : add_rn(add_rn(sp[0], sxy_), sxz_));
+    const T syy = diag(uo1, LEAN ? add_rn(sp[1], add_rn(sxy_, syz_)) : add_rn(add_rn(sp[1], sxy_), syz_));
+    const T szz = diag(uo2, LEAN ? add_rn(sp[2], add_rn(sxz_, syz_)) : add_rn(add_rn(sp[2], sxz_), syz_));
+    const T sxy = fma_(-uo0, uo1, sub_rn(sp[3], sp[4]));
+    const T sxz = fma_(-uo0, uo2, sub_rn(sp[5], sp[6]));
+    const T syz = fma_(-uo1, uo2, sub_rn(sp[7], sp[8]));
+    const T v0 = fma_(sxz, gz, fma_(sxy, gy, mul_rn(sxx, gx)));
+    const T v1 = fma_(syz, gz, fma_(syy, gy, mul_rn(sxy, gx)));
+    const T v2 = fma_(szz, gz, fma_(syz, gy, mul_rn(sxz, gx)));
+    F0 = LEAN ? fma_(k.visc_drho, v0, F0) : fma_(mul_rn(k.visc, v0), k.drho, F0);
+    F1 = LEAN ? fma_(k.visc_drho, v1, F1) : fma_(mul_rn(k.visc, v1), k.drho, F1);
+    F2 = LEAN ? fma_(k.visc_drho, v2, F2) : fma_(mul_rn(k.visc, v2), k.drho, F2);
   }
   if (k.has_gforce) {
     F0 = fma_(k.gforce[0], rho, F0);
@@ -644,49 +880,73 @@ __device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S
   }
 
   // 6. velocity (:442-447)
-  T u0, u1, u2;
-  {
-    const T hr = T(0.5) * rcp(rho_eff);
-    u0 = fma_(F0, hr, dp[0] + (dp[3] - dp[4]) + (dp[5] - dp[6]));
-    u1 = fma_(F1, hr, dp[1] + (dp[3] + dp[4]) + (dp[7] - dp[8]));
-    u2 = fma_(F2, hr, dp[2] + (dp[5] + dp[6]) + (dp[7] + dp[8]));
-    if (c & kSolid) u0 = u1 = u2 = T(0);
+  // 1 / rho_eff and 1 / (rho_eff cs2); in the gas and half of the interface rho_eff is the floor
+  T rr = k.inv_floor, rc = k.inv_floor_cs2;
+  if (!(rho < k.rho_floor)) {
+    rr = rcp_rn(rho);
+    rc = LEAN ? mul_rn(rr, L::inv_cs2()) : rcp_rn(mul_rn(rho, L::cs2()));
   }
-  const T b = fma_(u2, u2, fma_(u1, u1, u0 * u0)) * L.inv_two_cs2();
+  const T hr = mul_rn(T(0.5), rr);
+  T u0 = fma_(F0, hr, add_rn(add_rn(dp[0], sub_rn(dp[3], dp[4])), sub_rn(dp[5], dp[6])));
+  T u1 = fma_(F1, hr, add_rn(add_rn(dp[1], add_rn(dp[3], dp[4])), sub_rn(dp[7], dp[8])));
+  T u2 = fma_(F2, hr, add_rn(add_rn(dp[2], add_rn(dp[5], dp[6])), add_rn(dp[7], dp[8])));
+  if (c & kSolid) u0 = u1 = u2 = T(0);
+  a.st_u(0, u0);
+  a.st_u(1, u1);
+  a.st_u(2, u2);
+  const T usq = fma_(u2, u2, fma_(u1, u1, mul_rn(u0, u0)));
+  const T b = mul_rn(usq, L::inv_two_cs2());
+  const T Pb = FB ? fma_(-usq, L::inv_two_cs2(), P) : sub_rn(P, b);
 
   // 7. Allen-Cahn source (:450-494)
-  T S0, S1, S2;
-  {
-    T d0 = T(0), d1 = T(0), d2 = T(0);
-    if (!FIRST) {
-      d0 = fma_(phi, u0, -pp * uo0);
-      d1 = fma_(phi, u1, -pp * uo1);
-      d2 = fma_(phi, u2, -pp * uo2);
-    }
-    T gm = sqrt_mag<IMM>(fma_(gz, gz, fma_(gy, gy, gx * gx)));
-    gm = gm < T(1e-10) ? T(1e-10) : gm;
-    const T lam = ((T(4) * phi) * (T(1) - phi)) * k.inv_W;
-    T cl = L.cs2() * lam * k.ac_scale * rcp(gm);
-    if (k.wetting) cl = cl * (T(1) - k.sharpen_reduce * k.ww[c >> kWwShift]);
-    if constexpr (GMU) {
-      // grad mu of this node (k_gradmu)
-      const T mx = ld_pol(s.gmu + nn, pol.once), my = ld_pol(s.gmu + (Nu + nn), pol.once),
-              mz = ld_pol(s.gmu + (2 * Nu + nn), pol.once);
-      if (k.gmu_mode == kGmuCH) {
-        // Cahn-Hilliard: d(phi u) + M (grad mu - grad phi) tau_f / (tau_f - 1/2)  (:457-461)
-        S0 = d0 + (k.mob * (mx - gx)) * k.guo;
-        S1 = d1 + (k.mob * (my - gy)) * k.guo;
-        S2 = d2 + (k.mob * (mz - gz)) * k.guo;
+  T S0 = T(0), S1 = T(0), S2 = T(0);
+  if (!FIRST) {
+    S0 = fma_(phi, u0, mul_rn(-pp, uo0));
+    S1 = fma_(phi, u1, mul_rn(-pp, uo1));
+    S2 = fma_(phi, u2, mul_rn(-pp, uo2));
+  }
+  T mx = T(0), my = T(0), mz = T(0);
+  if constexpr (GMU) {
+    // grad mu of this node (k_gradmu)
+    const unsigned Np = (unsigned)k.Np;
+    mx = ld_pol(s.gmu + n, a.pol.once);
+    my = ld_pol(s.gmu + (Np + n), a.pol.once);
+    mz = ld_pol(s.gmu + (2 * Np + n), a.pol.once);
+  }
+  if (GMU && k.gmu_mode == kGmuCH) {
+    // Cahn-Hilliard: d(phi u) + M (grad mu - grad phi) tau_f / (tau_f - 1/2)  (:457-461)
+    S0 = fma_(mul_rn(k.mob, sub_rn(mx, gx)), k.guo, S0);
+    S1 = fma_(mul_rn(k.mob, sub_rn(my, gy)), k.guo, S1);
+    S2 = fma_(mul_rn(k.mob, sub_rn(mz, gz)), k.guo, S2);
+  } else {
+    // sharpening along grad / max(|grad|, 1e-10)
+    const T g2 = fma_(gz, gz, fma_(gy, gy, mul_rn(gx, gx)));
+    // 1 / max(|grad|, 1e-10); below 1e-21 (most of the gas) |grad|^2 needs no square root
+    T rg = T(1) / T(1e-10);
+    if (!(g2 < T(1e-21))) {
+      if constexpr (LEAN) {
+        if (!(g2 <= T(1e-20))) rg = rsqrt(g2);
       } else {
-        // Allen-Cahn with the mu drive: sharpening + d(phi u) + mu_drive M grad mu  (:484-486)
-        S0 = fma_(cl, gx, d0) + k.mu_drive_a * mx;
-        S1 = fma_(cl, gy, d1) + k.mu_drive_a * my;
-        S2 = fma_(cl, gz, d2) + k.mu_drive_a * mz;
+        const T gm = sqrt_rn(g2);
+        rg = rcp_rn(gm < T(1e-10) ? T(1e-10) : gm);
       }
+    }
+    T cl;
+    if constexpr (LEAN) {
+      cl = mul_rn(mul_rn(mul_rn(k.sharp, phi), omphi), rg);
     } else {
-      S0 = fma_(cl, gx, d0);
-      S1 = fma_(cl, gy, d1);
-      S2 = fma_(cl, gz, d2);
+      const T lam = mul_rn(mul_rn(mul_rn(T(4), phi), omphi), k.inv_W);
+      cl = mul_rn(mul_rn(mul_rn(L::cs2(), lam), k.ac_scale), rg);
+    }
+    if (k.wetting) cl = mul_rn(cl, fma_(-k.sharpen_reduce, k.ww[c >> kWwShift], T(1)));
+    S0 = fma_(cl, gx, S0);
+    S1 = fma_(cl, gy, S1);
+    S2 = fma_(cl, gz, S2);
+    if constexpr (GMU) {
+      // the mu drive: + mu_drive M grad mu  (:484-486)
+      S0 = fma_(k.mu_drive_a, mx, S0);
+      S1 = fma_(k.mu_drive_a, my, S1);
+      S2 = fma_(k.mu_drive_a, mz, S2);
     }
   }
 
@@ -694,72 +954,83 @@ __device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S
   // With ec = e_q.u / cs2 (odd in q) the equilibria split into a part even in
   // q and a part odd in q:
   //   g_eq_q = w (P - b + ec^2/2) + w ec,   f_eq_q = phi w (1 - b + ec^2/2) + phi w ec,
-  // and the forcing and Allen-Cahn source terms are odd, so each pair costs
-  // one even and one odd term per lattice.
+  // and the forcing and Allen-Cahn source terms are odd (f: FEval).
   T om;
   if (k.tau_const) {
     om = k.omega_g;
   } else {
-    const T eta = phi * k.rho_l * k.tl_m + (T(1) - phi) * k.rho_g * k.tg_m;
-    const T rden = phi * k.rho_l + (T(1) - phi) * k.rho_g;
-    om = rcp(T(0.5) + eta / rden);
+    const T gas = mul_rn(omphi, k.rho_g);
+    const T eta = fma_(mul_rn(phi, k.rho_l), k.tl_m, mul_rn(gas, k.tg_m));
+    om = rcp_rn(add_rn(T(0.5), div_rn(eta, fma_(phi, k.rho_l, gas))));
   }
-  const T omo = T(1) - om;
-  const T nsd = (T(1) - om * T(0.5)) * rcp(rho_eff * L.cs2());
-  const T Pb = P - b;
-  const T omb = T(1) - b;
-  const T pf = OMEGA1 ? phi : k.omega_f * phi;  // omega_f phi
-  const T u3x = u0 * L.inv_cs2(), u3y = u1 * L.inv_cs2(), u3z = u2 * L.inv_cs2();
-  T f[Q];
-  if (!OMEGA1) fetch_f<T, S, RAW, true, MAP>(f, k, s, n, N, nb, c, eps, pol.same);
-  auto store_g = [&](int q, T v) { st_pol(s.gout + (q * Nu + nu), IO::st_g(v, q, k), pol.once); };
-  auto store_f = [&](int q, T v) {
-    st_pol(s.fout + (q * Nu + nu), IO::st_f(v, q, IO::kDev ? ref_at(q) : T(0), k), pol.once);
+  const T omo = sub_rn(T(1), om);
+  const T nsd = mul_rn(fma_(om, T(-0.5), T(1)), rc);
+  const T u3x = mul_rn(u0, L::inv_cs2()), u3y = mul_rn(u1, L::inv_cs2()), u3z = mul_rn(u2, L::inv_cs2());
+  // e_q.u / cs2; the half form's first step fuses the x term of the diagonals that have one
+  auto ecdot = [&](int q) {
+    if (HALF && FIRST && q > 6 && ex(q) != 0)
+      return fma_(ex(q) > 0 ? u0 : -u0, L::inv_cs2(),
+                  ey(q) != 0 ? (ey(q) > 0 ? u3y : -u3y) : (ez(q) > 0 ? u3z : -u3z));
+    return edot(q, u3x, u3y, u3z);
   };
   {
-    const T ow = om * L.w(0);
-    store_g(0, fma_(omo, g[0], ow * Pb));
-    const T pw = pf * L.w(0);
-    const T f0 = pw * omb;
-    store_f(0, OMEGA1 ? f0 : fma_(T(1) - k.omega_f, f[0], f0));
-  }
-  // per weight class (axis pairs i < 3, diagonal pairs i >= 3): omega w,
-  // omega w / 2, omega w (P - b), nsd w; omega_f phi w, its half, omega_f phi w (1 - b)
-  const T wa = L.w(1), wd = L.w(7);
-  const T owa = om * wa, owd = om * wd;
-  const T howa = T(0.5) * owa, howd = T(0.5) * owd;
-  const T obpa = owa * Pb, obpd = owd * Pb;
-  const T nwa = nsd * wa, nwd = nsd * wd;
-  const T pwa = pf * wa, pwd = pf * wd;
-  const T hpwa = T(0.5) * pwa, hpwd = T(0.5) * pwd;
-  const T pwba = pwa * omb, pwbd = pwd * omb;
-  const T aca = k.wac3[1], acd = k.wac3[7];
+    const T ow0 = mul_rn(om, L::w(0)), owa = mul_rn(om, L::w(1)), owd = mul_rn(om, L::w(7));
+    const T wa_P = mul_rn(owa, Pb), wd_P = mul_rn(owd, Pb);
+    const T wa_h = mul_rn(T(0.5), owa), wd_h = mul_rn(T(0.5), owd);
+    const T wa_n = mul_rn(nsd, L::w(1)), wd_n = mul_rn(nsd, L::w(7));
+    // LEAN: the odd part is w e_q.V
+    const T V0 = fma_(om, u3x, mul_rn(nsd, F0)), V1 = fma_(om, u3y, mul_rn(nsd, F1)),
+            V2 = fma_(om, u3z, mul_rn(nsd, F2));
+    a.st_g(0, fma_(omo, g[0], mul_rn(ow0, Pb)));
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const int q = pair_first(i), p = opp(q);
-    const bool ax = i < 3;
-    const T ec = edot(q, u3x, u3y, u3z);
-    // hydrodynamic pair
-    const T ge = fma_((ax ? howa : howd) * ec, ec, ax ? obpa : obpd);
-    const T go = fma_(ax ? owa : owd, ec, (ax ? nwa : nwd) * edot(q, F0, F1, F2));
-    store_g(q, fma_(omo, g[q], ge + go));
-    store_g(p, fma_(omo, g[p], ge - go));
-    // phase-field pair
-    const T fe = fma_((ax ? hpwa : hpwd) * ec, ec, ax ? pwba : pwbd);
-    const T fo = fma_(ax ? pwa : pwd, ec, (ax ? aca : acd) * edot(q, S0, S1, S2));
-    if (OMEGA1) {
-      store_f(q, fe + fo);
-      store_f(p, fe - fo);
-    } else {
-      const T omf = T(1) - k.omega_f;
-      store_f(q, fma_(omf, f[q], fe + fo));
-      store_f(p, fma_(omf, f[p], fe - fo));
+    for (int i = 0; i < 9; ++i) {
+      const int q = pair_first(i), p = opp(q);
+      const bool ax = i < 3;
+      const T ec = ecdot(q);
+      const T ge = fma_(mul_rn(ax ? wa_h : wd_h, ec), ec, ax ? wa_P : wd_P);
+      if constexpr (LEAN) {
+        const T ev = edot(q, V0, V1, V2), w = L::w(q);
+        a.st_g(q, fma_(omo, g[q], fma_(w, ev, ge)));
+        a.st_g(p, fma_(omo, g[p], fma_(-w, ev, ge)));
+      } else {
+        const T go = fma_(ax ? owa : owd, ec, mul_rn(ax ? wa_n : wd_n, edot(q, F0, F1, F2)));
+        a.st_g(q, fma_(omo, g[q], add_rn(ge, go)));
+        a.st_g(p, fma_(omo, g[p], sub_rn(ge, go)));
+      }
     }
   }
-  st_pol(s.u + nu, u0, pol.once);
-  st_pol(s.u + (Nu + nu), u1, pol.once);
-  st_pol(s.u + (2 * Nu + nu), u2, pol.once);
-  if (STORE_PHI) st_pol(s.phi_out + nu, phi, pol.once);
+  if constexpr (SOUT) {
+    static_assert(OMEGA1 && !FIRST, "f follows from phi, u and S when tau_f == 1");
+    a.st_s(0, S0);
+    a.st_s(1, S1);
+    a.st_s(2, S2);
+    return;
+  }
+  const T pf = OMEGA1 ? phi : mul_rn(k.omega_f, phi);
+  const FEval<T> fe(k, pf, u3x, u3y, u3z, FB ? fma_(-usq, L::inv_two_cs2(), T(1)) : sub_rn(T(1), b), S0, S1, S2);
+  if constexpr (OMEGA1) {
+    a.st_f(0, fe.f0);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      T fq, fp;
+      fe.pair(pair_first(i), ecdot(pair_first(i)), fq, fp);
+      a.st_f(pair_first(i), fq);
+      a.st_f(opp(pair_first(i)), fp);
+    }
+  } else {
+    T f[Q];
+    a.load_f(f, c, eps);
+    const T omf = sub_rn(T(1), k.omega_f);
+    a.st_f(0, fma_(omf, f[0], fe.f0));
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const int q = pair_first(i), p = opp(q);
+      T fq, fp;
+      fe.pair(q, ecdot(q), fq, fp);
+      a.st_f(q, fma_(omf, f[q], fq));
+      a.st_f(p, fma_(omf, f[p], fp));
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -801,7 +1072,8 @@ __device__ __forceinline__ bool grid_phi_total(TileSum<T>& ts, double* partials,
   if constexpr (sizeof(T) == 8) {
     return last_block_total(block_sum(ts.a), partials, counter, total, blk, nblk);
   } else {
-    __shared__ unsigned long long s_warp[kBlock / 32];
+    __shared__ unsigned long long s_warp[32];
+    const int nw = (int)(blockDim.x >> 5);
     __shared__ bool s_last;
     unsigned long long v = ts.a;
 #pragma unroll
@@ -813,8 +1085,7 @@ __device__ __forceinline__ bool grid_phi_total(TileSum<T>& ts, double* partials,
     unsigned long long* up = reinterpret_cast<unsigned long long*>(partials);
     if (threadIdx.x == 0) {
       unsigned long long r = 0ull;
-#pragma unroll
-      for (int i = 0; i < kBlock / 32; ++i) r += s_warp[i];
+for (int i = 0; i < nw; ++i) r += s_warp[i];
       up[blk] = nan ? kSumNaN : r;
       __threadfence();
       s_last = (atomicAdd(counter, 1u) == (unsigned)nblk - 1);
@@ -836,14 +1107,65 @@ __device__ __forceinline__ bool grid_phi_total(TileSum<T>& ts, double* partials,
     __syncthreads();
     if (threadIdx.x == 0) {
       unsigned long long r = 0ull;
-#pragma unroll
-      for (int i = 0; i < kBlock / 32; ++i) r += s_warp[i];
+for (int i = 0; i < nw; ++i) r += s_warp[i];
       *total = any_nan ? __longlong_as_double(0x7ff8000000000000ll) : (double)r / kFix;
       *counter = 0u;
     }
     return threadIdx.x == 0;
   }
 }
+
+// TileNode: a node of the fused kernel's tile: the phi stencil and classes come
+// from the tile's shared memory (strides sx, sy, 1), and with STAGED g, u and
+// the previous phi from the node's cp.async staging slot (word j at st[j kBlock]).
+template <typename T, typename S, bool RAW, bool STAGED>
+struct TileNode : NodeAt<T, S, RAW, true> {
+  using Base = NodeAt<T, S, RAW, true>;
+  const T* sphi;
+  const uint8_t* scls;
+  const int sx, sy;
+  const T* st;
+  __device__ __forceinline__ TileNode(const Consts<T>& k_, const State<T, S>& s_, const Pol& p_, const Nbr& nb_, int n_,
+                                      const T* sphi_, const uint8_t* scls_, int sx_, int sy_, const T* st_)
+      : Base(k_, s_, p_, nb_, n_), sphi(sphi_), scls(scls_), sx(sx_), sy(sy_), st(st_) {}
+  __device__ __forceinline__ int off(int q) const { return ex(q) * sx + ey(q) * sy + ez(q); }
+  __device__ __forceinline__ T phi_at(int q) const { return sphi[off(q)]; }
+  __device__ __forceinline__ T ref_at(int q) const { return sphi[off(q)]; }
+  __device__ __forceinline__ bool solid_at(int q) const { return (scls[off(q)] & kSolid) != 0; }
+  __device__ __forceinline__ void st_f(int q, T v) const {
+    st_pol(this->s.fout + (q * this->Np + this->e), Base::IO::st_f(v, q, Base::IO::kDev ? ref_at(q) : T(0), this->k),
+           this->pol.once);
+  }
+  __device__ __forceinline__ void load_g(T (&g)[Q], uint8_t c, T eps) const {
+    if constexpr (STAGED) {
+      const T* gin = reinterpret_cast<const T*>(this->s.gin);
+      if (!RAW && (c & kSolid)) {
+        // bounce-back: the node's own opposite values, not the staged pulled ones
+#pragma unroll
+        for (int q = 0; q < Q; ++q) g[q] = ldg(gin + (opp(q) * this->Np + this->e));
+      } else {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) g[q] = st[q * kBlock];
+      }
+      if (!RAW && (c & kPartial)) {
+        const T one_m = sub_rn(T(1), eps);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          g[q] = fma_(one_m, g[q], mul_rn(eps, ldg(gin + (opp(q) * this->Np + this->e))));
+      }
+    } else {
+      Base::load_g(g, c, eps);
+    }
+  }
+  __device__ __forceinline__ T u_old(int d) const {
+    if constexpr (STAGED) return st[(Q + d) * kBlock];
+    else return Base::u_old(d);
+  }
+  __device__ __forceinline__ T phi_old() const {
+    if constexpr (STAGED) return st[(Q + 3) * kBlock];
+    else return Base::phi_old();
+  }
+};
 
 // ---------------------------------------------------------------------------
 // The fused time step
@@ -930,13 +1252,7 @@ __global__ void __launch_bounds__(kBlock, StepOccupancy<T, S>::blocks) k_step(Co
       const int n = n00 + (hx * k.ny + hy) * k.nz + hz;
       const uint8_t c = s.cls[n];
       const bool own = hx >= 1 && hx <= ex_ && hy >= 1 && hy <= ey_ && hz >= 1 && hz <= ez_;
-      T phi = T(0);
-      if (!(c & kSolid)) {
-        const T eps = (c & kPartial) ? s.eps[n] : T(0);
-        T v[Q];
-        fetch_f<T, S, RAW, true, true>(v, k, s, n, N, nbc, c, eps, pol.keep);
-        phi = clamp01(seqsum(v));
-      }
+      const T phi = (c & kSolid) ? T(0) : phi_value<T, S, RAW, true>(k, s, n, c, nbc, pol.keep);
       sphi[h] = phi;
       scls[h] = c;
       if (own) part.add(phi);
@@ -955,13 +1271,8 @@ __global__ void __launch_bounds__(kBlock, StepOccupancy<T, S>::blocks) k_step(Co
       const uint8_t c = s.cls[n];
       const bool own = hx >= 1 && hx <= ex_ && hy >= 1 && hy <= ey_ && hz >= 1 && hz <= ez_;
       T phi = T(0);
-      if (!(c & kSolid)) {
-        const Nbr nb = make_nbr_xyz(gx, gy, gz, k.nx, k.ny, k.nz);
-        const T eps = (c & kPartial) ? s.eps[n] : T(0);
-        T v[Q];
-        fetch_f<T, S, RAW, true, true>(v, k, s, n, N, nb, c, eps, pol.keep);
-        phi = clamp01(seqsum(v));
-      }
+      if (!(c & kSolid))
+        phi = phi_value<T, S, RAW, true>(k, s, n, c, make_nbr_xyz(gx, gy, gz, k.nx, k.ny, k.nz), pol.keep);
       sphi[h] = phi;
       scls[h] = c;
       if (own) part.add(phi);
@@ -1003,13 +1314,10 @@ __global__ void __launch_bounds__(kBlock, StepOccupancy<T, S>::blocks) k_step(Co
       const int h = ((lx + 1) * HY + (ly + 1)) * HZ + (lz + 1);
       const int n = ((x0 + lx) * k.ny + (y0 + ly)) * k.nz + (z0 + lz);
       const Nbr nb = make_nbr_xyz(x0 + lx, y0 + ly, z0 + lz, k.nx, k.ny, k.nz);
-      // phi of this step at x + e_q (also the deviation reference, in the half
-      // form, of the next step's reader of slot (x, q))
-      update_node<T, S, RAW, FIRST, OMEGA1, STAGED, true, false, true>(
-          k, s, n, nb, scls[h], sphi[h], [&](int q) { return sphi[h + ex(q) * sx + ey(q) * HZ + ez(q)]; },
-          [&](int q) { return (scls[h + ex(q) * sx + ey(q) * HZ + ez(q)] & kSolid) != 0; },
-          [&](int q) { return sphi[h + ex(q) * sx + ey(q) * HZ + ez(q)]; }, pol,
-          stage + (j & 1) * kStage * kBlock + threadIdx.x);
+      const TileNode<T, S, RAW, STAGED> node(k, s, pol, nb, n, sphi + h, scls + h, sx, HZ,
+                                             stage + (j & 1) * kStage * kBlock + threadIdx.x);
+      update_node<T, S, FIRST, OMEGA1, false, false>(k, s, node, scls[h], sphi[h]);
+      st_pol(s.phi_out + node.e, sphi[h], pol.once);
     }
   }
   if constexpr (STAGED) cp_async_wait<0>();
@@ -1023,14 +1331,6 @@ __global__ void __launch_bounds__(kBlock, StepOccupancy<T, S>::blocks) k_step(Co
 // omega_f == 1 f is read by k_phi only, and the pair moves the algorithmic
 // bytes of the step plus the phi stencil's L2 traffic.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void decode(const FastDiv& dz, const FastDiv& dy, int n, int nz, int ny, int& ix,
-                                       int& iy, int& iz) {
-  const int t = (int)dz.div((unsigned)n);
-  iz = n - t * nz;
-  ix = (int)dy.div((unsigned)t);
-  iy = t - ix * ny;
-}
-
 // Persistent: a grid of about one wave strides over the nodes, so that the
 // per-block publication of the partial sum happens once per block.
 // phi of node n (written to phi_out) added to the block's sum.
@@ -1041,12 +1341,9 @@ __device__ __forceinline__ void phi_node(const Consts<T>& k, const State<T, S>& 
   if (!(c & kSolid)) {
     int ix, iy, iz;
     decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
-    const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
-    const T eps = (c & kPartial) ? s.eps[n] : T(0);
-    T v[Q];
-    // f is read again by k_update only when omega_f != 1
-    fetch_f<T, S, RAW, true, MAP>(v, k, s, n, (size_t)k.N, nb, c, eps, k.omega_f == T(1) ? pol.once : pol.keep);
-    phi = clamp01(seqsum(v));
+    // f is read again by the update kernel only when omega_f != 1
+    phi = phi_value<T, S, RAW, MAP>(k, s, n, c, make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz),
+                                    k.omega_f == T(1) ? pol.once : pol.keep);
   }
   st_pol(s.phi_out + (MAP ? sidx(k, n) : (unsigned)n), phi, pol.keep);  // read back (stencil) by k_update
   part.add(phi);
@@ -1089,30 +1386,44 @@ struct UpdateOccupancy {
   static constexpr int blocks = sizeof(T) == 8 ? 1 : 4;
 };
 
-template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1, bool GMU, bool MAP = false>
+template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1, bool GMU, bool SOUT, bool MAP = false>
 __device__ __forceinline__ void update_one(const Consts<T>& k, const State<T, S>& s, int n, const Pol& pol) {
   int ix, iy, iz;
   decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
-  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
-  const T* __restrict__ pc = s.phi_out;  // phi of this step (k_phi)
-  const uint8_t c = s.cls[n];
-  auto I = [&](int m) -> unsigned { return MAP ? sidx(k, m) : (unsigned)m; };
-  const T phi = ld_pol(pc + I(n), pol.keep);
-  update_node<T, S, RAW, FIRST, OMEGA1, false, false, GMU, MAP>(
-      k, s, n, nb, c, phi, [&](int q) { return ld_pol(pc + I(nb.at(n, ex(q), ey(q), ez(q))), pol.keep); },
-      [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; },
-      [&](int q) { return ld_pol(pc + I(nb.at(n, ex(q), ey(q), ez(q))), pol.keep); }, pol, (const T*)nullptr);
+  const NodeAt<T, S, RAW, MAP> node(k, s, pol, make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz), n);
+  update_node<T, S, FIRST, OMEGA1, GMU, SOUT>(k, s, node, s.cls[n], ld_pol(s.phi_out + node.e, pol.keep));
 }
 
-// One thread per node, linear order.  (Measured slower on the 150x150x107
-// case: a persistent grid-stride form, and forms that stage the next node's
-// g, u and previous phi in shared memory with cp.async or with bulk copies
-// per chunk of nodes -- the copies, the smaller L1 and the block-wide waits
-// cost more than the latency they hide.)
-template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1, bool GMU = false>
+// The update of the nodes [n0, n0 + BS) of a linear-layout grid by one block,
+// one thread per node: blocks that lie inside 1 <= x <= nx - 2 take the cheap
+// addressing (NodeIn: 1,063 -> 890 instructions per warp and 136 -> 131 us with
+// stored populations on the 150x150x107 case), the blocks on the first and last
+// planes, whose x neighbours wrap around, the general one.
+template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS>
+__device__ __forceinline__ void update_block(const Consts<T>& k, const State<T, S>& s, int n0) {
+  const int n = n0 + threadIdx.x, P = k.ny * k.nz;
+  const Pol pol = Pol::make();
+  if (n0 >= P && n0 + BS <= k.N - P) {
+    int ix, iy, iz;
+    decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+    const NodeIn<T, S> node(k, s, pol, n, iy, iz);
+    update_node<T, S, false, OMEGA1, GMU, SOUT>(k, s, node, s.cls[n], ld_pol(s.phi_out + n, pol.keep));
+  } else if (n < k.N) {
+    update_one<T, S, false, false, OMEGA1, GMU, SOUT>(k, s, n, pol);
+  }
+}
+
+// One thread per node, linear order.  What bounds it: 197 bytes per node (source
+// form) took 80 us on the 150x150x107 case in a kernel of the same loads and
+// stores without the arithmetic; with it 102.5 us (float), half of the warps'
+// time waiting for loads, half of the issue slots used.  (Measured slower there: a
+// persistent grid-stride form, 108 -> 112 us; all loads first with 80 to 96
+// registers, 105 -> 115 us; forms that stage the next node's g, u and previous
+// phi in shared memory with cp.async or with bulk copies per chunk of nodes.)
+template <typename T, typename S, bool OMEGA1, bool GMU = false>
 __global__ void __launch_bounds__(kBlock, UpdateOccupancy<T, S, GMU>::blocks) k_update(Consts<T> k, State<T, S> s) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n < k.N) update_one<T, S, RAW, FIRST, OMEGA1, GMU, true>(k, s, n, Pol::make());
+  if (n < k.N) update_one<T, S, true, true, OMEGA1, GMU, false, true>(k, s, n, Pol::make());
 }
 
 // Gradient of the chemical potential of every node (mu from k_mu), for the
@@ -1155,7 +1466,7 @@ __global__ void __launch_bounds__(kBlock) k_mu(Consts<T> k, State<T, S> s) {
   for (int q = 1; q < Q; ++q) ps[q] = ld_pol(pc + sidx(k, nb.at(n, ex(q), ey(q), ez(q))), pol.keep);
   auto solid_at = [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; };
   T gx, gy, gz, lap;
-  grad_lap<T, true, State<T, S>, decltype(solid_at), true>(k, s, n, c, phi, ps, solid_at, gx, gy, gz, lap);
+  grad_lap<T, true>(k, s, n, c, phi, ps, solid_at, gx, gy, gz, lap);
   st_pol(s.mu + n, chem_pot(k, c, phi, lap), pol.keep);
 }
 
@@ -1175,6 +1486,8 @@ struct CaseDesc {
   State<T, S> s;
   int phi_blk0, phi_nblk;  // the case's blocks in the k_phi_batch grid
   int upd_blk0, upd_nblk;  // and in the k_update_batch grid
+  int phs_blk0;            // first block in the k_phis_batch grid
+  PhiTile tile;            // and the tiles of that pass
 };
 
 // Programmatic dependent launch between the step kernels: a kernel launched
@@ -1195,40 +1508,62 @@ __device__ __forceinline__ void load_desc(D& dst, const D* src) {
   __syncthreads();
 }
 
+// Block b of the nb that share a grid's phi pass.
 template <typename T, typename S>
-__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 3 : 4) k_phi_batch(const CaseDesc<T, S>* __restrict__ cases,
-                                                     const unsigned short* __restrict__ blk2case) {
-  __shared__ CaseDesc<T, S> d;
-  load_desc(d, cases + (blk2case ? blk2case[blockIdx.x] : 0));
-  pdl_trigger();
-  pdl_wait();  // f of the previous update kernel
+__device__ __forceinline__ void phi_block(const Consts<T>& k, const State<T, S>& s, int b, int nb) {
   const Pol pol = Pol::make();
-  const int b = blockIdx.x - d.phi_blk0, nb = d.phi_nblk;
   TileSum<T> part;
   // the class byte of the thread's next node is loaded one node ahead, so
   // that the pulled loads of a node do not wait for its class load
-  const int N = d.k.N, stride = nb * kBlock;
+  const int N = k.N, stride = nb * kBlock;
   int n = b * kBlock + threadIdx.x;
-  uint8_t c = n < N ? d.s.cls[n] : 0;
+  uint8_t c = n < N ? s.cls[n] : 0;
   for (; n < N; n += stride) {
-    const uint8_t c_next = n + stride < N ? d.s.cls[n + stride] : 0;
-    phi_node<T, S, false>(d.k, d.s, n, c, pol, part);
+    const uint8_t c_next = n + stride < N ? s.cls[n + stride] : 0;
+    phi_node<T, S, false>(k, s, n, c, pol, part);
     c = c_next;
   }
-  phi_finish(d.s, part, b, nb);
+  phi_finish(s, part, b, nb);
+}
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 3 : 4) k_phi_batch(
+    const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ blk2case, int blk0) {
+  // blk0: the first block of the table's phi part that this launch runs
+  __shared__ CaseDesc<T, S> d;
+  load_desc(d, cases + blk2case[blk0 + blockIdx.x]);
+  pdl_trigger();
+  pdl_wait();  // f of the previous update kernel
+  phi_block(d.k, d.s, blk0 + blockIdx.x - d.phi_blk0, d.phi_nblk);
 }
 
 // BS threads per block (the autotuners choose 128 or 256), compiled for the
 // same registers per thread at either size.
-template <typename T, typename S, bool OMEGA1, bool GMU = false, int BS = kBlock>
-__global__ void __launch_bounds__(BS, UpdateOccupancy<T, S, GMU>::blocks * kBlock / BS) k_update_batch(
+template <typename T, typename S, bool OMEGA1, bool SOUT, int BS = kBlock>
+__global__ void __launch_bounds__(BS, UpdateOccupancy<T, S>::blocks * kBlock / BS) k_update_batch(
     const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ blk2case) {
   __shared__ CaseDesc<T, S> d;
   load_desc(d, cases + (blk2case ? blk2case[blockIdx.x] : 0));
   pdl_trigger();
+  pdl_wait();  // phi of the phi kernel
+  update_block<T, S, OMEGA1, false, SOUT, BS>(d.k, d.s, (blockIdx.x - d.upd_blk0) * BS);
+}
+
+// The step kernels of one grid alone: the descriptor is a kernel parameter, so
+// its constants and pointers are constant-bank operands and the block starts
+// without reading a table.
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 3 : 4) k_phi_one(const __grid_constant__ CaseDesc<T, S> d) {
+  pdl_trigger();
+  pdl_wait();  // f of the previous update kernel
+  phi_block(d.k, d.s, blockIdx.x, gridDim.x);
+}
+template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS = kBlock>
+__global__ void __launch_bounds__(BS, UpdateOccupancy<T, S, GMU>::blocks * kBlock / BS)
+    k_update_one(const __grid_constant__ CaseDesc<T, S> d) {
+  pdl_trigger();
   pdl_wait();  // phi of the phi kernel (mu of k_mu with GMU)
-  const int n = (blockIdx.x - d.upd_blk0) * BS + threadIdx.x;
-  if (n < d.k.N) update_one<T, S, false, false, OMEGA1, GMU>(d.k, d.s, n, Pol::make());
+  update_block<T, S, OMEGA1, GMU, SOUT, BS>(d.k, d.s, blockIdx.x * BS);
 }
 
 // ---------------------------------------------------------------------------
@@ -1246,37 +1581,25 @@ __global__ void __launch_bounds__(kBlock, UpdateOccupancy<T, S>::blocks) k_batch
     const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ b2c, int phi_blocks,
     int upd_blocks_om1, int upd_blocks_other) {
   __shared__ CaseDesc<T, S> d;
-  const Pol pol = Pol::make();
   for (int vb = blockIdx.x; vb < phi_blocks; vb += gridDim.x) {
     __syncthreads();  // the previous virtual block is done with d
     load_desc(d, cases + b2c[vb]);
-    const int b = vb - d.phi_blk0, nb = d.phi_nblk;
-    TileSum<T> part;
-    const int N = d.k.N, stride = nb * kBlock;
-    int n = b * kBlock + threadIdx.x;
-    uint8_t c = n < N ? d.s.cls[n] : 0;
-    for (; n < N; n += stride) {
-      const uint8_t c_next = n + stride < N ? d.s.cls[n + stride] : 0;
-      phi_node<T, S, false>(d.k, d.s, n, c, pol, part);
-      c = c_next;
-    }
-    phi_finish(d.s, part, b, nb);
+    phi_block(d.k, d.s, vb - d.phi_blk0, d.phi_nblk);
   }
   cooperative_groups::this_grid().sync();
   const int upd_blocks = upd_blocks_om1 + upd_blocks_other;
   for (int vb = blockIdx.x; vb < upd_blocks; vb += gridDim.x) {
     __syncthreads();
     load_desc(d, cases + b2c[phi_blocks + vb]);
-    const int n = (vb - (vb < upd_blocks_om1 ? 0 : upd_blocks_om1) - d.upd_blk0) * kBlock + threadIdx.x;
-    if (n < d.k.N) {
-      if (vb < upd_blocks_om1) update_one<T, S, false, false, true, false>(d.k, d.s, n, pol);
-      else update_one<T, S, false, false, false, false>(d.k, d.s, n, pol);
-    }
+    const int n0 = (vb - (vb < upd_blocks_om1 ? 0 : upd_blocks_om1) - d.upd_blk0) * kBlock;
+    if (vb < upd_blocks_om1) update_block<T, S, true, false, false, kBlock>(d.k, d.s, n0);
+    else update_block<T, S, false, false, false, kBlock>(d.k, d.s, n0);
   }
 }
 
 }  // namespace lbm
 
+#include "lbm_phis.cuh"
 #include "lbm_pair.cuh"
 
 namespace lbm {
@@ -1694,7 +2017,7 @@ template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1>
 static cudaError_t launch_step_t(const Consts<T>& k, const State<T, S>& s, const Tiling& tl, cudaStream_t st) {
   const size_t sm = step_smem_bytes<T, S>(tl);
   auto fn = k_step<T, S, RAW, FIRST, OMEGA1>;
-  if (sm > 48 * 1024) {
+  if (sm > 46 * 1024) {  // dynamic and static shared memory together may pass 48 KB
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
   }
@@ -1702,30 +2025,30 @@ static cudaError_t launch_step_t(const Consts<T>& k, const State<T, S>& s, const
   return cudaGetLastError();
 }
 
-template <typename T, typename S, bool RAW, bool FIRST, bool OMEGA1>
-static cudaError_t launch_two_t(const Consts<T>& k, const State<T, S>& s, cudaStream_t st, cudaEvent_t mid) {
+// The first step after init: k_phi, [k_mu, k_gradmu], k_update on the raw state.
+template <typename T, typename S, bool OMEGA1>
+static cudaError_t launch_first_t(const Consts<T>& k, const State<T, S>& s, cudaStream_t st, cudaEvent_t mid) {
   int gphi = 0;
-  cudaError_t e = resident_grid(k_phi<T, S, RAW>, k.N, &gphi);
+  cudaError_t e = resident_grid(k_phi<T, S, true>, k.N, &gphi);
   if (e != cudaSuccess) return e;
-  k_phi<T, S, RAW><<<gphi, kBlock, 0, st>>>(k, s);
+  k_phi<T, S, true><<<gphi, kBlock, 0, st>>>(k, s);
   if (mid) {
     e = cudaEventRecord(mid, st);
     if (e != cudaSuccess) return e;
   }
   const int blocks = (k.N + kBlock - 1) / kBlock;
   if (k.gmu_mode) {
-    // the gradient-of-mu modes: float and double storage, first step here
-    // (later steps run the batched kernels)
-    if constexpr (RAW && FIRST && sizeof(S) != 2) {
+    // the gradient-of-mu modes: float and double storage
+    if constexpr (sizeof(S) != 2) {
       k_mu<T, S><<<blocks, kBlock, 0, st>>>(k, s);
       k_gradmu<T, S><<<blocks, kBlock, 0, st>>>(k, s);
-      k_update<T, S, RAW, FIRST, OMEGA1, true><<<blocks, kBlock, 0, st>>>(k, s);
+      k_update<T, S, OMEGA1, true><<<blocks, kBlock, 0, st>>>(k, s);
       return cudaGetLastError();
     } else {
       return cudaErrorNotSupported;
     }
   }
-  k_update<T, S, RAW, FIRST, OMEGA1><<<blocks, kBlock, 0, st>>>(k, s);
+  k_update<T, S, OMEGA1><<<blocks, kBlock, 0, st>>>(k, s);
   return cudaGetLastError();
 }
 
@@ -1740,12 +2063,9 @@ cudaError_t launch_step(const Consts<T>& k, const State<T, S>& s, const Tiling& 
   if (raw != first) return cudaErrorInvalidValue;
   if (k.gmu_mode && tl.tx != 0) return cudaErrorNotSupported;  // no fused-kernel form of these modes
   if (tl.tx == 0) {
-    const bool om1 = k.omega_f == T(1);
-    if (raw)
-      return om1 ? launch_two_t<T, S, true, true, true>(k, s, st, mid)
-                 : launch_two_t<T, S, true, true, false>(k, s, st, mid);
-    return om1 ? launch_two_t<T, S, false, false, true>(k, s, st, mid)
-               : launch_two_t<T, S, false, false, false>(k, s, st, mid);
+    // every later two-kernel step goes through the descriptor kernels
+    if (!raw) return cudaErrorInvalidValue;
+    return k.omega_f == T(1) ? launch_first_t<T, S, true>(k, s, st, mid) : launch_first_t<T, S, false>(k, s, st, mid);
   }
   if (mid) {
     cudaError_t e = cudaEventRecord(mid, st);
@@ -1761,11 +2081,12 @@ cudaError_t launch_step(const Consts<T>& k, const State<T, S>& s, const Tiling& 
 // Launch with programmatic stream serialization (see pdl_wait).
 constexpr int kPdlOn = 1;  // 0: plain stream serialization
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl_bs(void (*fn)(KArgs...), int blocks, int threads, cudaStream_t st, Args... args) {
+static cudaError_t launch_pdl_bs(void (*fn)(KArgs...), int blocks, int threads, cudaStream_t st,
+                                 const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = threads == kPhisNT ? kPhisShared : 0;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1775,40 +2096,97 @@ static cudaError_t launch_pdl_bs(void (*fn)(KArgs...), int blocks, int threads, 
   return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*fn)(KArgs...), int blocks, cudaStream_t st, Args... args) {
+static cudaError_t launch_pdl(void (*fn)(KArgs...), int blocks, cudaStream_t st, const Args&... args) {
   return launch_pdl_bs(fn, blocks, kBlock, st, args...);
 }
 
-// Batched step kernels over a device case table; blocks: the grid (the
-// length of the block -> case table).
+// Batched step kernels over a device case table; blocks: the grid (the part
+// of the block -> case table that starts at blk0).
 template <typename T, typename S>
-cudaError_t launch_phi_batch(const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
+cudaError_t launch_phi_batch(const void* cases, const unsigned short* b2c, int blk0, int blocks, cudaStream_t st) {
   if (blocks <= 0) return cudaSuccess;
-  return launch_pdl(k_phi_batch<T, S>, blocks, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
+  return launch_pdl(k_phi_batch<T, S>, blocks, st, static_cast<const CaseDesc<T, S>*>(cases), b2c, blk0);
 }
-// bs: threads per block of the update kernel, 256 or (without the
-// gradient-of-mu modes) 128.
+// bs: threads per block of the update kernel, 256 or 128.  sout: f is written as J.
 template <typename T, typename S>
-cudaError_t launch_update_batch(const void* cases, const unsigned short* b2c, int blocks, bool omega1,
-                                cudaStream_t st, bool gmu, int bs) {
+cudaError_t launch_update_batch(const void* cases, const unsigned short* b2c, int blocks, bool omega1, bool sout,
+                                cudaStream_t st, int bs) {
   if (blocks <= 0) return cudaSuccess;
+  if (bs != 128 && bs != kBlock) return cudaErrorInvalidValue;
   auto c = static_cast<const CaseDesc<T, S>*>(cases);
+  if constexpr (sizeof(T) == 4) {
+    if (omega1 && sout)
+      return bs == 128 ? launch_pdl_bs(k_update_batch<T, S, true, true, 128>, blocks, 128, st, c, b2c)
+                       : launch_pdl(k_update_batch<T, S, true, true>, blocks, st, c, b2c);
+  }
+  if (bs == 128)
+    return omega1 ? launch_pdl_bs(k_update_batch<T, S, true, false, 128>, blocks, 128, st, c, b2c)
+                  : launch_pdl_bs(k_update_batch<T, S, false, false, 128>, blocks, 128, st, c, b2c);
+  return omega1 ? launch_pdl(k_update_batch<T, S, true, false>, blocks, st, c, b2c)
+                : launch_pdl(k_update_batch<T, S, false, false>, blocks, st, c, b2c);
+}
+// The step kernels of one linear-layout grid, its descriptor passed by value
+// (a block of case_desc_bytes filled by fill_case_desc in host memory).
+template <typename T, typename S>
+cudaError_t launch_phi_one(const void* desc, cudaStream_t st) {
+  const CaseDesc<T, S>& d = *static_cast<const CaseDesc<T, S>*>(desc);
+  return launch_pdl(k_phi_one<T, S>, d.phi_nblk, st, d);
+}
+template <typename T, typename S, bool GMU, int BS>
+static cudaError_t launch_update_one_t(const CaseDesc<T, S>& d, bool omega1, bool sout, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4) {
+    if (omega1 && sout) return launch_pdl_bs(k_update_one<T, S, true, GMU, true, BS>, d.upd_nblk, BS, st, d);
+  }
+  return omega1 ? launch_pdl_bs(k_update_one<T, S, true, GMU, false, BS>, d.upd_nblk, BS, st, d)
+                : launch_pdl_bs(k_update_one<T, S, false, GMU, false, BS>, d.upd_nblk, BS, st, d);
+}
+template <typename T, typename S>
+cudaError_t launch_update_one(const void* desc, bool omega1, bool sout, cudaStream_t st, bool gmu, int bs) {
+  const CaseDesc<T, S>& d = *static_cast<const CaseDesc<T, S>*>(desc);
   if (gmu) {
     if constexpr (sizeof(S) != 2) {
       if (bs != kBlock) return cudaErrorInvalidValue;
-      if (omega1) return launch_pdl(k_update_batch<T, S, true, true>, blocks, st, c, b2c);
-      return launch_pdl(k_update_batch<T, S, false, true>, blocks, st, c, b2c);
+      return launch_update_one_t<T, S, true, kBlock>(d, omega1, sout, st);
     } else {
       return cudaErrorNotSupported;
     }
   }
-  if (bs == 128) {
-    if (omega1) return launch_pdl_bs(k_update_batch<T, S, true, false, 128>, blocks, 128, st, c, b2c);
-    return launch_pdl_bs(k_update_batch<T, S, false, false, 128>, blocks, 128, st, c, b2c);
-  }
+  if (bs == 128) return launch_update_one_t<T, S, false, 128>(d, omega1, sout, st);
   if (bs != kBlock) return cudaErrorInvalidValue;
-  if (omega1) return launch_pdl(k_update_batch<T, S, true>, blocks, st, c, b2c);
-  return launch_pdl(k_update_batch<T, S, false>, blocks, st, c, b2c);
+  return launch_update_one_t<T, S, false, kBlock>(d, omega1, sout, st);
+}
+// The phi pass of a state that holds S (float compute only), and the
+// populations back from J: s.fout = the populations of the state s.fin.
+template <typename T, typename S>
+cudaError_t launch_phis_batch(const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    return cudaErrorNotSupported;
+  } else {
+    if (blocks <= 0) return cudaSuccess;
+    const cudaError_t e = phis_shared(k_phis_batch<T, S>);
+    if (e != cudaSuccess) return e;
+    return launch_pdl_bs(k_phis_batch<T, S>, blocks, kPhisNT, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
+  }
+}
+template <typename T, typename S>
+cudaError_t launch_phis_one(const void* desc, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    return cudaErrorNotSupported;
+  } else {
+    const CaseDesc<T, S>& d = *static_cast<const CaseDesc<T, S>*>(desc);
+    const cudaError_t e = phis_shared(k_phis_one<T, S>);
+    if (e != cudaSuccess) return e;
+    return launch_pdl_bs(k_phis_one<T, S>, d.tile.blocks(), kPhisNT, st, d);
+  }
+}
+template <typename T, typename S>
+cudaError_t launch_expand(const Consts<T>& k, const State<T, S>& s, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    return cudaErrorNotSupported;
+  } else {
+    k_expand<T, S><<<(k.N + kBlock - 1) / kBlock, kBlock, 0, st>>>(k, s);
+    return cudaGetLastError();
+  }
 }
 // The paired-layout step kernels over a device case table of paired grids.
 // (float compute only: float64 grids keep the linear layout)
@@ -1898,9 +2276,11 @@ size_t case_desc_bytes() {
 // Fills one descriptor in host memory.
 template <typename T, typename S>
 void fill_case_desc(void* dst, const Consts<T>& k, const State<T, S>& s, int phi_blk0, int phi_nblk, int upd_blk0,
-                    int upd_nblk) {
+                    int upd_nblk, int phs_blk0, const PhiTile& tile) {
   CaseDesc<T, S> d;
   std::memset(&d, 0, sizeof(d));
+  d.phs_blk0 = phs_blk0;
+  d.tile = tile;
   d.k = k;
   d.s = s;
   d.phi_blk0 = phi_blk0;
@@ -1962,11 +2342,14 @@ cudaError_t launch_momentum(int N, const T* phi, const T* u, int us, int nh, dou
   k_momentum<T><<<grid, kBlock, 0, st>>>(N, phi, u, us, nh, rho_l, rho_g, partials, counter, out3);
   return cudaGetLastError();
 }
+#if LBM_PART == 0
 template cudaError_t launch_momentum<float>(int, const float*, const float*, int, int, double, double, double*, int,
                                             unsigned*, double*, cudaStream_t);
 template cudaError_t launch_momentum<double>(int, const double*, const double*, int, int, double, double, double*,
                                              int, unsigned*, double*, cudaStream_t);
+#endif
 
+#if LBM_PART == 0
 // ---------------------------------------------------------------------------
 // Allocation-free spread diagnostics.  Some callers cannot allocate device
 // memory: code that runs inside a memory pool handed out by another runtime,
@@ -2033,11 +2416,14 @@ template cudaError_t launch_measure_static<float>(int, int, int, const float*, c
 template cudaError_t launch_measure_static<double>(int, int, int, const double*, const uint8_t*, double*,
                                                    cudaStream_t);
 
-template size_t step_smem_bytes<float, float>(const Tiling&);
-template size_t step_smem_bytes<double, double>(const Tiling&);
-template size_t step_smem_bytes<float, __half>(const Tiling&);
+#endif  // LBM_PART == 0
+
+// This file is compiled once per compute / storage type pair (LBM_PART: 0
+// float / float and the type-independent parts, 1 double / double, 2 float /
+// half), in parallel.
 
 #define LBM_INSTANTIATE(T, S)                                                                                   \
+  template size_t step_smem_bytes<T, S>(const Tiling&);                                                         \
   template cudaError_t launch_step<T, S>(const Consts<T>&, const State<T, S>&, const Tiling&, bool, bool,        \
                                          cudaStream_t, cudaEvent_t);                                             \
   template cudaError_t launch_init<T, S, float>(const Consts<T>&, const State<T, S>&, const float*, const float*,  \
@@ -2050,30 +2436,43 @@ template size_t step_smem_bytes<float, __half>(const Tiling&);
   template cudaError_t launch_inject<T, S>(const Consts<T>&, const State<T, S>&, bool, const InjectParams&,        \
                                            const T*, unsigned*, cudaStream_t);
 
-LBM_INSTANTIATE(float, float)
-LBM_INSTANTIATE(double, double)
-LBM_INSTANTIATE(float, __half)
-#undef LBM_INSTANTIATE
 
 #define LBM_INSTANTIATE_BATCH(T, S)                                                                             \
-  template cudaError_t launch_phi_batch<T, S>(const void*, const unsigned short*, int, cudaStream_t);           \
-  template cudaError_t launch_update_batch<T, S>(const void*, const unsigned short*, int, bool, cudaStream_t,    \
-                                                 bool, int);                                                     \
+  template cudaError_t launch_phi_batch<T, S>(const void*, const unsigned short*, int, int, cudaStream_t);      \
+  template cudaError_t launch_update_batch<T, S>(const void*, const unsigned short*, int, bool, bool,            \
+                                                 cudaStream_t, int);                                             \
+  template cudaError_t launch_phi_one<T, S>(const void*, cudaStream_t);                                         \
+  template cudaError_t launch_update_one<T, S>(const void*, bool, bool, cudaStream_t, bool, int);               \
+  template cudaError_t launch_phis_batch<T, S>(const void*, const unsigned short*, int, cudaStream_t);          \
+  template cudaError_t launch_phis_one<T, S>(const void*, cudaStream_t);                                        \
+  template cudaError_t launch_expand<T, S>(const Consts<T>&, const State<T, S>&, cudaStream_t);                 \
   template cudaError_t launch_mu<T, S>(const Consts<T>&, const State<T, S>&, cudaStream_t);                     \
   template cudaError_t launch_phi_pair<T, S>(const void*, const unsigned short*, int, cudaStream_t);            \
   template cudaError_t launch_batch_coop<T, S>(const void*, const unsigned short*, int, int, int, cudaStream_t);  \
   template cudaError_t launch_update_pair<T, S>(const void*, const unsigned short*, int, bool, cudaStream_t,     \
                                                 bool);                                                          \
   template size_t case_desc_bytes<T, S>();                                                                      \
-  template void fill_case_desc<T, S>(void*, const Consts<T>&, const State<T, S>&, int, int, int, int);
+  template void fill_case_desc<T, S>(void*, const Consts<T>&, const State<T, S>&, int, int, int, int, int,         \
+                                     const PhiTile&);
+
+#if LBM_PART == 0
+LBM_INSTANTIATE(float, float)
 LBM_INSTANTIATE_BATCH(float, float)
+#elif LBM_PART == 1
+LBM_INSTANTIATE(double, double)
 LBM_INSTANTIATE_BATCH(double, double)
+#elif LBM_PART == 2
+LBM_INSTANTIATE(float, __half)
 LBM_INSTANTIATE_BATCH(float, __half)
+#endif
+#undef LBM_INSTANTIATE
 #undef LBM_INSTANTIATE_BATCH
 
+#if LBM_PART == 0
 template cudaError_t launch_measure<float>(int, int, int, const float*, const uint8_t*, double*, int, unsigned*,
                                            double*, cudaStream_t, double*);
 template cudaError_t launch_measure<double>(int, int, int, const double*, const uint8_t*, double*, int, unsigned*,
                                             double*, cudaStream_t, double*);
+#endif
 
 }  // namespace lbm

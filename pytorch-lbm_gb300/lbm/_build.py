@@ -1,7 +1,7 @@
 """Build liblbm_gb300.so in-tree for sm_103a.
 
-Six translation units compiled in parallel and linked with nvcc:
-  csrc/lbm_kernels.cu   device kernels (nvcc, sm_103a)
+Translation units compiled in parallel and linked with nvcc:
+  csrc/lbm_kernels.cu   device kernels (nvcc, sm_103a), once per type pair
   csrc/lbm_kernels2d.cu device kernels of the 2-D D2Q9 form (nvcc, sm_103a)
   csrc/lbm_capi.cu      the C ABI of include/lbm_gb300.h (nvcc host code)
   csrc/lbm_geometry.cu  device geometry precompute of a handle (explicitly
@@ -56,14 +56,17 @@ def build(force=False, verbose=False):
     nvcc = _nvcc()
     common = ["-O3", "-std=c++17", "-I", INCLUDE, "-I", CSRC]
     jobs = []
-    for src in ("lbm_kernels.cu", "lbm_kernels2d.cu", "lbm_geometry.cu", "lbm_capi.cu"):
-        obj = os.path.join(obj_dir, src + ".o")
+    # lbm_kernels.cu is compiled once per compute / storage type pair, in parallel
+    cuda = [("lbm_kernels.cu", part) for part in range(3)]
+    cuda += [(src, 0) for src in ("lbm_kernels2d.cu", "lbm_geometry.cu", "lbm_capi.cu")]
+    for src, part in cuda:
+        obj = os.path.join(obj_dir, f"{src}.{part}.o")
         # the 2-D kernels keep the reference's separate multiplies and adds
         # (no contraction into FMAs): their grids are small, and float32
         # parity with the reference is closer without contraction; the
         # geometry tables must be bit-exact
         extra = ["-fmad=false"] if src in ("lbm_kernels2d.cu", "lbm_geometry.cu") else []
-        jobs.append([nvcc, *common, *ARCH, "-lineinfo", *extra, "-Xcompiler", HOST_FLAGS, "-c",
+        jobs.append([nvcc, *common, *ARCH, "-lineinfo", f"-DLBM_PART={part}", *extra, "-Xcompiler", HOST_FLAGS, "-c",
                      os.path.join(CSRC, src), "-o", obj])
     for src in ("lbm_geometry.cpp", "lbm_io.cpp"):
         obj = os.path.join(obj_dir, src + ".o")
