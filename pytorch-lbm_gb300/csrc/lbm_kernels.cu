@@ -46,11 +46,14 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <type_traits>
 
 #include "lbm_common.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 
@@ -537,16 +540,14 @@ __device__ __forceinline__ void grad_mu(const Consts<T>& k, const St& s, int n, 
   for (int q = 1; q < Q; ++q) {
     T v = mu_at(q);
     if (ghost && nsolid(q)) {
-      float nde = 0.0f;
-      nde = __fadd_rn(nde, __fmul_rn(n0, (float)ex(q)));
-      nde = __fadd_rn(nde, __fmul_rn(n1, (float)ey(q)));
-      nde = __fadd_rn(nde, __fmul_rn(n2, (float)ez(q)));
-      v = k.linear ? mu - (T)__fmul_rn(nde, k.h_over_kappa_f) : mu + (T)__fmul_rn(nde, k.pcok_f) * mu * (T(1) - mu);
+      const float nde = edot(q, n0, n1, n2);
+      v = k.linear ? sub_rn(mu, (T)__fmul_rn(nde, k.h_over_kappa_f))
+                   : fma_(mul_rn((T)__fmul_rn(nde, k.pcok_f), mu), sub_rn(T(1), mu), mu);
     }
-    const T w = Lat<T>::wc(q);
-    if (ex(q) != 0) gx = add_rn(gx, mul_rn(ex(q) > 0 ? w : -w, v));
-    if (ey(q) != 0) gy = add_rn(gy, mul_rn(ey(q) > 0 ? w : -w, v));
-    if (ez(q) != 0) gz = add_rn(gz, mul_rn(ez(q) > 0 ? w : -w, v));
+    const T t = mul_rn(Lat<T>::wc(q), v);
+    if (ex(q) != 0) gx = ex(q) > 0 ? add_rn(gx, t) : sub_rn(gx, t);
+    if (ey(q) != 0) gy = ey(q) > 0 ? add_rn(gy, t) : sub_rn(gy, t);
+    if (ez(q) != 0) gz = ez(q) > 0 ? add_rn(gz, t) : sub_rn(gz, t);
   }
 }
 
@@ -604,6 +605,7 @@ struct NodeAt {
   __device__ __forceinline__ int nbr(int q) const { return nb.at(n, ex(q), ey(q), ez(q)); }
   __device__ __forceinline__ unsigned el(int m) const { return MAP ? sidx(k, m) : (unsigned)m; }
   __device__ __forceinline__ T phi_at(int q) const { return ld_pol(s.phi_out + el(nbr(q)), pol.keep); }
+  __device__ __forceinline__ T mu_at(int q) const { return ld_pol(s.mu + nbr(q), pol.keep); }
   __device__ __forceinline__ bool solid_at(int q) const { return (s.cls[nbr(q)] & kSolid) != 0; }
   __device__ __forceinline__ void load_g(T (&g)[Q], uint8_t c, T eps) const {
     fetch_pop<T, S, RAW, false, false, true, MAP>(g, k, s.gin, s.phi_in, n, (size_t)k.N, nb, c, eps, T(1), pol.once);
@@ -652,6 +654,9 @@ struct NodeIn {
   }
   __device__ __forceinline__ T phi_at(int q) const {
     return ld_pol(s.phi_out + (ex(q) * P + o[ey(q) + 1][ez(q) + 1]), pol.keep);
+  }
+  __device__ __forceinline__ T mu_at(int q) const {
+    return ld_pol(s.mu + (ex(q) * P + o[ey(q) + 1][ez(q) + 1]), pol.keep);
   }
   __device__ __forceinline__ bool solid_at(int q) const {
     return (s.cls[ex(q) * P + o[ey(q) + 1][ez(q) + 1]] & kSolid) != 0;
@@ -1426,25 +1431,33 @@ __global__ void __launch_bounds__(kBlock, UpdateOccupancy<T, S, GMU>::blocks) k_
   if (n < k.N) update_one<T, S, true, true, OMEGA1, GMU, false, true>(k, s, n, Pol::make());
 }
 
+// Runs fn(node) for the block's node n0 + threadIdx.x through the accessor that
+// serves the block (see update_block; a paired layout always through NodeAt).
+template <typename T, typename S, typename Fn>
+__device__ __forceinline__ void with_node(const Consts<T>& k, const State<T, S>& s, int n0, int bs, Fn fn) {
+  const int n = n0 + threadIdx.x, P = k.ny * k.nz;
+  if (n >= k.N) return;
+  const Pol pol = Pol::make();
+  int ix, iy, iz;
+  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+  if (n0 >= P && n0 + bs <= k.N - P && k.nh == 0) fn(NodeIn<T, S>(k, s, pol, n, iy, iz));
+  else fn(NodeAt<T, S, false, true>(k, s, pol, make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz), n));
+}
+
 // Gradient of the chemical potential of every node (mu from k_mu), for the
 // modes whose interface source needs it; read by the update kernel.
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock) k_gradmu(Consts<T> k, State<T, S> s) {
-  const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
-  int ix, iy, iz;
-  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
-  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
-  const Pol pol = Pol::make();
-  const uint8_t c = s.cls[n];
-  const T mu = ld_pol(s.mu + n, pol.keep);
-  T mx, my, mz;
-  grad_mu(k, s, n, c, mu, [&](int q) { return ld_pol(s.mu + nb.at(n, ex(q), ey(q), ez(q)), pol.keep); },
-          [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; }, mx, my, mz);
-  const unsigned Nu = (unsigned)k.Np, nu = (unsigned)n;
-  st_pol(s.gmu + nu, mx, pol.keep);
-  st_pol(s.gmu + (Nu + nu), my, pol.keep);
-  st_pol(s.gmu + (2 * Nu + nu), mz, pol.keep);
+  with_node(k, s, blockIdx.x * kBlock, kBlock, [&](const auto& a) {
+    const T mu = ld_pol(s.mu + a.n, a.pol.keep);
+    T mx, my, mz;
+    grad_mu(k, s, a.n, s.cls[a.n], mu, [&](int q) { return a.mu_at(q); }, [&](int q) { return a.solid_at(q); }, mx, my,
+            mz);
+    const unsigned Nu = (unsigned)k.Np, nu = (unsigned)a.n;
+    st_pol(s.gmu + nu, mx, a.pol.keep);
+    st_pol(s.gmu + (Nu + nu), my, a.pol.keep);
+    st_pol(s.gmu + (2 * Nu + nu), mz, a.pol.keep);
+  });
 }
 
 // Chemical potential of every node of this step (phi from the phi kernel),
@@ -1452,22 +1465,16 @@ __global__ void __launch_bounds__(kBlock) k_gradmu(Consts<T> k, State<T, S> s) {
 // stencil and arithmetic as the update kernel's.
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock) k_mu(Consts<T> k, State<T, S> s) {
-  const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
-  int ix, iy, iz;
-  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
-  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
-  const Pol pol = Pol::make();
-  const T* __restrict__ pc = s.phi_out;
-  const uint8_t c = s.cls[n];
-  const T phi = ld_pol(pc + sidx(k, n), pol.keep);
-  T ps[Q];
+  with_node(k, s, blockIdx.x * kBlock, kBlock, [&](const auto& a) {
+    const uint8_t c = s.cls[a.n];
+    const T phi = ld_pol(s.phi_out + sidx(k, a.n), a.pol.keep);
+    T ps[Q];
 #pragma unroll
-  for (int q = 1; q < Q; ++q) ps[q] = ld_pol(pc + sidx(k, nb.at(n, ex(q), ey(q), ez(q))), pol.keep);
-  auto solid_at = [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; };
-  T gx, gy, gz, lap;
-  grad_lap<T, true>(k, s, n, c, phi, ps, solid_at, gx, gy, gz, lap);
-  st_pol(s.mu + n, chem_pot(k, c, phi, lap), pol.keep);
+    for (int q = 1; q < Q; ++q) ps[q] = a.phi_at(q);
+    T gx, gy, gz, lap;
+    grad_lap<T, true>(k, s, a.n, c, phi, ps, [&](int q) { return a.solid_at(q); }, gx, gy, gz, lap);
+    st_pol(s.mu + a.n, chem_pot(k, c, phi, lap), a.pol.keep);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -1489,15 +1496,6 @@ struct CaseDesc {
   int phs_blk0;            // first block in the k_phis_batch grid
   PhiTile tile;            // and the tiles of that pass
 };
-
-// Programmatic dependent launch between the step kernels: a kernel launched
-// with the programmatic-serialization attribute may start while the kernel
-// before it drains; it reads its descriptor, lets the next kernel be
-// scheduled (each block triggers on entry, so the next grid starts during
-// this grid's last wave), and waits for the previous grid to complete and
-// flush its memory before it reads anything that grid wrote.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename D>
 __device__ __forceinline__ void load_desc(D& dst, const D* src) {
@@ -1768,16 +1766,10 @@ __global__ void __launch_bounds__(kBlock) k_inject(Consts<T> k, State<T, S> s, I
 // ---------------------------------------------------------------------------
 enum ObserveMode { kObsInit = 0, kObsStep = 1 };
 
-template <typename T, typename S, bool RAW_IN>
-__global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, unsigned mask, int mode,
-                                                    T* phi_o, T* rho_o, T* u_o, T* P_o, T* p_o, T* mu_o) {
-  const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
-  const size_t N = (size_t)k.N;
-  const uint8_t c = s.cls[n];
-  const unsigned e = sidx(k, n);
-  const T phi = s.phi_out[e];
-  const T rho = phi * k.rho_l + (T(1) - phi) * k.rho_g;
+// phi, rho and u of one node.
+template <typename T, typename S>
+__device__ __forceinline__ void observe_own(const Consts<T>& k, const State<T, S>& s, int n, unsigned e, uint8_t c,
+                                            T phi, unsigned mask, int mode, T* phi_o, T* rho_o, T* u_o) {
   if (mask & 1u) {
     T v = phi;
     if (mode == kObsStep) {
@@ -1790,36 +1782,60 @@ __global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, 
     }
     phi_o[n] = v;
   }
-  if (mask & 2u) rho_o[n] = rho;
+  if (mask & 2u) rho_o[n] = phi * k.rho_l + (T(1) - phi) * k.rho_g;
   if (mask & 4u) {
+    const size_t N = (size_t)k.N;
     u_o[n] = s.u[e];
     u_o[N + n] = s.u[k.Np + e];
     u_o[2 * N + n] = s.u[2 * (size_t)k.Np + e];
   }
-  if (mask & (8u | 16u | 32u)) {
-    int ix, iy, iz;
-    const Nbr nb = make_nbr(n, k.nx, k.ny, k.nz, &ix, &iy, &iz);
-    if (mask & (8u | 16u)) {
-      T P = T(0);
-      if (mode == kObsStep) {
-        const T eps = (c & kPartial) ? s.eps[n] : T(0);
-        T g[Q];
-        fetch_pop<T, S, RAW_IN, false, false, false, true>(g, k, s.gin, s.phi_in, n, N, nb, c, eps, T(1));
-        P = seqsum(g);
-      }
-      if (mask & 8u) P_o[n] = P;
-      if (mask & 16u) p_o[n] = mode == kObsStep ? P * k.cs2 : rho * k.cs2;
+}
+
+// The fields without a stencil (phi, rho, u): a copy, bound by memory.  Apart
+// from the other fields' code it needs few registers (the form for all fields
+// took 26.6 us for phi and u of a 128x128x96 grid, this one 16.8).
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) k_observe_own(Consts<T> k, State<T, S> s, unsigned mask, int mode, T* phi_o,
+                                                        T* rho_o, T* u_o) {
+  const int n = blockIdx.x * kBlock + threadIdx.x;
+  if (n >= k.N) return;
+  const unsigned e = sidx(k, n);
+  observe_own(k, s, n, e, s.cls[n], s.phi_out[e], mask, mode, phi_o, rho_o, u_o);
+}
+
+template <typename T, typename S, bool RAW_IN>
+__global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, unsigned mask, int mode,
+                                                    T* phi_o, T* rho_o, T* u_o, T* P_o, T* p_o, T* mu_o) {
+  const int n = blockIdx.x * kBlock + threadIdx.x;
+  if (n >= k.N) return;
+  const size_t N = (size_t)k.N;
+  const uint8_t c = s.cls[n];
+  const unsigned e = sidx(k, n);
+  const T phi = s.phi_out[e];
+  observe_own(k, s, n, e, c, phi, mask, mode, phi_o, rho_o, u_o);
+  int ix, iy, iz;
+  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
+  if (mask & (8u | 16u)) {
+    T P = T(0);
+    if (mode == kObsStep) {
+      const T eps = (c & kPartial) ? s.eps[n] : T(0);
+      T g[Q];
+      fetch_pop<T, S, RAW_IN, false, false, false, true>(g, k, s.gin, s.phi_in, n, N, nb, c, eps, T(1));
+      P = seqsum(g);
     }
-    if (mask & 32u) {
-      T ps[Q];
+    if (mask & 8u) P_o[n] = P;
+    if (mask & 16u) p_o[n] = mode == kObsStep ? P * k.cs2 : (phi * k.rho_l + (T(1) - phi) * k.rho_g) * k.cs2;
+  }
+  if (mask & 32u) {
+    T ps[Q];
 #pragma unroll
-      for (int q = 1; q < Q; ++q) ps[q] = ldg(s.phi_out + sidx(k, nb.at(n, ex(q), ey(q), ez(q))));
-      auto nsolid = [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; };
-      T gx, gy, gz, lap;
-      if (mode == kObsStep) grad_lap<T, true>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
-      else grad_lap<T, false>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
-      mu_o[n] = chem_pot(k, c, phi, lap);
-    }
+    for (int q = 1; q < Q; ++q) ps[q] = ldg(s.phi_out + sidx(k, nb.at(n, ex(q), ey(q), ez(q))));
+    auto nsolid = [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; };
+    T gx, gy, gz, lap;
+    if (mode == kObsStep) grad_lap<T, true>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
+    else grad_lap<T, false>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
+    mu_o[n] = chem_pot(k, c, phi, lap);
   }
 }
 
@@ -1832,7 +1848,8 @@ __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S>
   const size_t N = (size_t)k.N;
   const uint8_t c = s.cls[n];
   int ix, iy, iz;
-  const Nbr nb = make_nbr(n, k.nx, k.ny, k.nz, &ix, &iy, &iz);
+  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q];
   if (f_o) {
@@ -1874,32 +1891,57 @@ __global__ void __launch_bounds__(kBlock) k_measure(int nx, int ny, int nz, cons
                                                    const uint8_t* __restrict__ cls, double* partials,
                                                    unsigned* counter, double* out, double* ext6) {
   const int N = nx * ny * nz;
-  double v[kMeasVals] = {0.0, -1e300, 1e300, -1e300, 1e300, -1e300, 1e300, -1e300, 0.0, 0.0, 0.0};
+  // The sum in float64, everything else as integers and values of T: the float64
+  // pipe is slow, and a reduction of all eleven values on it took 67 us of a
+  // 128x128x96 field (42 us this way).
+  double sum = 0.0;
+  T mx = -INFINITY;
+  bool nan = false;
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
+  unsigned cnt = 0;
+  unsigned long long sz = 0;
   for (int n = blockIdx.x * kBlock + threadIdx.x; n < N; n += gridDim.x * kBlock) {
     T p = phi[n];
     if (cls[n] & kSolid) p = T(0);
-    const double d = (double)p;
-    if (!(d == d)) v[10] = 1.0;
-    v[0] += d;
-    v[1] = d > v[1] ? d : v[1];
+    nan |= !(p == p);
+    sum += (double)p;
+    mx = p > mx ? p : mx;
     if (p > T(0.5)) {
       const int iz = n % nz, t = n / nz, iy = t % ny, ix = t / ny;
-      v[2] = fmin(v[2], (double)ix); v[3] = fmax(v[3], (double)ix);
-      v[4] = fmin(v[4], (double)iy); v[5] = fmax(v[5], (double)iy);
-      v[6] = fmin(v[6], (double)iz); v[7] = fmax(v[7], (double)iz);
-      v[8] += (double)iz;
-      v[9] += 1.0;
+      lo[0] = min(lo[0], ix); hi[0] = max(hi[0], ix);
+      lo[1] = min(lo[1], iy); hi[1] = max(hi[1], iy);
+      lo[2] = min(lo[2], iz); hi[2] = max(hi[2], iz);
+      sz += (unsigned)iz;
+      ++cnt;
     }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    double q[kMeasVals];
-#pragma unroll
-    for (int j = 0; j < kMeasVals; ++j) q[j] = __shfl_down_sync(0xffffffffu, v[j], o);
-    meas_merge(v, q);
+    sum += __shfl_down_sync(0xffffffffu, sum, o);
+    const T m = __shfl_down_sync(0xffffffffu, mx, o);
+    mx = m > mx ? m : mx;
+    sz += __shfl_down_sync(0xffffffffu, sz, o);
   }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    lo[j] = __reduce_min_sync(0xffffffffu, lo[j]);
+    hi[j] = __reduce_max_sync(0xffffffffu, hi[j]);
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  nan = __any_sync(0xffffffffu, nan);
   __shared__ double sw[kBlock / 32][kMeasVals];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double v[kMeasVals];
+  v[0] = sum;
+  v[1] = mx == -INFINITY ? -1e300 : (double)mx;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v[2 + 2 * j] = cnt ? (double)lo[j] : 1e300;
+    v[3 + 2 * j] = cnt ? (double)hi[j] : -1e300;
+  }
+  v[8] = (double)sz;
+  v[9] = (double)cnt;
+  v[10] = nan ? 1.0 : 0.0;
   if (lane == 0)
     for (int j = 0; j < kMeasVals; ++j) sw[wid][j] = v[j];
   __syncthreads();
@@ -1959,8 +2001,8 @@ __global__ void __launch_bounds__(kBlock) k_measure(int nx, int ny, int nz, cons
 
 // Total momentum sum_x rho(phi) u of a field pair (phi dense [N], u with
 // component stride us), rho = phi rho_l + (1 - phi) rho_g, accumulated in
-// float64 per node in a fixed order (block partials, then the last block
-// sums them in block order).  Writes out3.
+// float64 per node in a fixed order (block partials, then the last block's
+// tree over them).  Writes out3.
 // u in the state's layout: nh pairs (paired layout) or 0 (linear).
 struct NhOnly {
   int nh;
@@ -1972,42 +2014,50 @@ __global__ void __launch_bounds__(kBlock) k_momentum(int N, const T* __restrict_
   double m[3] = {0.0, 0.0, 0.0};
   const NhOnly lay{nh};
   for (int n = blockIdx.x * kBlock + threadIdx.x; n < N; n += gridDim.x * kBlock) {
-    const double p = (double)phi[n];
-    const double rho = p * rho_l + (1.0 - p) * rho_g;
+    const double rho = fma((double)phi[n], rho_l - rho_g, rho_g);
     const unsigned e = sidx(lay, n);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) m[d] += rho * (double)u[(size_t)d * us + e];
+    for (int d = 0; d < 3; ++d) m[d] = fma(rho, (double)u[(size_t)d * us + e], m[d]);
   }
   __shared__ double sw[kBlock / 32][3];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // the block's sums, in thread 0
+  auto block3 = [&] {
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double v = m[d];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sw[wid][d] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
     for (int d = 0; d < 3; ++d) {
-      double v = 0.0;
-      for (int w = 0; w < kBlock / 32; ++w) v += sw[w][d];
-      partials[(size_t)blockIdx.x * 3 + d] = v;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m[d] += __shfl_down_sync(0xffffffffu, m[d], o);
+      if (lane == 0) sw[wid][d] = m[d];
     }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int d = 0; d < 3; ++d)
+        for (int w = 1; w < kBlock / 32; ++w) m[d] += sw[w][d];
+  };
+  block3();
+  if (threadIdx.x == 0) {
+    for (int d = 0; d < 3; ++d) partials[(size_t)blockIdx.x * 3 + d] = m[d];
     __threadfence();
     s_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
   __syncthreads();
-  if (!s_last || threadIdx.x != 0) return;
+  if (!s_last) return;
   __threadfence();
+  // the last block: each thread a strided subset of the block sums, then the
+  // same tree (fixed order; one thread over 1,024 blocks took 150 us)
   const volatile double* pp = partials;
-  for (int d = 0; d < 3; ++d) {
-    double v = 0.0;
-    for (unsigned b = 0; b < gridDim.x; ++b) v += pp[(size_t)b * 3 + d];
-    out3[d] = v;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) m[d] = 0.0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += kBlock)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) m[d] += pp[(size_t)b * 3 + d];
+  __syncthreads();
+  block3();
+  if (threadIdx.x == 0) {
+    for (int d = 0; d < 3; ++d) out3[d] = m[d];
+    *counter = 0u;
   }
-  *counter = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -2078,28 +2128,6 @@ cudaError_t launch_step(const Consts<T>& k, const State<T, S>& s, const Tiling& 
              : launch_step_t<T, S, false, false, false>(k, s, tl, st);
 }
 
-// Launch with programmatic stream serialization (see pdl_wait).
-constexpr int kPdlOn = 1;  // 0: plain stream serialization
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl_bs(void (*fn)(KArgs...), int blocks, int threads, cudaStream_t st,
-                                 const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)blocks);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = threads == kPhisNT ? kPhisShared : 0;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = kPdlOn;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, args...);
-}
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*fn)(KArgs...), int blocks, cudaStream_t st, const Args&... args) {
-  return launch_pdl_bs(fn, blocks, kBlock, st, args...);
-}
-
 // Batched step kernels over a device case table; blocks: the grid (the part
 // of the block -> case table that starts at blk0).
 template <typename T, typename S>
@@ -2165,7 +2193,7 @@ cudaError_t launch_phis_batch(const void* cases, const unsigned short* b2c, int 
     if (blocks <= 0) return cudaSuccess;
     const cudaError_t e = phis_shared(k_phis_batch<T, S>);
     if (e != cudaSuccess) return e;
-    return launch_pdl_bs(k_phis_batch<T, S>, blocks, kPhisNT, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
+    return launch_pdl_sm(k_phis_batch<T, S>, blocks, kPhisNT, kPhisShared, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
   }
 }
 template <typename T, typename S>
@@ -2176,7 +2204,7 @@ cudaError_t launch_phis_one(const void* desc, cudaStream_t st) {
     const CaseDesc<T, S>& d = *static_cast<const CaseDesc<T, S>*>(desc);
     const cudaError_t e = phis_shared(k_phis_one<T, S>);
     if (e != cudaSuccess) return e;
-    return launch_pdl_bs(k_phis_one<T, S>, d.tile.blocks(), kPhisNT, st, d);
+    return launch_pdl_sm(k_phis_one<T, S>, d.tile.blocks(), kPhisNT, kPhisShared, st, d);
   }
 }
 template <typename T, typename S>
@@ -2312,7 +2340,8 @@ template <typename T, typename S>
 cudaError_t launch_observe(const Consts<T>& k, const State<T, S>& s, bool raw_in, unsigned mask, int mode,
                            T* phi, T* rho, T* u, T* P, T* p, T* mu, cudaStream_t st) {
   const int grid = (k.N + kBlock - 1) / kBlock;
-  if (raw_in) k_observe<T, S, true><<<grid, kBlock, 0, st>>>(k, s, mask, mode, phi, rho, u, P, p, mu);
+  if (!(mask & (8u | 16u | 32u))) k_observe_own<T, S><<<grid, kBlock, 0, st>>>(k, s, mask, mode, phi, rho, u);
+  else if (raw_in) k_observe<T, S, true><<<grid, kBlock, 0, st>>>(k, s, mask, mode, phi, rho, u, P, p, mu);
   else k_observe<T, S, false><<<grid, kBlock, 0, st>>>(k, s, mask, mode, phi, rho, u, P, p, mu);
   return cudaGetLastError();
 }
