@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "lbm_common.cuh"
+#include "lbm_launch.cuh"
 
 namespace lbm {
 namespace d2 {
@@ -50,8 +51,9 @@ struct Nb2 {
   int ox[3], oy[3];
   __device__ __forceinline__ int at(int n, int dx, int dy) const { return n + ox[dx + 1] + oy[dy + 1]; }
 };
-__device__ __forceinline__ Nb2 make_nb2(int n, int nx, int ny) {
-  const int ix = n / ny, iy = n - (n / ny) * ny;
+template <typename T>
+__device__ __forceinline__ Nb2 make_nb2(const Consts<T>& k, int n) {
+  const int nx = k.nx, ny = k.ny, ix = (int)k.dy.div((unsigned)n), iy = n - ix * ny;
   Nb2 b;
   b.ox[0] = ix == 0 ? (nx - 1) * ny : -ny;
   b.ox[1] = 0;
@@ -204,18 +206,42 @@ __device__ __forceinline__ T edot(int q, T a0, T a1) {
   return T(0);
 }
 
+// x / d, correctly rounded, from r = 1 / d correctly rounded: q = x r, then
+// q + r (x - d q) with the remainder exact in a fused multiply-add (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34(1), 1990).  Three operations where the division's general
+// form takes about ten; several quotients by one d share its reciprocal.  The
+// same values as x / d except where the remainder underflows (|x| below ~1e-31
+// in float) and for infinite x (NaN).
+template <typename T>
+struct Div {
+  T d, r;
+  __device__ __forceinline__ T operator()(T x) const {
+    const T q = x * r;
+    return fma(fma(-d, q, x), r, q);
+  }
+};
+__device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
+__device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
+template <typename T>
+__device__ __forceinline__ Div<T> by(T d) { return Div<T>{d, rcp_rn(d)}; }
+template <typename T>
+__device__ __forceinline__ Div<T> by_cs2() { return Div<T>{cs2<T>(), T(1) / cs2<T>()}; }
+template <typename T>
+__device__ __forceinline__ Div<T> by_two_cs2() { return Div<T>{T(2) * cs2<T>(), T(1) / (T(2) * cs2<T>())}; }
+
 // t[q] = (c e_q . (a0, a1)) / d for every q, with one division per opposite
 // pair (q, opp q): e_opp(q) . a = -(e_q . a) exactly, and (c (-x)) / d =
 // -((c x) / d) in IEEE arithmetic, so the opposite's value is the negation.
-// c and d depend on the weight class (cw: per q); the rest value is
-// (c 0) / d.  Same values as the per-q expression of the reference.
+// c and d depend on the weight class (cw: per q); the rest value is 0.
+// Same values as the per-q expression of the reference.
 template <typename T, typename CW>
-__device__ __forceinline__ void pair_div(T (&t)[Q9], T a0, T a1, CW cw, T d) {
-  t[0] = (cw(0) * edot(0, a0, a1)) / d;
+__device__ __forceinline__ void pair_div(T (&t)[Q9], T a0, T a1, CW cw, const Div<T>& d) {
+  t[0] = T(0);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int q = i < 2 ? 1 + 2 * i : 5 + (i - 2);  // 1, 3, 5, 6
-    t[q] = (cw(q) * edot(q, a0, a1)) / d;
+    t[q] = d(cw(q) * edot(q, a0, a1));
     t[opp(q)] = -t[q];
   }
 }
@@ -349,6 +375,8 @@ __global__ void __launch_bounds__(kBlock) k2_init(Consts<T> k, State<T, T> s, co
 // blocks publish partial sums.
 template <typename T, bool RAW>
 __global__ void __launch_bounds__(kBlock) k2_phi(Consts<T> k, State<T, T> s) {
+  pdl_trigger();
+  pdl_wait();  // f of the previous update kernel
   double pd = 0.0;
   unsigned long long pu = 0ull;
   bool nan = false;
@@ -356,7 +384,7 @@ __global__ void __launch_bounds__(kBlock) k2_phi(Consts<T> k, State<T, T> s) {
     const uint8_t c = s.cls[n];
     T phi = T(0);
     if (!(c & kSolid)) {
-      const Nb2 nb = make_nb2(n, k.nx, k.ny);
+      const Nb2 nb = make_nb2(k, n);
       const T eps = (c & kPartial) ? s.eps[n] : T(0);
       T v[Q9];
       fetch_f9<T, RAW>(v, k, s, n, nb, c, eps);
@@ -387,7 +415,7 @@ __global__ void __launch_bounds__(kBlock) k2_mu(Consts<T> k, State<T, T> s) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const uint8_t c = s.cls[n];
-  const Nb2 nb = make_nb2(n, k.nx, k.ny);
+  const Nb2 nb = make_nb2(k, n);
   const T phi = s.phi_out[n];
   T gx, gy, lap;
   grad_lap<T, true>(k, s, n, nb, c, phi, s.phi_out, gx, gy, lap);
@@ -401,7 +429,7 @@ __global__ void __launch_bounds__(kBlock) k2_gradmu(Consts<T> k, State<T, T> s) 
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const uint8_t c = s.cls[n];
-  const Nb2 nb = make_nb2(n, k.nx, k.ny);
+  const Nb2 nb = make_nb2(k, n);
   const T mu = s.mu[n];
   const bool gh = k.wetting && (c & kBoundary);
   const float n0 = gh ? s.wn[n] : 0.0f, n1 = gh ? s.wn[k.N + n] : 0.0f;
@@ -429,16 +457,23 @@ __global__ void __launch_bounds__(kBlock) k2_gradmu(Consts<T> k, State<T, T> s) 
 // than a factor of two apart).
 template <typename T, bool RAW, bool FIRST, bool GMU, bool OMEGA1 = false>
 __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, double ac) {
+  pdl_trigger();
+  pdl_wait();  // phi of k2_phi (grad mu of k2_gradmu)
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const int Np = k.Np;
   const uint8_t c = s.cls[n];
-  const Nb2 nb = make_nb2(n, k.nx, k.ny);
+  const Nb2 nb = make_nb2(k, n);
   const T phi = s.phi_out[n];
   T gx, gy, lap;
   grad_lap<T, true>(k, s, n, nb, c, phi, s.phi_out, gx, gy, lap);
   const T rho = phi * k.rho_l + (T(1) - phi) * k.rho_g;
-  const T rho_eff = rho < k.rho_floor ? k.rho_floor : rho;
+  // divisors rho_eff and rho_eff cs2: in the gas and half of the interface rho_eff is the floor
+  Div<T> by_rho{k.rho_floor, k.inv_floor}, by_rho_cs2{k.rho_floor * cs2<T>(), k.inv_floor_cs2};
+  if (!(rho < k.rho_floor)) {
+    by_rho = by(rho);
+    by_rho_cs2 = by(rho * cs2<T>());
+  }
   const T mu = GMU ? s.mu[n] : chem_pot(k, c, phi, lap);
 
   // geometric contact-angle gradient correction (fe_wetting.py:448-539); the
@@ -478,9 +513,9 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
   T sxx = T(0), syy = T(0), sxy = T(0);
   {
     const T usq = uo0 * uo0 + uo1 * uo1;
-    const T b = usq / (T(2) * cs2<T>());
+    const T b = by_two_cs2<T>()(usq);
     T ecs[Q9];
-    pair_div(ecs, uo0, uo1, [](int) { return T(1); }, cs2<T>());
+    pair_div(ecs, uo0, uo1, [](int) { return T(1); }, by_cs2<T>());
 #pragma unroll
     for (int q = 1; q < Q9; ++q) {
       const T ec = ecs[q];
@@ -524,7 +559,7 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
       fy = false;
     }
   }
-  T u0 = ux + (T(0.5) * F0) / rho_eff, u1 = uy + (T(0.5) * F1) / rho_eff;
+  T u0 = ux + by_rho(T(0.5) * F0), u1 = uy + by_rho(T(0.5) * F1);
   if (c & kSolid) u0 = u1 = T(0);
 
   // 7. interface source (:450-494)
@@ -539,10 +574,15 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
     S0 = S0 + (k.mob * (mx - gx)) * k.guo;
     S1 = S1 + (k.mob * (my - gy)) * k.guo;
   } else {
-    T gm = sqrt(gx * gx + gy * gy);
-    gm = gm < T(1e-10) ? T(1e-10) : gm;
-    const T lam = ((T(4) * phi) * (T(1) - phi)) / k.W;
-    T sx = ((k.cs2 * lam) * (gx / gm)) * k.ac_scale, sy = ((k.cs2 * lam) * (gy / gm)) * k.ac_scale;
+    // |grad| clamped to 1e-10: below 1e-21 (most of the gas) its square needs no root
+    const T g2 = gx * gx + gy * gy;
+    Div<T> by_gm{T(1e-10), T(1) / T(1e-10)};
+    if (!(g2 < T(1e-21))) {
+      const T gm = sqrt(g2);
+      by_gm = by(gm < T(1e-10) ? T(1e-10) : gm);
+    }
+    const T lam = Div<T>{k.W, k.inv_W}((T(4) * phi) * (T(1) - phi));
+    T sx = ((k.cs2 * lam) * by_gm(gx)) * k.ac_scale, sy = ((k.cs2 * lam) * by_gm(gy)) * k.ac_scale;
     if (k.wetting) {
       const T red = T(1) - k.sharpen_reduce * k.ww[c >> kWwShift];
       sx = sx * red;
@@ -569,12 +609,12 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
   }
   ns = T(1) - om * T(0.5);
   const T usq = u0 * u0 + u1 * u1;
-  const T b = usq / (T(2) * cs2<T>());
+  const T b = by_two_cs2<T>()(usq);
   const T acT = (T)ac;
   T ecs[Q9], src[Q9], G[Q9];
-  pair_div(ecs, u0, u1, [](int) { return T(1); }, cs2<T>());
-  pair_div(src, S0, S1, [&](int q) { return acT * w<T>(q); }, cs2<T>());
-  pair_div(G, F0, F1, [&](int q) { return ns * w<T>(q); }, rho_eff * cs2<T>());
+  pair_div(ecs, u0, u1, [](int) { return T(1); }, by_cs2<T>());
+  pair_div(src, S0, S1, [&](int q) { return acT * w<T>(q); }, by_cs2<T>());
+  pair_div(G, F0, F1, [&](int q) { return ns * w<T>(q); }, by_rho_cs2);
 #pragma unroll
   for (int q = 0; q < Q9; ++q) {
     const T ec = ecs[q];
@@ -599,7 +639,7 @@ __global__ void __launch_bounds__(kBlock) k2_observe(Consts<T> k, State<T, T> s,
   const uint8_t c = s.cls[n];
   const T phi = s.phi_out[n];
   const T rho = phi * k.rho_l + (T(1) - phi) * k.rho_g;
-  const Nb2 nb = make_nb2(n, k.nx, k.ny);
+  const Nb2 nb = make_nb2(k, n);
   if (mask & 1u) {
     T v = phi;
     if (mode == 1) {
@@ -642,7 +682,7 @@ __global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const uint8_t c = s.cls[n];
-  const Nb2 nb = make_nb2(n, k.nx, k.ny);
+  const Nb2 nb = make_nb2(k, n);
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q9];
   if (f_o) {
@@ -673,7 +713,7 @@ __global__ void __launch_bounds__(kBlock) k2_inject(Consts<T> k, State<T, T> s, 
   if (n < k.N) {
     const int Np = k.Np;
     const uint8_t c = s.cls[n];
-    const Nb2 nb = make_nb2(n, k.nx, k.ny);
+    const Nb2 nb = make_nb2(k, n);
     const int ix = n / k.ny, iy = n - (n / k.ny) * k.ny;
     // the droplet as the reference builds it: float64 profile, stored as float32
     const double dx = ix - ip.c[0], dy = iy - ip.c[1];
@@ -767,9 +807,7 @@ template <typename T>
 cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool first, double ac, cudaStream_t st,
                           cudaEvent_t mid) {
   const int nb = d2::blocks_of(k.N), np = d2::phi_blocks_of(k.N);
-  if (raw) d2::k2_phi<T, true><<<np, kBlock, 0, st>>>(k, s);
-  else d2::k2_phi<T, false><<<np, kBlock, 0, st>>>(k, s);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = raw ? launch_pdl(d2::k2_phi<T, true>, np, st, k, s) : launch_pdl(d2::k2_phi<T, false>, np, st, k, s);
   if (e != cudaSuccess) return e;
   if (mid) {
     e = cudaEventRecord(mid, st);
@@ -780,9 +818,9 @@ cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bo
     d2::k2_mu<T><<<nb, kBlock, 0, st>>>(k, s);
     d2::k2_gradmu<T><<<nb, kBlock, 0, st>>>(k, s);
   }
-#define LBM_UPD2(R, F)                                                      \
-  if (gmu) d2::k2_update<T, R, F, true><<<nb, kBlock, 0, st>>>(k, s, ac);  \
-  else d2::k2_update<T, R, F, false><<<nb, kBlock, 0, st>>>(k, s, ac);
+#define LBM_UPD2(R, F)                                                        \
+  return gmu ? launch_pdl(d2::k2_update<T, R, F, true>, nb, st, k, s, ac)     \
+             : launch_pdl(d2::k2_update<T, R, F, false>, nb, st, k, s, ac);
   if (raw && first) {
     LBM_UPD2(true, true)
   } else if (raw) {
@@ -790,12 +828,11 @@ cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bo
   } else if (first) {
     LBM_UPD2(false, true)
   } else if (!gmu && k.omega_f == T(1)) {
-    d2::k2_update<T, false, false, false, true><<<nb, kBlock, 0, st>>>(k, s, ac);
+    return launch_pdl(d2::k2_update<T, false, false, false, true>, nb, st, k, s, ac);
   } else {
     LBM_UPD2(false, false)
   }
 #undef LBM_UPD2
-  return cudaGetLastError();
 }
 
 template <typename T>
