@@ -35,6 +35,8 @@ from . import _native as nat
 from .lattice import D2Q9, D3Q19
 
 _STAB = {"fakhari": 0, "liang": 1, "none": 2}
+# read-out fields in the order of the library's mask bits (nat.FIELD_*) and arguments
+_FIELD_INDEX = {"phi": 0, "rho": 1, "u": 2, "P": 3, "p": 4, "mu_phi": 5}
 
 
 def _host_array(x, dtype):
@@ -329,8 +331,9 @@ class AllenCahnSolver:
         """``nsteps`` time steps in one call."""
         if not self._initialized:
             raise RuntimeError("init_fields must be called before step()")
-        nat.check(self._lib.lbm_step(self._h, int(nsteps), nat.stream_ptr(stream)), "lbm_step")
-        self.step_count += int(nsteps)
+        n = int(nsteps)
+        nat.check(self._lib.lbm_step(self._h, n, nat.stream_ptr(stream)), "lbm_step")
+        self.step_count += n
         self.t += float(nsteps)
         self._cache.clear()
 
@@ -363,18 +366,16 @@ class AllenCahnSolver:
         if missing:
             if not self._initialized:
                 raise RuntimeError("fields are defined after init_fields")
-            bits = {"phi": nat.FIELD_PHI, "rho": nat.FIELD_RHO, "u": nat.FIELD_U, "P": nat.FIELD_P,
-                    "p": nat.FIELD_PRESS, "mu_phi": nat.FIELD_MU}
             mask = 0
             out = {}
+            ptrs = [None] * 6
             for k in missing:
+                i = _FIELD_INDEX[k]
                 shp = (self.ndim,) + self.shape if k == "u" else self.shape
-                out[k] = torch.empty(shp, dtype=self.dtype, device=self.device)
-                mask |= bits[k]
-            nat.check(self._lib.lbm_get_fields(
-                self._h, mask, nat.ptr(out.get("phi")), nat.ptr(out.get("rho")), nat.ptr(out.get("u")),
-                nat.ptr(out.get("P")), nat.ptr(out.get("p")), nat.ptr(out.get("mu_phi")),
-                nat.stream_ptr()), "lbm_get_fields")
+                t = out[k] = torch.empty(shp, dtype=self.dtype, device=self.device)
+                ptrs[i] = t.data_ptr()
+                mask |= 1 << i
+            nat.check(self._lib.lbm_get_fields(self._h, mask, *ptrs, nat.stream_ptr()), "lbm_get_fields")
             self._cache.update(out)
         return [self._cache[k] for k in want]
 
