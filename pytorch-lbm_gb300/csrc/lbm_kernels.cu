@@ -1649,12 +1649,19 @@ __global__ void __launch_bounds__(kBlock) k_init(Consts<T> k, State<T, S> s, con
     S* f = const_cast<S*>(s.fin);
     S* g = const_cast<S*>(s.gin);
     const unsigned e = sidx(k, n);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const T ec = edot(q, v0, v1, v2) / k.cs2;
+    // e_q.u / cs2 is odd in q: one division per opposite pair
+    auto put = [&](int q, T ec) {
       // the state right after init is read in place (RAW): deviation reference = own phi
       f[(size_t)q * k.Np + e] = IO::st_f(phi * (k.w[q] * (((T(1) + ec) + ec * ec / T(2)) - b)), q, phi, k);
       g[(size_t)q * k.Np + e] = IO::st_g(T(0) * k.w[q] + k.w[q] * ((ec + ec * ec / T(2)) - b), q, k);
+    };
+    put(0, T(0));
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const int q = pair_first(i);
+      const T ec = edot(q, v0, v1, v2) / k.cs2;
+      put(q, ec);
+      put(opp(q), -ec);
     }
     s.u[e] = v0;
     s.u[k.Np + e] = v1;
