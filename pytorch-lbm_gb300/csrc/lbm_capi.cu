@@ -1797,6 +1797,11 @@ struct LbmBatch {
   int phi_blocks_om1 = 0;               // linear phi blocks of the omega_f == 1 cases (the first of them)
   bool graph_s = false;                 // the graph's phi pass reads S
   cudaStream_t cap = nullptr;           // stream used to capture the two-step graph
+  // large grids (batch_apart): each case steps through its own launches on one of these streams
+  std::vector<cudaStream_t> lanes;
+  std::vector<int> lane_of;             // of each case
+  std::vector<cudaEvent_t> joins;       // one per lane
+  cudaEvent_t fork = nullptr;
   cudaGraphExec_t graph = nullptr;
 };
 
@@ -1949,6 +1954,96 @@ int batch_graph(LbmBatch* b, bool phis_in) {
   return LBM_OK;
 }
 
+// Whether the cases of a batch step apart, each through the launches of a grid
+// alone, on up to kApartLanes streams.  The kernels of a grid alone have their
+// constants and pointers as constant-bank operands instead of a shared-memory
+// descriptor, and one case's phi pass (bound by its instructions) runs beside
+// another's update (bound by memory); but each case costs two launches a step.
+// us per step of a batch, table kernels / 1, 2, 4, 8 streams:
+//   8 x 48^3      float 75 / 141, 83, 75, 73      half  88 / 162, 92, 81, 80
+//   8 x 80x80x64  float 245 / 309, 217, 212, 216  half 266 / 355, 242, 223, 224
+//   6 x 128x128x96 float 634 / 614, 552, 562, 571 half 661 / 663, 556, 561, 563
+//   2 x 192x192x128 float 597 / 551, 532          half 611 / 539, 502
+// Below a mean of 48^3 nodes the launches bound it.  (Linear layouts in 32-bit
+// compute; the cooperative form is one launch by request.)
+constexpr int64_t kApartNodes = 110000;
+constexpr int kApartLanes = 4;
+bool batch_apart(const LbmBatch* b) {
+  if (b->coop || b->prec == LBM_F64) return false;
+  int64_t nodes = 0;
+  for (const LbmHandle* h : b->h) {
+    if (h->paired) return false;
+    nodes += h->N;
+  }
+  return nodes >= (int64_t)b->h.size() * kApartNodes;
+}
+
+// Streams of the cases that step apart: the largest case to the least loaded stream.
+cudaError_t apart_create(LbmBatch* b) {
+  const size_t n = b->h.size(), lanes = std::min<size_t>(n, kApartLanes);
+  cudaError_t e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+  for (size_t i = 0; i < lanes && e == cudaSuccess; ++i) {
+    cudaStream_t st = nullptr;
+    cudaEvent_t ev = nullptr;
+    e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) b->lanes.push_back(st);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) b->joins.push_back(ev);
+  }
+  if (e != cudaSuccess) return e;
+  std::vector<int> order(n);
+  for (size_t i = 0; i < n; ++i) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return b->h[i]->N > b->h[j]->N; });
+  std::vector<int64_t> load(lanes, 0);
+  b->lane_of.assign(n, 0);
+  for (int i : order) {
+    const size_t l = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+    b->lane_of[i] = (int)l;
+    load[l] += b->h[i]->N;
+  }
+  return cudaSuccess;
+}
+
+// nsteps steps of every case through the kernels of a grid alone; the work of
+// `st` so far comes before them, what is put on `st` later after them.
+// advance: false re-reads the current state (autotuning).
+template <typename T, typename S>
+int apart_step_t(LbmBatch* b, int nsteps, bool advance, cudaStream_t st) {
+  CUDA_TRY(cudaEventRecord(b->fork, st));
+  for (cudaStream_t l : b->lanes) CUDA_TRY(cudaStreamWaitEvent(l, b->fork, 0));
+  int rc = LBM_OK;
+  for (int k = 0; k < nsteps && rc == LBM_OK; ++k)
+    for (size_t i = 0; i < b->h.size() && rc == LBM_OK; ++i) {
+      LbmHandle* h = b->h[i];
+      const int per = h->phi_per_thread, bs = h->upd_block;
+      h->phi_per_thread = b->phi_per_thread;
+      h->upd_block = b->upd_block;
+      rc = launch_next<T, S>(h, Tiling{}, b->lanes[b->lane_of[i]], nullptr);
+      h->phi_per_thread = per;
+      h->upd_block = bs;
+      if (rc == LBM_OK && advance) {
+        h->sform = wants_s(h);
+        h->last_raw_in = h->obs_init = false;
+        h->cur ^= 1;
+        h->pc ^= 1;
+        h->c_last ^= 1;
+        ++h->steps;
+      }
+    }
+  for (size_t l = 0; l < b->lanes.size(); ++l) {
+    CUDA_TRY(cudaEventRecord(b->joins[l], b->lanes[l]));
+    CUDA_TRY(cudaStreamWaitEvent(st, b->joins[l], 0));
+  }
+  return rc;
+}
+int apart_step(LbmBatch* b, int nsteps, bool advance, cudaStream_t st) {
+  return with_types(b->prec, [&](auto tag) {
+    return apart_step_t<typename decltype(tag)::T, typename decltype(tag)::S>(b, nsteps, advance, st);
+  });
+}
+
+bool steps_apart(const LbmBatch* b) { return !b->lanes.empty() && batch_apart(b); }
+
 void batch_advance(LbmBatch* b, int nsteps) {
   for (LbmHandle* h : b->h) {
     if (nsteps & 1) {
@@ -2008,7 +2103,9 @@ int lbm_batch_create(LbmHandle* const* handles, int n, LbmBatch** out) {
     lbm_batch_destroy(b);
     return fail(LBM_E_CUDA, std::string("lbm_batch_create: ") + cudaGetErrorString(e));
   }
-  const int rc = batch_layout(b);
+  if (batch_apart(b)) e = apart_create(b);
+  const int rc = e == cudaSuccess ? batch_layout(b)
+                                  : fail(LBM_E_CUDA, std::string("lbm_batch_create: ") + cudaGetErrorString(e));
   if (rc != LBM_OK) {
     lbm_batch_destroy(b);
     return rc;
@@ -2027,6 +2124,9 @@ int lbm_batch_destroy(LbmBatch* b) {
   if (b->staging) cudaFreeHost(b->staging);
   if (b->staged) cudaEventDestroy(b->staged);
   if (b->cap) cudaStreamDestroy(b->cap);
+  for (cudaStream_t l : b->lanes) cudaStreamDestroy(l);
+  for (cudaEvent_t ev : b->joins) cudaEventDestroy(ev);
+  if (b->fork) cudaEventDestroy(b->fork);
   delete b;
   return LBM_OK;
 }
@@ -2053,6 +2153,7 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
     --rest;
   }
   if (rest == 0) return LBM_OK;
+  if (steps_apart(b)) return apart_step(b, rest, true, st);
   bool phis_in = false;
   int rc = batch_form(b, st, &phis_in);
   if (rc == LBM_OK) rc = batch_fill(b, st);
@@ -2121,6 +2222,7 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
   bool phis_in = false;
+  const bool apart = steps_apart(b);
   int best = b->phi_per_thread, best_bs = b->upd_block, rc = batch_form(b, st, &phis_in);
   float best_t = 1e30f;
   for (int bs : {128, kBlock})
@@ -2130,11 +2232,17 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
     b->phi_per_thread = per;
     b->upd_block = bs;
     rc = batch_layout(b);
-    if (rc == LBM_OK) rc = batch_fill(b, st);
+    if (rc == LBM_OK && !apart) rc = batch_fill(b, st);
     if (rc != LBM_OK) break;
-    cudaError_t e = batch_launch(b, 0, phis_in, st);  // warm-up
+    auto once = [&] {
+      if (!apart) return batch_launch(b, 0, phis_in, st);
+      rc = apart_step(b, 1, false, st);
+      return cudaSuccess;
+    };
+    cudaError_t e = once();  // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = batch_launch(b, 0, phis_in, st);
+    for (int r = 0; r < reps && e == cudaSuccess && rc == LBM_OK; ++r) e = once();
+    if (rc != LBM_OK) break;
     if (e == cudaSuccess) e = cudaEventRecord(e1, st);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;
