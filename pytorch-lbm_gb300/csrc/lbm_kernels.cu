@@ -1813,36 +1813,43 @@ __global__ void __launch_bounds__(kBlock) k_observe_own(Consts<T> k, State<T, S>
 template <typename T, typename S, bool RAW_IN>
 __global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, unsigned mask, int mode,
                                                     T* phi_o, T* rho_o, T* u_o, T* P_o, T* p_o, T* mu_o) {
-  const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
-  const size_t N = (size_t)k.N;
-  const uint8_t c = s.cls[n];
-  const unsigned e = sidx(k, n);
-  const T phi = s.phi_out[e];
-  observe_own(k, s, n, e, c, phi, mask, mode, phi_o, rho_o, u_o);
-  int ix, iy, iz;
-  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
-  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
-  if (mask & (8u | 16u)) {
-    T P = T(0);
-    if (mode == kObsStep) {
-      const T eps = (c & kPartial) ? s.eps[n] : T(0);
-      T g[Q];
-      fetch_pop<T, S, RAW_IN, false, false, false, true>(g, k, s.gin, s.phi_in, n, N, nb, c, eps, T(1));
-      P = seqsum(g);
+  auto node = [&](const auto& a) {
+    const int n = a.n;
+    const uint8_t c = s.cls[n];
+    const unsigned e = sidx(k, n);
+    const T phi = ld_pol(s.phi_out + e, a.pol.keep);
+    observe_own(k, s, n, e, c, phi, mask, mode, phi_o, rho_o, u_o);
+    if (mask & (8u | 16u)) {
+      T P = T(0);
+      if (mode == kObsStep) {
+        const T eps = (c & kPartial) ? s.eps[n] : T(0);
+        T g[Q];
+        a.load_g(g, c, eps);
+        P = seqsum(g);
+      }
+      if (mask & 8u) P_o[n] = P;
+      if (mask & 16u) p_o[n] = mode == kObsStep ? P * k.cs2 : (phi * k.rho_l + (T(1) - phi) * k.rho_g) * k.cs2;
     }
-    if (mask & 8u) P_o[n] = P;
-    if (mask & 16u) p_o[n] = mode == kObsStep ? P * k.cs2 : (phi * k.rho_l + (T(1) - phi) * k.rho_g) * k.cs2;
-  }
-  if (mask & 32u) {
-    T ps[Q];
+    if (mask & 32u) {
+      T ps[Q];
 #pragma unroll
-    for (int q = 1; q < Q; ++q) ps[q] = ldg(s.phi_out + sidx(k, nb.at(n, ex(q), ey(q), ez(q))));
-    auto nsolid = [&](int q) { return (s.cls[nb.at(n, ex(q), ey(q), ez(q))] & kSolid) != 0; };
-    T gx, gy, gz, lap;
-    if (mode == kObsStep) grad_lap<T, true>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
-    else grad_lap<T, false>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
-    mu_o[n] = chem_pot(k, c, phi, lap);
+      for (int q = 1; q < Q; ++q) ps[q] = a.phi_at(q);
+      auto nsolid = [&](int q) { return a.solid_at(q); };
+      T gx, gy, gz, lap;
+      if (mode == kObsStep) grad_lap<T, true>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
+      else grad_lap<T, false>(k, s, n, c, phi, ps, nsolid, gx, gy, gz, lap);
+      mu_o[n] = chem_pot(k, c, phi, lap);
+    }
+  };
+  if constexpr (RAW_IN) {
+    const int n = blockIdx.x * kBlock + threadIdx.x;
+    if (n >= k.N) return;
+    const Pol pol = Pol::make();
+    int ix, iy, iz;
+    decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+    node(NodeAt<T, S, true, true>(k, s, pol, make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz), n));
+  } else {
+    with_node(k, s, blockIdx.x * kBlock, kBlock, node);
   }
 }
 
@@ -1874,23 +1881,59 @@ __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S>
 // ---------------------------------------------------------------------------
 // Spread diagnostics over a phi field (fe_measure.py:11-82 + sweep z_com):
 // volume, C_max, extents of phi > 0.5 (solid excluded), z centre, count, NaN.
-// Partials per block: [sum, max, minx, maxx, miny, maxy, minz, maxz, sumz, count, nan]
+// One partial per block, merged in a fixed order by the last block to finish.
+// The sum is in float64, everything else in integers and values of T: the
+// float64 pipe is slow, and it bounds the pass where more than the sum is
+// reduced on it (128x128x96: 67 us with all eleven values in float64, 42 us
+// with the merges between warps and blocks there, 21 us without).
 // ---------------------------------------------------------------------------
-constexpr int kMeasVals = 11;
+constexpr int kMeasVals = 11;  // doubles of room per block's partial
 
-// r <- merge(r, q): sum, max, (min, max) x 3 axes, sum, sum, max
-template <typename A, typename B>
-__device__ __forceinline__ void meas_merge(A& r, const B& q) {
-  r[0] += q[0];
-  r[1] = fmax(r[1], (double)q[1]);
+template <typename T>
+struct Meas {
+  double sum = 0.0;
+  unsigned long long sz = 0;  // of the nodes with phi > 0.5: sum of z, count, extents
+  unsigned cnt = 0;
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
+  unsigned nan = 0;
+  T mx = -INFINITY;
+};
+
+template <typename T>
+__device__ __forceinline__ void meas_merge(Meas<T>& r, const Meas<T>& q) {
+  r.sum += q.sum;
+  r.sz += q.sz;
+  r.cnt += q.cnt;
 #pragma unroll
-  for (int j = 2; j < 8; j += 2) {
-    r[j] = fmin(r[j], (double)q[j]);
-    r[j + 1] = fmax(r[j + 1], (double)q[j + 1]);
+  for (int j = 0; j < 3; ++j) {
+    r.lo[j] = min(r.lo[j], q.lo[j]);
+    r.hi[j] = max(r.hi[j], q.hi[j]);
   }
-  r[8] += q[8];
-  r[9] += q[9];
-  r[10] = fmax(r[10], (double)q[10]);
+  r.nan |= q.nan;
+  r.mx = q.mx > r.mx ? q.mx : r.mx;
+}
+
+// Merges the block's threads into thread 0's value.
+template <typename T>
+__device__ __forceinline__ void meas_block(Meas<T>& v, Meas<T>* sw) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v.sum += __shfl_down_sync(0xffffffffu, v.sum, o);
+    v.sz += __shfl_down_sync(0xffffffffu, v.sz, o);
+    const T m = __shfl_down_sync(0xffffffffu, v.mx, o);
+    v.mx = m > v.mx ? m : v.mx;
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    v.lo[j] = __reduce_min_sync(0xffffffffu, v.lo[j]);
+    v.hi[j] = __reduce_max_sync(0xffffffffu, v.hi[j]);
+  }
+  v.cnt = __reduce_add_sync(0xffffffffu, v.cnt);
+  v.nan = __reduce_or_sync(0xffffffffu, v.nan);
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < kBlock / 32; ++w) meas_merge(v, sw[w]);
 }
 
 template <typename T>
@@ -1898,64 +1941,30 @@ __global__ void __launch_bounds__(kBlock) k_measure(int nx, int ny, int nz, cons
                                                    const uint8_t* __restrict__ cls, double* partials,
                                                    unsigned* counter, double* out, double* ext6) {
   const int N = nx * ny * nz;
-  // The sum in float64, everything else as integers and values of T: the float64
-  // pipe is slow, and a reduction of all eleven values on it took 67 us of a
-  // 128x128x96 field (42 us this way).
-  double sum = 0.0;
-  T mx = -INFINITY;
-  bool nan = false;
-  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
-  unsigned cnt = 0;
-  unsigned long long sz = 0;
+  Meas<T> v;
+#pragma unroll 4
   for (int n = blockIdx.x * kBlock + threadIdx.x; n < N; n += gridDim.x * kBlock) {
     T p = phi[n];
     if (cls[n] & kSolid) p = T(0);
-    nan |= !(p == p);
-    sum += (double)p;
-    mx = p > mx ? p : mx;
+    v.nan |= !(p == p);
+    v.sum += (double)p;
+    v.mx = p > v.mx ? p : v.mx;
     if (p > T(0.5)) {
       const int iz = n % nz, t = n / nz, iy = t % ny, ix = t / ny;
-      lo[0] = min(lo[0], ix); hi[0] = max(hi[0], ix);
-      lo[1] = min(lo[1], iy); hi[1] = max(hi[1], iy);
-      lo[2] = min(lo[2], iz); hi[2] = max(hi[2], iz);
-      sz += (unsigned)iz;
-      ++cnt;
+      v.lo[0] = min(v.lo[0], ix); v.hi[0] = max(v.hi[0], ix);
+      v.lo[1] = min(v.lo[1], iy); v.hi[1] = max(v.hi[1], iy);
+      v.lo[2] = min(v.lo[2], iz); v.hi[2] = max(v.hi[2], iz);
+      v.sz += (unsigned)iz;
+      ++v.cnt;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sum += __shfl_down_sync(0xffffffffu, sum, o);
-    const T m = __shfl_down_sync(0xffffffffu, mx, o);
-    mx = m > mx ? m : mx;
-    sz += __shfl_down_sync(0xffffffffu, sz, o);
-  }
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    lo[j] = __reduce_min_sync(0xffffffffu, lo[j]);
-    hi[j] = __reduce_max_sync(0xffffffffu, hi[j]);
-  }
-  cnt = __reduce_add_sync(0xffffffffu, cnt);
-  nan = __any_sync(0xffffffffu, nan);
-  __shared__ double sw[kBlock / 32][kMeasVals];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double v[kMeasVals];
-  v[0] = sum;
-  v[1] = mx == -INFINITY ? -1e300 : (double)mx;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    v[2 + 2 * j] = cnt ? (double)lo[j] : 1e300;
-    v[3 + 2 * j] = cnt ? (double)hi[j] : -1e300;
-  }
-  v[8] = (double)sz;
-  v[9] = (double)cnt;
-  v[10] = nan ? 1.0 : 0.0;
-  if (lane == 0)
-    for (int j = 0; j < kMeasVals; ++j) sw[wid][j] = v[j];
-  __syncthreads();
+  __shared__ Meas<T> sw[kBlock / 32];
+  static_assert(sizeof(Meas<T>) <= kMeasVals * sizeof(double), "room of a partial");
+  Meas<T>* const part = reinterpret_cast<Meas<T>*>(partials);
+  meas_block(v, sw);
   __shared__ bool s_last;
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kBlock / 32; ++w) meas_merge(v, sw[w]);
-    for (int j = 0; j < kMeasVals; ++j) partials[(size_t)blockIdx.x * kMeasVals + j] = v[j];
+    part[blockIdx.x] = v;
     __threadfence();
     s_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
@@ -1964,43 +1973,40 @@ __global__ void __launch_bounds__(kBlock) k_measure(int nx, int ny, int nz, cons
   __threadfence();
   // last block: every thread merges a strided subset of the block partials,
   // then warps and finally thread 0 merge (a fixed, deterministic order)
-  double r[kMeasVals] = {0.0, -1e300, 1e300, -1e300, 1e300, -1e300, 1e300, -1e300, 0.0, 0.0, 0.0};
-  const volatile double* pp = partials;
+  Meas<T> r;
   for (unsigned b = threadIdx.x; b < gridDim.x; b += kBlock) {
-    double q[kMeasVals];
-    for (int j = 0; j < kMeasVals; ++j) q[j] = pp[(size_t)b * kMeasVals + j];
+    Meas<T> q;
+    constexpr int W = sizeof(Meas<T>) / 8;
+    static_assert(sizeof(Meas<T>) % 8 == 0, "partials are read as 8-byte words");
+    unsigned long long w[W];
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(part + b);
+#pragma unroll
+    for (int j = 0; j < W; ++j) w[j] = __ldcg(src + j);
+    memcpy(&q, w, sizeof(q));
     meas_merge(r, q);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double q[kMeasVals];
-#pragma unroll
-    for (int j = 0; j < kMeasVals; ++j) q[j] = __shfl_down_sync(0xffffffffu, r[j], o);
-    meas_merge(r, q);
-  }
-  __syncthreads();
-  if (lane == 0)
-    for (int j = 0; j < kMeasVals; ++j) sw[wid][j] = r[j];
-  __syncthreads();
+  meas_block(r, sw);
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kBlock / 32; ++w) meas_merge(r, sw[w]);
-    const bool any = r[9] > 0.0;
-    const double Dx = any ? r[3] - r[2] + 1.0 : 0.0;
-    const double Dy = any ? r[5] - r[4] + 1.0 : 0.0;
-    const double Dz = any ? r[7] - r[6] + 1.0 : 0.0;
-    out[0] = r[0];
-    out[1] = r[1];
+    const bool any = r.cnt > 0;
+    const double Dx = any ? (double)(r.hi[0] - r.lo[0] + 1) : 0.0;
+    const double Dy = any ? (double)(r.hi[1] - r.lo[1] + 1) : 0.0;
+    const double Dz = any ? (double)(r.hi[2] - r.lo[2] + 1) : 0.0;
+    out[0] = r.sum;
+    out[1] = r.mx == -INFINITY ? -1e300 : (double)r.mx;
     out[2] = Dx;
     out[3] = Dy;
     out[4] = Dz;
     out[5] = Dy > 0.0 ? Dx / Dy : 0.0;
-    out[6] = any ? r[8] / r[9] : 0.0;
-    out[7] = r[9];
-    out[8] = r[10];
+    out[6] = any ? (double)r.sz / (double)r.cnt : 0.0;
+    out[7] = (double)r.cnt;
+    out[8] = r.nan ? 1.0 : 0.0;
     if (ext6) {
       // first and last index of the phi > 0.5 set along x, y, z (-1 when empty)
 #pragma unroll
-      for (int j = 0; j < 6; ++j) ext6[j] = any ? r[2 + j] : -1.0;
+      for (int j = 0; j < 3; ++j) {
+        ext6[2 * j] = any ? (double)r.lo[j] : -1.0;
+        ext6[2 * j + 1] = any ? (double)r.hi[j] : -1.0;
+      }
     }
     *counter = 0u;
   }
