@@ -971,11 +971,20 @@ __device__ __forceinline__ void update_node(const Consts<T>& k, const State<T, S
   const T omo = sub_rn(T(1), om);
   const T nsd = mul_rn(fma_(om, T(-0.5), T(1)), rc);
   const T u3x = mul_rn(u0, L::inv_cs2()), u3y = mul_rn(u1, L::inv_cs2()), u3z = mul_rn(u2, L::inv_cs2());
-  // e_q.u / cs2; the half form's first step fuses the x term of the diagonals that have one
+  // e_q.u / cs2.  The half form's first step fuses one product of a diagonal:
+  // the first component's (with tau_f == 1 of e_x != 0 only, else of all but
+  // the pair of q = 8, whose second it is).
   auto ecdot = [&](int q) {
-    if (HALF && FIRST && q > 6 && ex(q) != 0)
-      return fma_(ex(q) > 0 ? u0 : -u0, L::inv_cs2(),
-                  ey(q) != 0 ? (ey(q) > 0 ? u3y : -u3y) : (ez(q) > 0 ? u3z : -u3z));
+    if (HALF && FIRST && q > 6 && (!OMEGA1 || ex(q) != 0)) {
+      const T uc[3] = {u0, u1, u2}, u3[3] = {u3x, u3y, u3z};
+      const int e[3] = {ex(q), ey(q), ez(q)};
+      int i = e[0] != 0 ? 0 : 1, j = e[2] != 0 ? 2 : 1;  // the two components
+      if (!OMEGA1 && pair_first(4) == q) {
+        i = 1;
+        j = 0;
+      }
+      return fma_(e[i] > 0 ? uc[i] : -uc[i], L::inv_cs2(), e[j] > 0 ? u3[j] : -u3[j]);
+    }
     return edot(q, u3x, u3y, u3z);
   };
   {
