@@ -71,7 +71,10 @@ cudaError_t launch_batch_coop(const void*, const unsigned short*, int, int, int,
 template <typename T, typename Src>
 cudaError_t launch_init2d(const Consts<T>&, const State<T, T>&, const Src*, const Src*, cudaStream_t);
 template <typename T>
-cudaError_t launch_step2d(const Consts<T>&, const State<T, T>&, bool, bool, double, cudaStream_t, cudaEvent_t);
+cudaError_t launch_step2d(const Consts<T>&, const State<T, T>&, bool, bool, bool, bool, double, cudaStream_t,
+                          cudaEvent_t);
+template <typename T>
+cudaError_t launch_expand2d(const Consts<T>&, const State<T, T>&, double, cudaStream_t);
 template <typename T>
 cudaError_t launch_observe2d(const Consts<T>&, const State<T, T>&, bool, unsigned, int, T*, T*, T*, T*, T*, T*,
                              cudaStream_t);
@@ -158,7 +161,7 @@ struct LbmHandle {
   bool raw = true;        // current state is the reference state itself (after init)
   bool first = true;      // phi*u of the previous step does not exist yet
   PhiTile tile{};         // work split of the source form's phi pass (phis_tile of the grid alone)
-  bool sform = false;     // f[cur] holds S (three T per node) instead of the populations (lbm_phis.cuh)
+  bool sform = false;     // f[cur] holds S (a T per dimension and node) instead of the populations (lbm_phis.cuh)
   int c_last = 0;         // cbuf slot of the last step's correction
   int64_t steps = 0;
   bool last_raw_in = true;  // mode of the last step's input (for P read-out)
@@ -534,14 +537,17 @@ bool is2d(const LbmHandle* h) { return h->nz == 1; }
 int nq_of(int64_t nz) { return nz == 1 ? kQ2 : Q; }
 int ndim_of(int64_t nz) { return nz == 1 ? 2 : 3; }
 
+// The python-double Allen-Cahn source coefficient 1 - 1 / (2 tau_f).
+double ac_of(const LbmHandle* h) { return 1.0 - 0.5 / (h->prm.tau_h > 0 ? h->prm.tau_h : h->prm.tau_l); }
+bool wants_s(const LbmHandle* h);
+
 // The 2-D step of the handle's current state (no bookkeeping).
 template <typename T>
 int launch_next2d(LbmHandle* h, cudaStream_t st, cudaEvent_t mid) {
   State<T, T> s = make_state<T, T>(*h, h->cur, h->pc);
   s.c_prev = h->c_last;
   s.c_cur = h->c_last ^ 1;
-  const double tau_f = h->prm.tau_h > 0 ? h->prm.tau_h : h->prm.tau_l;
-  CUDA_TRY(launch_step2d<T>(consts_of<T>(*h), s, h->raw, h->first, 1.0 - 0.5 / tau_f, st, mid));
+  CUDA_TRY(launch_step2d<T>(consts_of<T>(*h), s, h->raw, h->first, h->sform, wants_s(h), ac_of(h), st, mid));
   return LBM_OK;
 }
 
@@ -592,7 +598,12 @@ int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
 // Whether the two-kernel step of a grid leaves f in source form: tau_f == 1, float
 // compute, linear layout.  (float64 keeps the populations: its step is bound by
 // the float64 pipe, and the source form evaluates f again on each tile's halo.)
-bool wants_s(const LbmHandle* h) { return h->prec != LBM_F64 && h->nz > 1 && !h->paired && omega1_of(h); }
+// 2-D: not in the gradient-of-mu modes, whose update re-reads f, and not below
+// 32 columns, where a block's window would be mostly its two ends.
+bool wants_s(const LbmHandle* h) {
+  if (h->prec == LBM_F64 || h->paired || !omega1_of(h)) return false;
+  return h->nz > 1 || (!h->mu && h->ny >= 32);
+}
 
 // Tiles of the source form's phi pass: the (y, z) split whose blocks (tile plus
 // halo within kPhisThreads nodes) waste the fewest threads, then the planes of
@@ -710,6 +721,12 @@ int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid)
 template <typename T, typename S>
 int expand_t(LbmHandle* h, cudaStream_t st) {
   State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
+  if constexpr (sizeof(T) == sizeof(S)) {
+    if (is2d(h)) {
+      CUDA_TRY((launch_expand2d<T>(consts_of<T>(*h), s, ac_of(h), st)));
+      return LBM_OK;
+    }
+  }
   CUDA_TRY((launch_expand<T, S>(consts_of<T>(*h), s, st)));
   return LBM_OK;
 }

@@ -17,6 +17,8 @@
 // population non-equilibrium stress) instead of the restructured moment and
 // collision algebra of the 3-D kernels, and are compiled without FMA
 // contraction: float32 parity on the 2-D cases needed both.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "lbm_common.cuh"
@@ -132,13 +134,10 @@ __device__ __forceinline__ T relax_scale(T target, T sum_f) {
   return s < T(0.5) ? T(0.5) : (s > T(2.0) ? T(2.0) : s);
 }
 
-// f of node n at the start of the step (pull, correction, relaxation).
-template <typename T, bool RAW>
-__device__ __forceinline__ void fetch_f9(T (&v)[Q9], const Consts<T>& k, const State<T, T>& s, int n,
-                                         const Nb2& nb, uint8_t c, T eps) {
-  const T corr = RAW ? T(1) : s.cbuf[s.c_prev];
-  fetch9<T, RAW>(v, s.fin, k.Np, n, nb, c, eps, corr);
-  if (!RAW && k.relax_on && (c & kTop)) {
+// The boundary-phi relaxation of a node's corrected populations.
+template <typename T>
+__device__ __forceinline__ void relax9(T (&v)[Q9], const Consts<T>& k, const State<T, T>& s, int n, uint8_t c, T corr) {
+  if (k.relax_on && (c & kTop)) {
     const T r = relax_target(k, s.phi_in, s.nsw, s.cubic, n, s.phi_in[n], corr);
     if (r >= T(0)) {
       const T sc = relax_scale(r, seqsum(v));
@@ -146,6 +145,15 @@ __device__ __forceinline__ void fetch_f9(T (&v)[Q9], const Consts<T>& k, const S
       for (int q = 0; q < Q9; ++q) v[q] = v[q] * sc;
     }
   }
+}
+
+// f of node n at the start of the step (pull, correction, relaxation).
+template <typename T, bool RAW>
+__device__ __forceinline__ void fetch_f9(T (&v)[Q9], const Consts<T>& k, const State<T, T>& s, int n,
+                                         const Nb2& nb, uint8_t c, T eps) {
+  const T corr = RAW ? T(1) : s.cbuf[s.c_prev];
+  fetch9<T, RAW>(v, s.fin, k.Np, n, nb, c, eps, corr);
+  if (!RAW) relax9(v, k, s, n, c, corr);
 }
 
 // Ghost value of a boundary node's solid neighbour in direction q
@@ -252,11 +260,13 @@ __device__ __forceinline__ void pair_div(T (&t)[Q9], T a0, T a1, CW cw, const Di
 // with the grid total (exact for float phi: unsigned 64-bit fixed point with
 // 31 fraction bits; NaN carried by a flag).
 constexpr unsigned long long kNaN = ~0ull;
+constexpr int kMaxBlock = 384;  // the largest block that sums phi (k2_phis)
+
 template <typename T>
 __device__ __forceinline__ bool grid_total(double part_d, unsigned long long part_u, bool nan, double* partials,
                                            unsigned* counter, double* total) {
-  __shared__ unsigned long long su[kBlock / 32];
-  __shared__ double sd[kBlock / 32];
+  __shared__ unsigned long long su[kMaxBlock / 32];
+  __shared__ double sd[kMaxBlock / 32];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
@@ -273,7 +283,7 @@ __device__ __forceinline__ bool grid_total(double part_d, unsigned long long par
   if (threadIdx.x == 0) {
     unsigned long long r = 0ull;
     double d = 0.0;
-    for (int i = 0; i < kBlock / 32; ++i) {
+    for (int i = 0; i < (int)(blockDim.x / 32); ++i) {
       r += su[i];
       d += sd[i];
     }
@@ -288,7 +298,7 @@ __device__ __forceinline__ bool grid_total(double part_d, unsigned long long par
   double td = 0.0;
   unsigned long long tu = 0ull;
   bool nn = false;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += kBlock) {
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
     if (sizeof(T) == 8) {
       td += ((const volatile double*)partials)[b];
     } else {
@@ -311,7 +321,7 @@ __device__ __forceinline__ bool grid_total(double part_d, unsigned long long par
   if (threadIdx.x != 0) return false;
   double d = 0.0;
   unsigned long long r = 0ull;
-  for (int i = 0; i < kBlock / 32; ++i) {
+  for (int i = 0; i < (int)(blockDim.x / 32); ++i) {
     r += su[i];
     d += sd[i];
   }
@@ -369,6 +379,25 @@ __global__ void __launch_bounds__(kBlock) k2_init(Consts<T> k, State<T, T> s, co
   }
 }
 
+// The grid sum of a phi pass and the mass-correction factor, status word.
+template <typename T>
+__device__ __forceinline__ void phi_total(const State<T, T>& s, double pd, unsigned long long pu, bool nan) {
+  double total;
+  if (grid_total<T>(pd, pu, nan, s.partials, s.counter, &total)) {
+    const T sum = (T)total;
+    T corr = T(1);
+    if (sum > T(1e-6)) {
+      const T safe = sum < T(1e-6) ? T(1e-6) : sum;
+      corr = (T(1) / safe) * (T)s.scal[0];
+    } else {
+      atomicOr(s.status, 2u);
+    }
+    if (!(total == total) || total - total != 0.0) atomicOr(s.status, 1u);
+    s.cbuf[s.c_cur] = corr;
+    s.scal[1] = total;
+  }
+}
+
 // phi of every node of this step, its grid sum and the mass-correction factor
 // (lbm/fe_ac_solver.py:385-389, 582-589).
 // Persistent: a grid of about one wave strides over the nodes, so that few
@@ -393,20 +422,126 @@ __global__ void __launch_bounds__(kBlock) k2_phi(Consts<T> k, State<T, T> s) {
     s.phi_out[n] = phi;
     add_phi(phi, pd, pu, nan);
   }
-  double total;
-  if (grid_total<T>(pd, pu, nan, s.partials, s.counter, &total)) {
-    const T sum = (T)total;
-    T corr = T(1);
-    if (sum > T(1e-6)) {
-      const T safe = sum < T(1e-6) ? T(1e-6) : sum;
-      corr = (T(1) / safe) * (T)s.scal[0];
-    } else {
-      atomicOr(s.status, 2u);
-    }
-    if (!(total == total) || total - total != 0.0) atomicOr(s.status, 1u);
-    s.cbuf[s.c_cur] = corr;
-    s.scal[1] = total;
+  phi_total(s, pd, pu, nan);
+}
+
+// Source form (float, tau_f == 1, no gradient-of-mu mode): the update kernel
+// stores the interface source S (two values, at the start of the f buffer) from
+// which, with phi and u, the nine populations follow; 28 bytes per node less
+// written, and 16 less read by the phi pass.
+template <typename T>
+__device__ __forceinline__ void f_of_source(T phi, T u0, T u1, T S0, T S1, T acT, T (&f)[Q9]) {
+  const T usq = u0 * u0 + u1 * u1;
+  const T b = by_two_cs2<T>()(usq);
+  T ecs[Q9], src[Q9];
+  pair_div(ecs, u0, u1, [](int) { return T(1); }, by_cs2<T>());
+  pair_div(src, S0, S1, [&](int q) { return acT * w<T>(q); }, by_cs2<T>());
+#pragma unroll
+  for (int q = 0; q < Q9; ++q) {
+    const T ec = ecs[q], sq = ec * ec / T(2);
+    const T feq = phi * (w<T>(q) * (((T(1) + ec) + sq) - b));
+    f[q] = feq + src[q];
   }
+}
+
+// Populations of a state in source form (s.fin: S) into s.fout.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k2_expand(Consts<T> k, State<T, T> s, double ac) {
+  const int n = blockIdx.x * kBlock + threadIdx.x;
+  if (n >= k.N) return;
+  T f[Q9];
+  f_of_source<T>(s.phi_in[n], s.u[n], s.u[k.Np + n], s.fin[n], s.fin[k.Np + n], (T)ac, f);
+#pragma unroll
+  for (int q = 0; q < Q9; ++q) s.fout[q * k.Np + n] = f[q];
+}
+
+// Row among the six populations with e_y != 0 of a column.
+__host__ __device__ constexpr int row6(int q) {
+  int r = 0;
+  for (int p = 1; p < q; ++p) r += ey(p) != 0 ? 1 : 0;
+  return r;
+}
+
+// The phi pass of a state in source form.  A block walks cx rows of x over a
+// window of w columns, one thread per column and one more at either end
+// (periodic): it evaluates its node's populations, passes the six that leave the
+// column through shared memory (four slots of rows, so one barrier per row) and
+// completes the row before from the three rows around it; the next row's loads
+// are in flight meanwhile.  Same values and order of sums as k2_phi over stored
+// populations.  2048x1024, float: 29 us against k2_phi's 27, the update kernel 51
+// against 62, the step 81.2 -> 74.0 us.  (Blocks of at most 192, 256, 352 or 512
+// threads: 75.0, 75.9, 75.0, 79.7 us.)  What bounds it: latency, 33 warps per SM
+// at one barrier per row.
+template <typename T>
+__global__ void __launch_bounds__(kMaxBlock, 3) k2_phis(Consts<T> k, State<T, T> s, double ac, int nwin, int w_, int cx) {
+  __shared__ T sm[4][6][kMaxBlock];
+  pdl_trigger();
+  pdl_wait();  // S and u of the previous update kernel
+  const int chunk = blockIdx.x / nwin, win = blockIdx.x - chunk * nwin;
+  const int y0 = win * w_, ew = min(w_, k.ny - y0), x0 = chunk * cx, x1 = min(x0 + cx, k.nx);
+  const int t = threadIdx.x, Np = k.Np;
+  const bool inner = t >= 1 && t <= ew;
+  int y = t < ew + 2 ? y0 - 1 + t : 0;
+  y = y < 0 ? y + k.ny : (y >= k.ny ? y - k.ny : y);
+  const T corr = s.cbuf[s.c_prev], acT = (T)ac;
+  const T* __restrict__ src = s.fin;
+  struct Row {
+    T phi, u0, u1, S0, S1;
+    uint8_t c;
+  };
+  auto load = [&](int x) {
+    const int n = (x < 0 ? x + k.nx : (x >= k.nx ? x - k.nx : x)) * k.ny + y;
+    return Row{s.phi_in[n], s.u[n], s.u[Np + n], src[n], src[Np + n], s.cls[n]};
+  };
+  constexpr int qxp = 1;  // the velocity (+1, 0)
+  static_assert(ex(qxp) == 1 && ey(qxp) == 0, "D2Q9 order");
+  double pd = 0.0;
+  unsigned long long pu = 0ull;
+  bool nan = false;
+  T f0_last = T(0), fxp_last = T(0), fxp_before = T(0);  // of the last row, and the one before it
+  uint8_t c_last = 0;
+  Row nxt = load(x0 - 1);
+  for (int x = x0 - 1, j = 0; x <= x1; ++x, j = (j + 1) & 3) {
+    const Row v = nxt;
+    if (x < x1) nxt = load(x + 1);
+    T f[Q9];
+    f_of_source<T>(v.phi, v.u0, v.u1, v.S0, v.S1, acT, f);
+#pragma unroll
+    for (int q = 1; q < Q9; ++q)
+      if (ey(q) != 0) sm[j][row6(q)][t] = f[q];
+    __syncthreads();
+    if (inner && x > x0) {
+      const int n = (x - 1) * k.ny + y;
+      T phi = T(0);
+      if (!(c_last & kSolid)) {
+        T v9[Q9];
+#pragma unroll
+        for (int q = 0; q < Q9; ++q) {
+          if (q == 0) v9[q] = f0_last;
+          else if (ey(q) == 0) v9[q] = ex(q) > 0 ? fxp_before : f[q];
+          else v9[q] = sm[(j + (ex(q) > 0 ? 2 : (ex(q) == 0 ? 3 : 0))) & 3][row6(q)][t - ey(q)];
+        }
+        if (c_last & kPartial) {
+          const T eps = s.eps[n], one_m = T(1) - eps;
+          T o[Q9];
+          f_of_source<T>(s.phi_in[n], s.u[n], s.u[Np + n], src[n], src[Np + n], acT, o);
+#pragma unroll
+          for (int q = 0; q < Q9; ++q) v9[q] = one_m * v9[q] + eps * o[opp(q)];
+        }
+#pragma unroll
+        for (int q = 0; q < Q9; ++q) v9[q] = v9[q] * corr;
+        relax9(v9, k, s, n, c_last, corr);
+        phi = clamp01(seqsum(v9));
+      }
+      s.phi_out[n] = phi;
+      add_phi(phi, pd, pu, nan);
+    }
+    f0_last = f[0];
+    fxp_before = fxp_last;
+    fxp_last = f[qxp];
+    c_last = v.c;
+  }
+  phi_total(s, pd, pu, nan);
 }
 
 // mu of every node from this step's phi (the update kernel's arithmetic).
@@ -454,8 +589,8 @@ __global__ void __launch_bounds__(kBlock) k2_gradmu(Consts<T> k, State<T, T> s) 
 // OMEGA1: tau_f == 1 (the reference's default tau_h), where the phase-field
 // collision f - (f - f_eq) + src is taken as f_eq + src and f is not read
 // again (the two differ by at most an ulp of f where f and f_eq are more
-// than a factor of two apart).
-template <typename T, bool RAW, bool FIRST, bool GMU, bool OMEGA1 = false>
+// than a factor of two apart).  SOUT: S is stored instead of f (f_of_source).
+template <typename T, bool RAW, bool FIRST, bool GMU, bool OMEGA1 = false, bool SOUT = false>
 __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, double ac) {
   pdl_trigger();
   pdl_wait();  // phi of k2_phi (grad mu of k2_gradmu)
@@ -620,9 +755,13 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
     const T ec = ecs[q];
     const T sq = ec * ec / T(2);
     const T feq = phi * (w<T>(q) * (((T(1) + ec) + sq) - b));
-    s.fout[q * Np + n] = OMEGA1 ? feq + src[q] : (f[q] - k.omega_f * (f[q] - feq)) + src[q];
+    if (!SOUT) s.fout[q * Np + n] = OMEGA1 ? feq + src[q] : (f[q] - k.omega_f * (f[q] - feq)) + src[q];
     const T geq = P * w<T>(q) + w<T>(q) * ((ec + sq) - b);
     s.gout[q * Np + n] = (g[q] - om * (g[q] - geq)) + G[q];
+  }
+  if (SOUT) {
+    s.fout[n] = S0;
+    s.fout[Np + n] = S1;
   }
   s.u[n] = u0;
   s.u[Np + n] = u1;
@@ -801,13 +940,45 @@ cudaError_t launch_init2d(const Consts<T>& k, const State<T, T>& s, const Src* p
   return cudaGetLastError();
 }
 
-// One step: k2_phi, [k2_mu, k2_gradmu], k2_update.  `mid` (may be null) is
-// recorded between the phi kernel and the rest.
+// Launch of k2_phis: the fewest windows of columns that a block's threads cover,
+// then the rows per block that keep the device busy for the shortest time (two
+// more rows are evaluated at a block's ends).
 template <typename T>
-cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool first, double ac, cudaStream_t st,
-                          cudaEvent_t mid) {
+cudaError_t launch_phis2d(const Consts<T>& k, const State<T, T>& s, double ac, cudaStream_t st) {
+  if constexpr (sizeof(T) == 8) {
+    return cudaErrorNotSupported;
+  } else {
+    const int nwin = (k.ny + d2::kMaxBlock - 3) / (d2::kMaxBlock - 2), w = (k.ny + nwin - 1) / nwin;
+    const int threads = (w + 2 + 31) / 32 * 32;
+    const int slots = d2::phi_blocks_of(0x7fffff00) / 8 * std::min(16, 3 * d2::kMaxBlock / threads);
+    int cx = 2;
+    long long best = -1;
+    for (int c = 2; c <= 64; ++c) {
+      const long long cost = ((long long)nwin * ((k.nx + c - 1) / c) + slots - 1) / slots * (c + 2);
+      if (best < 0 || cost < best) {
+        best = cost;
+        cx = c;
+      }
+    }
+    return launch_pdl_bs(d2::k2_phis<T>, nwin * ((k.nx + cx - 1) / cx), threads, st, k, s, ac, nwin, w, cx);
+  }
+}
+template <typename T>
+cudaError_t launch_expand2d(const Consts<T>& k, const State<T, T>& s, double ac, cudaStream_t st) {
+  d2::k2_expand<T><<<d2::blocks_of(k.N), kBlock, 0, st>>>(k, s, ac);
+  return cudaGetLastError();
+}
+
+// One step: k2_phi, [k2_mu, k2_gradmu], k2_update.  `mid` (may be null) is
+// recorded between the phi kernel and the rest.  sin: s.fin is in source form;
+// sout: s.fout is to be (not raw, not first).
+template <typename T>
+cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool first, bool sin, bool sout, double ac,
+                          cudaStream_t st, cudaEvent_t mid) {
   const int nb = d2::blocks_of(k.N), np = d2::phi_blocks_of(k.N);
-  cudaError_t e = raw ? launch_pdl(d2::k2_phi<T, true>, np, st, k, s) : launch_pdl(d2::k2_phi<T, false>, np, st, k, s);
+  cudaError_t e = sin ? launch_phis2d<T>(k, s, ac, st)
+                  : raw ? launch_pdl(d2::k2_phi<T, true>, np, st, k, s)
+                        : launch_pdl(d2::k2_phi<T, false>, np, st, k, s);
   if (e != cudaSuccess) return e;
   if (mid) {
     e = cudaEventRecord(mid, st);
@@ -828,7 +999,8 @@ cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bo
   } else if (first) {
     LBM_UPD2(false, true)
   } else if (!gmu && k.omega_f == T(1)) {
-    return launch_pdl(d2::k2_update<T, false, false, false, true>, nb, st, k, s, ac);
+    return sout ? launch_pdl(d2::k2_update<T, false, false, false, true, true>, nb, st, k, s, ac)
+                : launch_pdl(d2::k2_update<T, false, false, false, true>, nb, st, k, s, ac);
   } else {
     LBM_UPD2(false, false)
   }
@@ -866,8 +1038,9 @@ cudaError_t launch_inject2d(const Consts<T>& k, const State<T, T>& s, bool raw, 
                                                cudaStream_t);                                                       \
   template cudaError_t launch_init2d<T, double>(const Consts<T>&, const State<T, T>&, const double*, const double*, \
                                                 cudaStream_t);                                                      \
-  template cudaError_t launch_step2d<T>(const Consts<T>&, const State<T, T>&, bool, bool, double, cudaStream_t,     \
-                                        cudaEvent_t);                                                               \
+  template cudaError_t launch_step2d<T>(const Consts<T>&, const State<T, T>&, bool, bool, bool, bool, double,       \
+                                        cudaStream_t, cudaEvent_t);                                                 \
+  template cudaError_t launch_expand2d<T>(const Consts<T>&, const State<T, T>&, double, cudaStream_t);              \
   template cudaError_t launch_observe2d<T>(const Consts<T>&, const State<T, T>&, bool, unsigned, int, T*, T*, T*,   \
                                            T*, T*, T*, cudaStream_t);                                               \
   template cudaError_t launch_populations2d<T>(const Consts<T>&, const State<T, T>&, bool, T*, T*, cudaStream_t);  \
