@@ -22,7 +22,7 @@ One "step" is one lattice time step of the whole grid.  Reported:
   roofline   the dominant kernel (k_update): algorithmic bytes per launch /
              its CUDA-event duration (from a separate pass with events between
              the kernels), against the measured HBM copy peak; step_roofline:
-             the whole step's 336 B/node over the timed region.
+             the whole step's bytes (224 B/node) over the timed region.
   cpu_baseline  the numpy oracle (oracle/ac_oracle.py) on a bounded sample of
              the same workload, one host core; the reference's own PyTorch
              CPU figure, measured where the reference is installed, beside it.
@@ -47,27 +47,29 @@ sys.path.insert(0, ROOT)
 
 import numpy as np  # noqa: E402
 
-# Algorithmic bytes per node and step, float32 state: f and g (2 x 19
-# populations), u (3) and the previous phi (1), each read once and written
-# once: 2 x 4 x (38 + 3 + 1) = 336 B.  Half-precision population storage:
-# 2 x 2 x 38 + 2 x 4 x 4 = 184 B.
-B_ALG_STEP = {"fp32": 336, "fp16": 184}
+# Algorithmic bytes per node and step, float32 state.  The two-kernel step
+# keeps the source vector S in place of f (tau_f == 1): g (19), u (3), S (3)
+# and the previous phi (1), each read once and written once:
+# 2 x 4 x (19 + 3 + 3 + 1) = 208 B, and 4 x 4 more because the phi kernel and
+# the update kernel both read u and the previous phi.  Half-precision population
+# storage: 2 x 2 x 19 + 2 x 4 x 7 + 16 = 148 B.  The fused kernel keeps f and g:
+# 2 x 4 x (38 + 3 + 1) = 336 B, or 184 B.
+B_ALG_STEP = {"fp32": 224, "fp16": 148}
+B_ALG_STEP_FUSED = {"fp32": 336, "fp16": 184}
 # Per kernel (each adds the node-class byte it reads):
-#   k_phi     f read (76 | 38), phi written (4), in the half form also the
-#             previous phi (4, the deviation reference)
-#   k_update  g (76 | 38), u (12) and previous phi (4) read; f, g (76 + 76 |
-#             38 + 38) and u (12) written; the phi stencil comes from L2
+#   k_phi     previous phi (4), u (12), S (12) read, phi written (4)
+#   k_update  g (76 | 38), u (12) and previous phi (4) read; g (76 | 38), u (12)
+#             and S (12) written; the phi stencil comes from L2
 #   k_step    the fused kernel: the whole step
-B_ALG_KERNEL = {"fp32": {"k_phi": 81, "k_update": 257, "k_step": 337},
-                "fp16": {"k_phi": 47, "k_update": 143, "k_step": 185}}
-# 2-D (D2Q9) grids, float32: f and g (2 x 9), u (2), previous phi (1), read
-# and written once: 2 x 4 x 21 = 168 B per node and step.  k2_phi reads f
-# (36) and the class byte and writes phi (4); k2_update reads g (36), u (8),
-# the previous phi (4) and the class byte and writes f, g (72) and u (8).
-# (k2_update also reads f again for the collision: traffic beyond these
-# algorithmic bytes.)
-B_ALG_STEP_2D = 168
-B_ALG_KERNEL_2D = {"k2_phi": 41, "k2_update": 129}
+B_ALG_KERNEL = {"fp32": {"k_phi": 33, "k_update": 193, "k_step": 337},
+                "fp16": {"k_phi": 33, "k_update": 117, "k_step": 185}}
+# 2-D (D2Q9) grids, float32: S (2) in place of f, g (9), u (2), previous phi (1),
+# read and written once: 2 x 4 x 14 = 112 B, and 4 x 3 more for u and the
+# previous phi read by both kernels.  k2_phis reads the previous phi (4), u (8),
+# S (8) and the class byte and writes phi (4); k2_update reads g (36), u (8), the
+# previous phi (4) and the class byte and writes g (36), u (8) and S (8).
+B_ALG_STEP_2D = 124
+B_ALG_KERNEL_2D = {"k2_phi": 25, "k2_update": 101}
 
 WORKLOADS = {
     "ridge150": dict(grid=(150, 150, 107), substrate=("ridge", 1.0, 22.5), center=(75, 75, 80),
@@ -395,7 +397,7 @@ def run_ours(args, rank, world, device):
     if rank == 0:
         peak, peak_kind = peaks()
         f16 = args.precision == "fp16"
-        b_step = B_ALG_STEP_2D if two_d else B_ALG_STEP[args.precision]
+        b_step = B_ALG_STEP_2D if two_d else (B_ALG_STEP if two_kernel else B_ALG_STEP_FUSED)[args.precision]
         # the dominant kernel of the step: k_update (two-kernel step) or k_step (fused)
         kname = ("k2_update" if two_d else "k_update") if two_kernel else "k_step"
         b_ker = B_ALG_KERNEL_2D[kname] if two_d else B_ALG_KERNEL[args.precision][kname]
