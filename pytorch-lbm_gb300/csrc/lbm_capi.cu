@@ -166,7 +166,7 @@ struct LbmHandle {
   int64_t steps = 0;
   bool last_raw_in = true;  // mode of the last step's input (for P read-out)
   bool obs_init = true;     // fields read as after init_fields (no step since init or an injection)
-  // the two-kernel step runs the batched kernels on a one-case table: device
+  // the paired layout runs its table kernels on a one-case table: device
   // descriptors for the two step parities, valid while desc_ok
   void* desc = nullptr;
   bool desc_ok = false;
@@ -651,7 +651,7 @@ int upd_blocks_of(const LbmHandle* h, int upd_block) {
   return (int)((units_of(h) + bs - 1) / bs);
 }
 
-// The handle's one-case descriptor table for the batched kernels: [0] the
+// The handle's one-case descriptor table for the paired kernels: [0] the
 // state as it is now, [1] after one more step.  The descriptor holds device
 // pointers that alternate with the step parity, constants and grid extents.
 template <typename T, typename S>
@@ -676,8 +676,8 @@ int fill_desc(LbmHandle* h, cudaStream_t st) {
 
 // Launches the step that would run next (no bookkeeping): the first step
 // after init and the fused kernel through launch_step; every other
-// two-kernel step through the batched kernels on the handle's one-case table,
-// so a grid gives the same results alone and in a batch.  `mid` (may be null)
+// two-kernel step through the kernels of a grid alone (linear layout), or the
+// paired kernels on the handle's one-case table.  `mid` (may be null)
 // is recorded between the two kernels (before the fused kernel).
 template <typename T, typename S>
 int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid) {

@@ -8,10 +8,12 @@
 //   k2_phi     phi of every node from the pulled f (bounce-back, volume
 //              penalisation, last step's mass correction and boundary-phi
 //              relaxation) and the grid sum of phi -> this step's correction;
+//              (k2_phis: the same from a state in source form);
 //   k2_mu, k2_gradmu  (Cahn-Hilliard and mu-drive modes only) mu of every
 //              node, then its isotropic gradient;
 //   k2_update  stencils, wetting, forces, velocity, both BGK collisions.
-// Besides: k2_init (init_fields), k2_inject (inject_droplet), k2_observe and
+// Besides: k2_init (init_fields), k2_expand (populations of a state in source
+// form), k2_inject (inject_droplet), k2_observe and
 // k2_populations (attribute read-out).
 // These kernels keep the reference's operation order (divisions, per-
 // population non-equilibrium stress) instead of the restructured moment and
