@@ -63,9 +63,26 @@ __device__ __forceinline__ T clamp01(T v) {
   return v < T(0) ? T(0) : (v > T(1) ? T(1) : v);
 }
 
-template <typename T>
-__device__ __forceinline__ T ldg(const T* p) {
-  return __ldg(p);
+// Loads of the state arrays (f or S, g, u, phi, mu), which the kernel before
+// writes while blocks of this one may already be resident (pdl_wait), which a
+// cooperative step writes before its grid barrier, and of which the update kernel
+// writes u in place.  So they are coherent loads (not ld.global.nc, whose data
+// has to stay unwritten while the kernel runs), and volatile asm like the
+// stores and pdl_wait, so that the compiler moves none of them across those.
+__device__ __forceinline__ float ld_state(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_state(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ __half ld_state(const __half* p) {
+  unsigned short v;
+  asm volatile("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p));
+  return __ushort_as_half(v);
 }
 
 // L2 cache policies.  KEEP (evict_last) marks the populations that phase A of
@@ -84,12 +101,12 @@ struct Pol {
 };
 __device__ __forceinline__ float ld_pol(const float* p, unsigned long long pol) {
   float v;
-  asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ double ld_pol(const double* p, unsigned long long pol) {
   double v;
-  asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ void st_pol(float* p, float v, unsigned long long pol) {
@@ -100,7 +117,7 @@ __device__ __forceinline__ void st_pol(double* p, double v, unsigned long long p
 }
 __device__ __forceinline__ __half ld_pol(const __half* p, unsigned long long pol) {
   unsigned short v;
-  asm("ld.global.nc.L2::cache_hint.b16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.b16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
   return __ushort_as_half(v);
 }
 __device__ __forceinline__ void st_pol(__half* p, __half v, unsigned long long pol) {
@@ -245,14 +262,12 @@ __device__ __forceinline__ bool last_block_total(double part, double* partials, 
 // ---------------------------------------------------------------------------
 // Population reconstruction (pull form -> reference state at step start)
 // ---------------------------------------------------------------------------
-// Loads of the step kernel carry an L2 policy; the read-out kernels (no
-// policy) use plain read-only loads.
+// Loads of the step kernel carry an L2 policy; those of the read-out kernels do not.
 template <bool USE_POL, typename S>
 __device__ __forceinline__ S ld_sel(const S* p, unsigned long long pol) {
   if constexpr (USE_POL) return ld_pol(p, pol);
-  else return ldg(p);
+  else return ld_state(p);
 }
-__device__ __forceinline__ __half ldg(const __half* p) { return __ldg(p); }
 
 // Populations of node n as the reference holds them at the start of the step
 // (before the mass correction, which WITH_C applies).  IS_F selects the
@@ -270,13 +285,13 @@ __device__ __forceinline__ void fetch_pop(T (&v)[Q], const Consts<T>& k, const S
   // element offsets q Np + m stay below 2^31 (checked when the grid is created)
   const unsigned Nu = (unsigned)k.Np, nu = I(n);
   (void)N;
-  const T ref_self = (IO::kDev && IS_F) ? ldg(phi_in + nu) : T(0);
+  const T ref_self = (IO::kDev && IS_F) ? ld_state(phi_in + nu) : T(0);
   auto ld = [&](int q, unsigned idx, T ref) -> T {
     const S raw = ld_sel<USE_POL>(F + idx, pol);
     return IS_F ? IO::ld_f(raw, q, ref, k) : IO::ld_g(raw, q, k);
   };
   auto ref_nb = [&](int q) -> T {
-    return (IO::kDev && IS_F) ? ldg(phi_in + I(nb.at(n, -ex(q), -ey(q), -ez(q)))) : T(0);
+    return (IO::kDev && IS_F) ? ld_state(phi_in + I(nb.at(n, -ex(q), -ey(q), -ez(q)))) : T(0);
   };
   if (RAW) {
 #pragma unroll
@@ -352,7 +367,7 @@ __device__ __forceinline__ void fetch_f(T (&v)[Q], const Consts<T>& k, const Sta
   fetch_pop<T, S, RAW, !RAW, true, USE_POL, MAP>(v, k, s.fin, s.phi_in, n, N, nb, c, eps, corr, pol);
   if (!RAW && k.relax_on && (c & kTop)) {
     const T r = relax_target<T, MAP>(k, s.phi_in, s.nsw, s.cubic, n,
-                                     ldg(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)), corr);
+                                     ld_state(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)), corr);
     if (r >= T(0)) {
       const T sc = relax_scale(r, seqsum(v));
 #pragma unroll
@@ -400,7 +415,7 @@ __device__ __forceinline__ T phi_value(const Consts<T>& k, const State<T, S>& s,
   if constexpr (RAW && PopIO<T, S>::kDev) {
     // the first step of the half form: deviation plus reference, weighted into the sum by fused multiply-adds
     const unsigned e = MAP ? sidx(k, n) : (unsigned)n;
-    const T ref = ldg(s.phi_in + e);
+    const T ref = ld_state(s.phi_in + e);
     auto h = [&](int q) { return add_rn(__half2float(ld_pol(s.fin + (q * (unsigned)k.Np + e), pol)), ref); };
     T sum = fma_(Lat<T>::w(0), h(0), mul_rn(Lat<T>::w(1), h(1)));
 #pragma unroll
@@ -410,7 +425,7 @@ __device__ __forceinline__ T phi_value(const Consts<T>& k, const State<T, S>& s,
   fetch_pop<T, S, RAW, false, true, true, MAP>(v, k, s.fin, s.phi_in, n, (size_t)k.N, nb, c, eps, T(1), pol);
   if (RAW) return clamp01(seqsum(v));
   return phi_of<T, S, MAP>(k, s, n, c, v, s.cbuf[s.c_prev],
-                           (k.relax_on && (c & kTop)) ? ldg(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)) : T(0));
+                           (k.relax_on && (c & kTop)) ? ld_state(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)) : T(0));
 }
 
 // Lattice constants as the paired step kernels read them: compile-time immediates
@@ -1156,7 +1171,7 @@ struct TileNode : NodeAt<T, S, RAW, true> {
       if (!RAW && (c & kSolid)) {
         // bounce-back: the node's own opposite values, not the staged pulled ones
 #pragma unroll
-        for (int q = 0; q < Q; ++q) g[q] = ldg(gin + (opp(q) * this->Np + this->e));
+        for (int q = 0; q < Q; ++q) g[q] = ld_state(gin + (opp(q) * this->Np + this->e));
       } else {
 #pragma unroll
         for (int q = 0; q < Q; ++q) g[q] = st[q * kBlock];
@@ -1165,7 +1180,7 @@ struct TileNode : NodeAt<T, S, RAW, true> {
         const T one_m = sub_rn(T(1), eps);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
-          g[q] = fma_(one_m, g[q], mul_rn(eps, ldg(gin + (opp(q) * this->Np + this->e))));
+          g[q] = fma_(one_m, g[q], mul_rn(eps, ld_state(gin + (opp(q) * this->Np + this->e))));
       }
     } else {
       Base::load_g(g, c, eps);

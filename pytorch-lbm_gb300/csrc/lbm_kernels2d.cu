@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kMaxBlock, 3) k2_phis(Consts<T> k, State<T, T>
   int y = t < ew + 2 ? y0 - 1 + t : 0;
   y = y < 0 ? y + k.ny : (y >= k.ny ? y - k.ny : y);
   const T corr = s.cbuf[s.c_prev], acT = (T)ac;
-  const T* __restrict__ src = s.fin;
+  const T* src = s.fin;
   struct Row {
     T phi, u0, u1, S0, S1;
     uint8_t c;

@@ -82,20 +82,20 @@ __device__ __forceinline__ T& lane(V2<T>& v, int l) { return l ? v.y : v.x; }
 template <typename T>
 __device__ __forceinline__ T lane(const V2<T>& v, int l) { return l ? v.y : v.x; }
 
-// Loads and stores of one pair word with an L2 policy.
+// Loads (coherent, see ld_state) and stores of one pair word with an L2 policy.
 __device__ __forceinline__ float2 ld2_pol(const float* p, unsigned long long pol) {
   float2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ double2 ld2_pol(const double* p, unsigned long long pol) {
   double2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ __half2 ld2_pol(const __half* p, unsigned long long pol) {
   unsigned r;
-  asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
   __half2 h;
   memcpy(&h, &r, 4);
   return h;
@@ -256,7 +256,7 @@ __device__ __forceinline__ void fetch_f_pair(V2<T> (&v)[Q], const Consts<T>& k, 
     for (int l = 0; l < 2; ++l) {
       if (!((l ? c1 : c0) & kTop)) continue;
       const int n = p + l * k.nh;
-      const T r = relax_target<T, true>(k, s.phi_in, s.nsw, s.cubic, n, ldg(s.phi_in + 2u * (unsigned)p + l), corr);
+      const T r = relax_target<T, true>(k, s.phi_in, s.nsw, s.cubic, n, ld_state(s.phi_in + 2u * (unsigned)p + l), corr);
       if (r >= T(0)) {
         const T sc = relax_scale(r, lane<T>(sum, l));
 #pragma unroll
@@ -303,7 +303,7 @@ __device__ __forceinline__ void phi_pair(const Consts<T>& k, const State<T, S>& 
         const uint8_t c = l ? c1 : c0;
         if ((c & (kTop | kSolid | kPartial)) != kTop) continue;
         const int n = p + l * k.nh;
-        const T r = relax_target<T, true>(k, s.phi_in, s.nsw, s.cubic, n, ldg(s.phi_in + e + l), corr);
+        const T r = relax_target<T, true>(k, s.phi_in, s.nsw, s.cubic, n, ld_state(s.phi_in + e + l), corr);
         if (r >= T(0)) {
           const T sc = relax_scale(r, lane<T>(sum, l));
           // fetch_f scales each value, then sums: two roundings per term
@@ -384,7 +384,7 @@ __device__ __forceinline__ void update_pair(const Consts<T>& k, const State<T, S
   const PNbr nb = make_pnbr(k, p);
   const uint8_t c0 = s.cls[p], c1 = s.cls[p + nh];
   const uint8_t cor = c0 | c1;
-  const T* __restrict__ pc = s.phi_out;  // phi of this step (phi kernel)
+  const T* pc = s.phi_out;  // phi of this step (phi kernel)
   const V phi = ld2_pol(pc + e, pol.keep);
 
   // 2. the stencil: gradient and laplacian with the ghost-node wetting values

@@ -117,7 +117,7 @@ __device__ __forceinline__ void phis_block(const Consts<float>& k, const State<f
   y = act ? (y < 0 ? y + k.ny : (y >= k.ny ? y - k.ny : y)) : 0;
   z = z < 0 ? z + k.nz : (z >= k.nz ? z - k.nz : z);
   const unsigned m = (unsigned)(y * k.nz + z), P = (unsigned)(k.ny * k.nz), Np = (unsigned)k.Np;
-  const float* __restrict__ src = reinterpret_cast<const float*>(s.fin);
+  const float* src = reinterpret_cast<const float*>(s.fin);
   const float corr = s.cbuf[s.c_prev];
 
   struct Nodes {  // of two planes
@@ -174,7 +174,7 @@ __device__ __forceinline__ void phis_block(const Consts<float>& k, const State<f
             const Nbr nb = make_nbr_xyz(x, y, z, k.nx, k.ny, k.nz);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
-              o[q] = stored_f<S>(k, q, o[q], ldg(s.phi_in + nb.at((int)n, ex(q), ey(q), ez(q))));
+              o[q] = stored_f<S>(k, q, o[q], ld_state(s.phi_in + nb.at((int)n, ex(q), ey(q), ez(q))));
           }
 #pragma unroll
           for (int q = 0; q < Q; ++q) w[q] = fma_(one_m, w[q], mul_rn(eps, o[opp(q)]));
