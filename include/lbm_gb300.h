@@ -236,7 +236,9 @@ int lbm_get_fields(LbmHandle* h, uint32_t mask, void* phi, void* rho, void* u,
 
 /* Current populations f, g (19N each, 9N on a 2-D grid; caller device buffers of the handle's
  * compute type) as the reference holds them between steps (AllenCahnSolver.f/.g,
- * lbm/fe_ac_solver.py:97-98). */
+ * lbm/fe_ac_solver.py:97-98).  Writes nothing of the state: on another stream than
+ * the steps', ordered after the last of them, it may overlap the next step (where f has
+ * to be evaluated from u, the next step's stream waits for it by itself). */
 int lbm_get_populations(LbmHandle* h, void* f, void* g, void* stream);
 
 /* Inject a droplet mid-run: centre (3 doubles, lattice units), radius,

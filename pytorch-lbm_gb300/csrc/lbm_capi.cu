@@ -32,7 +32,7 @@ template <typename T, typename S>
 cudaError_t launch_observe(const Consts<T>&, const State<T, S>&, bool, unsigned, int, T*, T*, T*, T*, T*, T*,
                            cudaStream_t);
 template <typename T, typename S>
-cudaError_t launch_populations(const Consts<T>&, const State<T, S>&, bool, T*, T*, cudaStream_t);
+cudaError_t launch_populations(const Consts<T>&, const State<T, S>&, bool, bool, T*, T*, cudaStream_t);
 template <typename T, typename S>
 cudaError_t launch_inject(const Consts<T>&, const State<T, S>&, bool, const InjectParams&, const T*, unsigned*,
                           cudaStream_t);
@@ -79,7 +79,7 @@ template <typename T>
 cudaError_t launch_observe2d(const Consts<T>&, const State<T, T>&, bool, unsigned, int, T*, T*, T*, T*, T*, T*,
                              cudaStream_t);
 template <typename T>
-cudaError_t launch_populations2d(const Consts<T>&, const State<T, T>&, bool, T*, T*, cudaStream_t);
+cudaError_t launch_populations2d(const Consts<T>&, const State<T, T>&, bool, bool, double, T*, T*, cudaStream_t);
 template <typename T>
 cudaError_t launch_inject2d(const Consts<T>&, const State<T, T>&, bool, const InjectParams&, const T*, unsigned*,
                             cudaStream_t);
@@ -164,6 +164,9 @@ struct LbmHandle {
   bool sform = false;     // f[cur] holds S (a T per dimension and node) instead of the populations (lbm_phis.cuh)
   int c_last = 0;         // cbuf slot of the last step's correction
   int64_t steps = 0;
+  // read-outs of f in source form read u: their end, which what overwrites u waits for (after_reads)
+  cudaEvent_t read = nullptr;
+  bool read_open = false;
   bool last_raw_in = true;  // mode of the last step's input (for P read-out)
   bool obs_init = true;     // fields read as after init_fields (no step since init or an injection)
   // the paired layout runs its table kernels on a one-case table: device
@@ -522,6 +525,7 @@ void free_all(LbmHandle* h) {
   const bool on_dev = cudaSetDevice(h->device) == cudaSuccess;
   if (on_dev) cudaDeviceSynchronize();
   for (void* p : ptrs) cache_release(p);
+  if (h->read) cudaEventDestroy(h->read);
   if (on_dev && cur >= 0) (void)cudaSetDevice(cur);
 }
 
@@ -540,6 +544,25 @@ int ndim_of(int64_t nz) { return nz == 1 ? 2 : 3; }
 // The python-double Allen-Cahn source coefficient 1 - 1 / (2 tau_f).
 double ac_of(const LbmHandle* h) { return 1.0 - 0.5 / (h->prm.tau_h > 0 ? h->prm.tau_h : h->prm.tau_l); }
 bool wants_s(const LbmHandle* h);
+
+// Whether work put on `st` is recorded into a graph.
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+    (void)cudaGetLastError();  // the legacy stream beside another stream's capture
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+
+// Orders what overwrites u on `st` after the read-outs of f that still read it
+// on some other stream.  (A capture cannot wait for work outside of it.)
+int after_reads(LbmHandle* h, cudaStream_t st) {
+  if (!h->read_open || capturing(st)) return LBM_OK;
+  CUDA_TRY(cudaStreamWaitEvent(st, h->read, 0));
+  h->read_open = false;
+  return LBM_OK;
+}
 
 // The 2-D step of the handle's current state (no bookkeeping).
 template <typename T>
@@ -715,9 +738,8 @@ int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid)
   return LBM_OK;
 }
 
-// The state's populations, rebuilt from S where the state is in source form: callers that
-// read or save f.  They are evaluated into the buffer the next step would
-// write, which then takes the place of the current one.
+// The populations of a state in source form, evaluated into the buffer the next
+// step would write.
 template <typename T, typename S>
 int expand_t(LbmHandle* h, cudaStream_t st) {
   State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
@@ -730,11 +752,15 @@ int expand_t(LbmHandle* h, cudaStream_t st) {
   CUDA_TRY((launch_expand<T, S>(consts_of<T>(*h), s, st)));
   return LBM_OK;
 }
-int ensure_populations(LbmHandle* h, cudaStream_t st) {
-  if (!h->sform) return LBM_OK;
-  const int rc = with_types(h->prec, [&](auto tag) {
+int expand(LbmHandle* h, cudaStream_t st) {
+  return with_types(h->prec, [&](auto tag) {
     return expand_t<typename decltype(tag)::T, typename decltype(tag)::S>(h, st);
   });
+}
+// From source form to stored populations, for what steps on from them.
+int ensure_populations(LbmHandle* h, cudaStream_t st) {
+  if (!h->sform) return LBM_OK;
+  const int rc = expand(h, st);
   if (rc != LBM_OK) return rc;
   std::swap(h->f[0], h->f[1]);
   h->sform = false;
@@ -744,6 +770,10 @@ int ensure_populations(LbmHandle* h, cudaStream_t st) {
 
 template <typename T, typename S>
 int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr) {
+  if (nsteps > 0) {
+    const int rc = after_reads(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   if (nsteps > 0 && h->tiling.tx != 0) {
     const int rc = ensure_populations(h, st);  // the fused kernel reads f
     if (rc != LBM_OK) return rc;
@@ -1116,6 +1146,10 @@ int lbm_init_fields(LbmHandle* h, const void* phi, const void* u, int src_dtype,
   // caller may free them on return as after a copy); elsewhere they are
   // staged through the (not yet used) second g buffer: 19 N T-elements hold
   // the 4 N source elements.
+  {
+    const int rc = after_reads(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   int in = h->cur;
   const void* dphi = phi;
   const void* du = u;
@@ -1220,6 +1254,10 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_autotune: call lbm_init_fields first");
   if (reps <= 0) reps = 5;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  {
+    const int rc = after_reads(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   const size_t ub = 3 * (size_t)h->Np * h->tsize;
   void* u_save = nullptr;
   CUDA_TRY(cudaMalloc(&u_save, ub));
@@ -1393,7 +1431,8 @@ int lbm_inject_droplet(LbmHandle* h, const double* center3, double radius, doubl
   if (!(radius >= 0.0) || !(xi > 0.0)) return fail(LBM_E_ARG, "lbm_inject_droplet: radius >= 0 and xi > 0 required");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   {
-    const int rc = ensure_populations(h, st);
+    int rc = after_reads(h, st);
+    if (rc == LBM_OK) rc = ensure_populations(h, st);
     if (rc != LBM_OK) return rc;
   }
   InjectParams ip;
@@ -1459,10 +1498,6 @@ int lbm_get_populations(LbmHandle* h, void* f, void* g, void* stream) {
   if (!h) return fail(LBM_E_ARG, "lbm_get_populations: null handle");
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_get_populations: not initialised");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (f) {
-    const int rc = ensure_populations(h, st);
-    if (rc != LBM_OK) return rc;
-  }
   cudaError_t e;
   // fin = the current state, phi_in = the latest phi, c_prev = its correction
   e = with_types(h->prec, [&](auto tag) {
@@ -1471,11 +1506,18 @@ int lbm_get_populations(LbmHandle* h, void* f, void* g, void* stream) {
     State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
     s.c_prev = h->c_last;
     if constexpr (sizeof(S) == sizeof(T)) {
-      if (is2d(h)) return launch_populations2d<T>(consts_of<T>(*h), s, h->raw, (T*)f, (T*)g, st);
+      if (is2d(h)) return launch_populations2d<T>(consts_of<T>(*h), s, h->raw, h->sform, ac_of(h), (T*)f, (T*)g, st);
     }
-    return launch_populations<T, S>(consts_of<T>(*h), s, h->raw, (T*)f, (T*)g, st);
+    return launch_populations<T, S>(consts_of<T>(*h), s, h->raw, h->sform, (T*)f, (T*)g, st);
   });
   if (e != cudaSuccess) return fail(LBM_E_CUDA, std::string("lbm_get_populations: ") + cudaGetErrorString(e));
+  if (f && h->sform && !capturing(st)) {
+    // f came from u, which the next step overwrites in place
+    if (!h->read) CUDA_TRY(cudaEventCreateWithFlags(&h->read, cudaEventDisableTiming));
+    if (h->read_open) CUDA_TRY(cudaStreamWaitEvent(st, h->read, 0));  // an earlier read, perhaps on another stream
+    CUDA_TRY(cudaEventRecord(h->read, st));
+    h->read_open = true;
+  }
   return LBM_OK;
 }
 
@@ -1637,8 +1679,10 @@ int lbm_save_state(LbmHandle* h, void* host, int64_t bytes, void* stream) {
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_save_state: call lbm_init_fields first");
   if (bytes != (int64_t)state_bytes(h)) return fail(LBM_E_ARG, "lbm_save_state: buffer size is not lbm_state_bytes");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  {
-    const int rc = ensure_populations(h, st);  // the blob holds populations
+  if (h->sform) {
+    // the blob holds populations: evaluated into the buffer the next step
+    // writes, which holds no state between steps
+    const int rc = expand(h, st);
     if (rc != LBM_OK) return rc;
   }
   StateHeader hd;
@@ -1666,7 +1710,8 @@ int lbm_save_state(LbmHandle* h, void* host, int64_t bytes, void* stream) {
   CUDA_TRY(cudaMemcpyAsync(&hd.status, h->counters + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   char* out = static_cast<char*>(host) + sizeof(StateHeader);
   for (const StatePart& p : state_parts(h)) {
-    CUDA_TRY(cudaMemcpyAsync(out, p.dev, p.bytes, cudaMemcpyDeviceToHost, st));
+    const void* src = p.dev == h->f[h->cur] && h->sform ? h->f[h->cur ^ 1] : p.dev;
+    CUDA_TRY(cudaMemcpyAsync(out, src, p.bytes, cudaMemcpyDeviceToHost, st));
     out += p.bytes;
   }
   CUDA_TRY(cudaStreamSynchronize(st));
@@ -2170,6 +2215,10 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
     --rest;
   }
   if (rest == 0) return LBM_OK;
+  for (LbmHandle* h : b->h) {
+    const int rc = after_reads(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   if (steps_apart(b)) return apart_step(b, rest, true, st);
   bool phis_in = false;
   int rc = batch_form(b, st, &phis_in);
@@ -2228,6 +2277,10 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   for (LbmHandle* h : b->h)
     if (!h->initialized || h->raw || h->first)
       return fail(LBM_E_STATE, "lbm_batch_autotune: every case must have taken a step");
+  for (LbmHandle* h : b->h) {
+    const int rc = after_reads(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   // time batched steps that re-read the current state (u, updated in place, is restored after)
   std::vector<void*> usave(b->h.size(), nullptr);
   for (size_t i = 0; i < b->h.size(); ++i) {

@@ -359,13 +359,10 @@ __device__ __forceinline__ T relax_scale(T target, T sum_f) {
   return s < T(0.5) ? T(0.5) : (s > T(2.0) ? T(2.0) : s);
 }
 
-// f at node n as the reference holds it at the start of the step.
-template <typename T, typename S, bool RAW, bool USE_POL = false, bool MAP = false>
-__device__ __forceinline__ void fetch_f(T (&v)[Q], const Consts<T>& k, const State<T, S>& s, int n, size_t N,
-                                        const Nbr& nb, uint8_t c, T eps, unsigned long long pol = 0ull) {
-  const T corr = RAW ? T(1) : s.cbuf[s.c_prev];
-  fetch_pop<T, S, RAW, !RAW, true, USE_POL, MAP>(v, k, s.fin, s.phi_in, n, N, nb, c, eps, corr, pol);
-  if (!RAW && k.relax_on && (c & kTop)) {
+// The boundary-phi relaxation of a node's corrected populations.
+template <typename T, typename S, bool MAP>
+__device__ __forceinline__ void relax_f(T (&v)[Q], const Consts<T>& k, const State<T, S>& s, int n, uint8_t c, T corr) {
+  if (k.relax_on && (c & kTop)) {
     const T r = relax_target<T, MAP>(k, s.phi_in, s.nsw, s.cubic, n,
                                      ld_state(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)), corr);
     if (r >= T(0)) {
@@ -374,6 +371,15 @@ __device__ __forceinline__ void fetch_f(T (&v)[Q], const Consts<T>& k, const Sta
       for (int q = 0; q < Q; ++q) v[q] = mul_rn(v[q], sc);
     }
   }
+}
+
+// f at node n as the reference holds it at the start of the step.
+template <typename T, typename S, bool RAW, bool USE_POL = false, bool MAP = false>
+__device__ __forceinline__ void fetch_f(T (&v)[Q], const Consts<T>& k, const State<T, S>& s, int n, size_t N,
+                                        const Nbr& nb, uint8_t c, T eps, unsigned long long pol = 0ull) {
+  const T corr = RAW ? T(1) : s.cbuf[s.c_prev];
+  fetch_pop<T, S, RAW, !RAW, true, USE_POL, MAP>(v, k, s.fin, s.phi_in, n, N, nb, c, eps, corr, pol);
+  if (!RAW) relax_f<T, S, MAP>(v, k, s, n, c, corr);
 }
 
 // phi of fluid node n from its populations v (pulled, bounced back and blended):
@@ -1879,8 +1885,10 @@ __global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, 
 }
 
 // Current populations in the reference layout: s.fin/s.gin hold the last
-// step's output, s.phi_in that step's phi and s.c_prev its correction.
-template <typename T, typename S, bool RAW>
+// step's output, s.phi_in that step's phi and s.c_prev its correction.  SRC:
+// s.fin holds S; the 19 pulled values are evaluated from their nodes' phi, u
+// and S, so that a read-out writes nothing of the state.
+template <typename T, typename S, bool RAW, bool SRC = false>
 __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
@@ -1892,7 +1900,8 @@ __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S>
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q];
   if (f_o) {
-    fetch_f<T, S, RAW, false, true>(v, k, s, n, N, nb, c, eps);
+    if constexpr (SRC) fetch_f_source<S>(v, k, s, n, nb, c, eps);
+    else fetch_f<T, S, RAW, false, true>(v, k, s, n, N, nb, c, eps);
 #pragma unroll
     for (int q = 0; q < Q; ++q) f_o[(size_t)q * N + n] = v[q];
   }
@@ -2385,8 +2394,17 @@ cudaError_t launch_observe(const Consts<T>& k, const State<T, S>& s, bool raw_in
 }
 
 template <typename T, typename S>
-cudaError_t launch_populations(const Consts<T>& k, const State<T, S>& s, bool raw, T* f, T* g, cudaStream_t st) {
+cudaError_t launch_populations(const Consts<T>& k, const State<T, S>& s, bool raw, bool src, T* f, T* g,
+                               cudaStream_t st) {
   const int grid = (k.N + kBlock - 1) / kBlock;
+  if (src) {
+    if constexpr (sizeof(T) == 8) {
+      return cudaErrorNotSupported;
+    } else {
+      k_populations<T, S, false, true><<<grid, kBlock, 0, st>>>(k, s, f, g);
+      return cudaGetLastError();
+    }
+  }
   if (raw) k_populations<T, S, true><<<grid, kBlock, 0, st>>>(k, s, f, g);
   else k_populations<T, S, false><<<grid, kBlock, 0, st>>>(k, s, f, g);
   return cudaGetLastError();
@@ -2499,7 +2517,8 @@ template cudaError_t launch_measure_static<double>(int, int, int, const double*,
                                                  const double*, cudaStream_t);                                    \
   template cudaError_t launch_observe<T, S>(const Consts<T>&, const State<T, S>&, bool, unsigned, int, T*, T*, T*, \
                                             T*, T*, T*, cudaStream_t);                                           \
-  template cudaError_t launch_populations<T, S>(const Consts<T>&, const State<T, S>&, bool, T*, T*, cudaStream_t);  \
+  template cudaError_t launch_populations<T, S>(const Consts<T>&, const State<T, S>&, bool, bool, T*, T*,       \
+                                                 cudaStream_t);                                                  \
   template cudaError_t launch_inject<T, S>(const Consts<T>&, const State<T, S>&, bool, const InjectParams&,        \
                                            const T*, unsigned*, cudaStream_t);
 

@@ -817,9 +817,32 @@ __global__ void __launch_bounds__(kBlock) k2_observe(Consts<T> k, State<T, T> s,
   }
 }
 
-// Current populations in the reference layout [9][N].
-template <typename T, bool RAW>
-__global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T> s, T* f_o, T* g_o) {
+// fetch_f9 of a state in source form (s.fin holds S): each slot that node n
+// reads, evaluated at the slot's node.
+template <typename T>
+__device__ __forceinline__ void fetch_f9_source(T (&v)[Q9], const Consts<T>& k, const State<T, T>& s, int n, const Nb2& nb,
+                                                uint8_t c, T eps, T acT) {
+  const int Np = k.Np;
+  const T corr = s.cbuf[s.c_prev], one_m = T(1) - eps;
+  auto slot = [&](int q, int m) {
+    T f[Q9];
+    f_of_source<T>(s.phi_in[m], s.u[m], s.u[Np + m], s.fin[m], s.fin[Np + m], acT, f);
+    return f[q];
+  };
+#pragma unroll
+  for (int q = 0; q < Q9; ++q) {
+    const int m = nb.at(n, -ex(q), -ey(q));
+    if (c & kSolid) v[q] = slot(opp(q), n);
+    else if (c & kPartial) v[q] = one_m * slot(q, m) + eps * slot(opp(q), n);
+    else v[q] = slot(q, m);
+    v[q] = v[q] * corr;
+  }
+  relax9(v, k, s, n, c, corr);
+}
+
+// Current populations in the reference layout [9][N].  SRC: s.fin holds S.
+template <typename T, bool RAW, bool SRC = false>
+__global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T> s, double ac, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const uint8_t c = s.cls[n];
@@ -827,7 +850,8 @@ __global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q9];
   if (f_o) {
-    fetch_f9<T, RAW>(v, k, s, n, nb, c, eps);
+    if constexpr (SRC) fetch_f9_source<T>(v, k, s, n, nb, c, eps, (T)ac);
+    else fetch_f9<T, RAW>(v, k, s, n, nb, c, eps);
 #pragma unroll
     for (int q = 0; q < Q9; ++q) f_o[q * k.N + n] = v[q];
   }
@@ -1019,10 +1043,12 @@ cudaError_t launch_observe2d(const Consts<T>& k, const State<T, T>& s, bool raw_
 }
 
 template <typename T>
-cudaError_t launch_populations2d(const Consts<T>& k, const State<T, T>& s, bool raw, T* f, T* g, cudaStream_t st) {
+cudaError_t launch_populations2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool src, double ac, T* f, T* g,
+                                 cudaStream_t st) {
   const int nb = d2::blocks_of(k.N);
-  if (raw) d2::k2_populations<T, true><<<nb, kBlock, 0, st>>>(k, s, f, g);
-  else d2::k2_populations<T, false><<<nb, kBlock, 0, st>>>(k, s, f, g);
+  if (src) d2::k2_populations<T, false, true><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
+  else if (raw) d2::k2_populations<T, true><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
+  else d2::k2_populations<T, false><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
   return cudaGetLastError();
 }
 
@@ -1045,7 +1071,8 @@ cudaError_t launch_inject2d(const Consts<T>& k, const State<T, T>& s, bool raw, 
   template cudaError_t launch_expand2d<T>(const Consts<T>&, const State<T, T>&, double, cudaStream_t);              \
   template cudaError_t launch_observe2d<T>(const Consts<T>&, const State<T, T>&, bool, unsigned, int, T*, T*, T*,   \
                                            T*, T*, T*, cudaStream_t);                                               \
-  template cudaError_t launch_populations2d<T>(const Consts<T>&, const State<T, T>&, bool, T*, T*, cudaStream_t);  \
+  template cudaError_t launch_populations2d<T>(const Consts<T>&, const State<T, T>&, bool, bool, double, T*, T*,   \
+                                               cudaStream_t);                                                       \
   template cudaError_t launch_inject2d<T>(const Consts<T>&, const State<T, T>&, bool, const InjectParams&, const T*, \
                                           unsigned*, cudaStream_t);
 LBM_INST2D(float)

@@ -101,6 +101,38 @@ __device__ __forceinline__ void feval_all(const Consts<float>& k, float phi, con
   }
 }
 
+// fetch_f of a state in source form (s.fin holds S): the value of each slot
+// that node n reads, evaluated at the slot's node.  Linear layout.
+template <typename S>
+__device__ __forceinline__ void fetch_f_source(float (&v)[Q], const Consts<float>& k, const State<float, S>& s, int n,
+                                               const Nbr& nb, uint8_t c, float eps) {
+  constexpr bool DEV = PopIO<float, S>::kDev;
+  const float* src = reinterpret_cast<const float*>(s.fin);
+  const unsigned Np = (unsigned)k.Np;
+  const float corr = s.cbuf[s.c_prev];
+  // population q of node m, stored with the deviation reference ref and read back
+  auto slot = [&](int q, unsigned m, float ref) {
+    const float u[3] = {s.u[m], s.u[Np + m], s.u[2 * Np + m]}, sv[3] = {src[m], src[Np + m], src[2 * Np + m]};
+    float f[Q];
+    feval_all<S>(k, s.phi_in[m], u, sv, f);
+    return DEV ? stored_f<S>(k, q, f[q], ref) : f[q];
+  };
+  const float ref_self = DEV ? s.phi_in[n] : 0.0f, one_m = sub_rn(1.0f, eps);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const unsigned m = (unsigned)nb.at(n, -ex(q), -ey(q), -ez(q));
+    if (c & (kSolid | kPartial)) {
+      // the node's own opposite slot: its reader is x - e_q
+      const float o = slot(opp(q), (unsigned)n, DEV ? s.phi_in[m] : 0.0f);
+      v[q] = (c & kSolid) ? o : fma_(one_m, slot(q, m, ref_self), mul_rn(eps, o));
+    } else {
+      v[q] = slot(q, m, ref_self);
+    }
+    v[q] = mul_rn(v[q], corr);
+  }
+  relax_f<float, S, false>(v, k, s, n, c, corr);
+}
+
 template <typename S>
 __device__ __forceinline__ void phis_block(const Consts<float>& k, const State<float, S>& s, const PhiTile& t, int b,
                                            int nblk, float2* sm) {
