@@ -71,7 +71,7 @@ cudaError_t launch_batch_coop(const void*, const unsigned short*, int, int, int,
 template <typename T, typename Src>
 cudaError_t launch_init2d(const Consts<T>&, const State<T, T>&, const Src*, const Src*, cudaStream_t);
 template <typename T>
-cudaError_t launch_step2d(const Consts<T>&, const State<T, T>&, bool, bool, bool, bool, double, cudaStream_t,
+cudaError_t launch_step2d(const Consts<T>&, const State<T, T>&, bool, bool, Form, bool, double, cudaStream_t,
                           cudaEvent_t);
 template <typename T>
 cudaError_t launch_expand2d(const Consts<T>&, const State<T, T>&, double, cudaStream_t);
@@ -139,7 +139,8 @@ struct LbmHandle {
   uint8_t* cls = nullptr;
   float* wn = nullptr;
   double* partials = nullptr;
-  unsigned* counters = nullptr;  // [0] step/init reductions, [1] measure, [2] status, [3] inject, [4] momentum
+  // [0] step/init reductions, [1] measure, [2] status, [3] inject, [4] momentum, [5] form (State::form)
+  unsigned* counters = nullptr;
   void* cbuf = nullptr;          // 2 x T
   double* scal = nullptr;        // [0] phi_mass_init [1] last sum [2..10] measure output [16..21] extents [24..26] momentum
   void* meas_phi = nullptr;      // N x T scratch for lbm_measure
@@ -162,6 +163,10 @@ struct LbmHandle {
   bool first = true;      // phi*u of the previous step does not exist yet
   PhiTile tile{};         // work split of the source form's phi pass (phis_tile of the grid alone)
   bool sform = false;     // f[cur] holds S (a T per dimension and node) instead of the populations (lbm_phis.cuh)
+  // Steps of this grid have been captured into a graph, whose replays change
+  // the form without the host: only the device's word tells it.
+  bool dual = false;
+  bool form_set = false;  // the device's word may be non-zero
   int c_last = 0;         // cbuf slot of the last step's correction
   int64_t steps = 0;
   // read-outs of f in source form read u: their end, which what overwrites u waits for (after_reads)
@@ -355,6 +360,8 @@ State<T, S> make_state(const LbmHandle& h, int in_buf, int phi_in) {
   s.cbuf = static_cast<T*>(h.cbuf);
   s.scal = h.scal;
   s.status = h.counters + 2;
+  s.form = h.counters + 5;
+  s.form_if = -1;
   return s;
 }
 
@@ -564,13 +571,45 @@ int after_reads(LbmHandle* h, cudaStream_t st) {
   return LBM_OK;
 }
 
-// The 2-D step of the handle's current state (no bookkeeping).
+// The form of f as the host knows it.
+Form form_of(const LbmHandle* h) {
+  if (h->raw || !wants_s(h)) return Form::populations;
+  return h->dual ? Form::any : h->sform ? Form::source : Form::populations;
+}
+
+// The device's word of the form: populations (asynchronous).
+int clear_form(LbmHandle* h, cudaStream_t st) {
+  if (h->form_set || h->dual || capturing(st)) CUDA_TRY(cudaMemsetAsync(h->counters + 5, 0, sizeof(unsigned), st));
+  h->form_set = h->sform = false;
+  return LBM_OK;
+}
+// What the host knows of the form (exactly that of f: not any), after kernels that wrote S without advancing the state.
+int restore_form(LbmHandle* h, cudaStream_t st) {
+  CUDA_TRY(cudaMemsetAsync(h->counters + 5, h->sform ? 1 : 0, sizeof(unsigned), st));
+  h->form_set = h->sform;
+  return LBM_OK;
+}
+// h->sform from the device's word where only that tells it (waits for `st`).
+int read_form(LbmHandle* h, cudaStream_t st) {
+  if (form_of(h) != Form::any) return LBM_OK;
+  unsigned w = 0;
+  CUDA_TRY(cudaMemcpyAsync(&w, h->counters + 5, sizeof(w), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  h->sform = w != 0;
+  return LBM_OK;
+}
+// Before steps on `st`.
+void note_capture(LbmHandle* h, cudaStream_t st) {
+  if (!h->dual && wants_s(h) && capturing(st)) h->dual = true;
+}
+
+// The 2-D step of the handle's current state, whose f has the form `in` (no bookkeeping).
 template <typename T>
-int launch_next2d(LbmHandle* h, cudaStream_t st, cudaEvent_t mid) {
+int launch_next2d(LbmHandle* h, Form in, cudaStream_t st, cudaEvent_t mid) {
   State<T, T> s = make_state<T, T>(*h, h->cur, h->pc);
   s.c_prev = h->c_last;
   s.c_cur = h->c_last ^ 1;
-  CUDA_TRY(launch_step2d<T>(consts_of<T>(*h), s, h->raw, h->first, h->sform, wants_s(h), ac_of(h), st, mid));
+  CUDA_TRY(launch_step2d<T>(consts_of<T>(*h), s, h->raw, h->first, in, wants_s(h), ac_of(h), st, mid));
   return LBM_OK;
 }
 
@@ -700,10 +739,12 @@ int fill_desc(LbmHandle* h, cudaStream_t st) {
 // Launches the step that would run next (no bookkeeping): the first step
 // after init and the fused kernel through launch_step; every other
 // two-kernel step through the kernels of a grid alone (linear layout), or the
-// paired kernels on the handle's one-case table.  `mid` (may be null)
-// is recorded between the two kernels (before the fused kernel).
+// paired kernels on the handle's one-case table.  in: the form of f (any: the phi
+// kernels of both forms, of which the state's runs; measured about 2 us more than
+// one of them).  `mid` (may be null) is recorded between the two kernels
+// (before the fused kernel).
 template <typename T, typename S>
-int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid) {
+int launch_next(LbmHandle* h, const Tiling& t, Form in, cudaStream_t st, cudaEvent_t mid) {
   if (t.tx == 0 && !h->raw && !h->first) {
     const bool gmu = h->mu != nullptr;
     State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
@@ -720,10 +761,22 @@ int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid)
       CUDA_TRY((launch_phi_pair<T, S>(d, nullptr, phi_blocks_of(h, h->phi_per_thread, true), st)));
     } else {
       if (case_desc_bytes<T, S>() > kDescBytes) return fail(LBM_E_ARG, "lbm_step: internal error: descriptor size");
-      fill_case_desc<T, S>(one, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread, true), 0,
-                           upd_blocks_of(h, h->upd_block), 0, h->tile);
-      if (h->sform) CUDA_TRY((launch_phis_one<T, S>(d, st)));
-      else CUDA_TRY((launch_phi_one<T, S>(d, st)));
+      auto fill = [&](int form_if) {
+        s.form_if = form_if;
+        fill_case_desc<T, S>(one, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread, true), 0,
+                             upd_blocks_of(h, h->upd_block), 0, h->tile);
+      };
+      if (in == Form::any) {
+        fill(1);
+        CUDA_TRY((launch_phis_one<T, S>(d, st)));
+        fill(0);
+        CUDA_TRY((launch_phi_one<T, S>(d, st)));
+        fill(-1);
+      } else {
+        fill(-1);
+        if (in == Form::source) CUDA_TRY((launch_phis_one<T, S>(d, st)));
+        else CUDA_TRY((launch_phi_one<T, S>(d, st)));
+      }
     }
     if (mid) CUDA_TRY(cudaEventRecord(mid, st));
     if (gmu) CUDA_TRY((launch_mu<T, S>(consts_of<T>(*h), s, st)));
@@ -739,10 +792,17 @@ int launch_next(LbmHandle* h, const Tiling& t, cudaStream_t st, cudaEvent_t mid)
 }
 
 // The populations of a state in source form, evaluated into the buffer the next
-// step would write.
+// step would write, or in place: f stays where it is, for steps captured before,
+// and S is read from a copy in the other buffer.
 template <typename T, typename S>
-int expand_t(LbmHandle* h, cudaStream_t st) {
+int expand_t(LbmHandle* h, bool in_place, cudaStream_t st) {
   State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
+  if (form_of(h) == Form::any) s.form_if = 1;
+  if (in_place) {
+    CUDA_TRY(cudaMemcpyAsync(s.fout, s.fin, (size_t)ndim_of(h->nz) * h->Np * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    s.fin = s.fout;
+    s.fout = static_cast<S*>(h->f[h->cur]);
+  }
   if constexpr (sizeof(T) == sizeof(S)) {
     if (is2d(h)) {
       CUDA_TRY((launch_expand2d<T>(consts_of<T>(*h), s, ac_of(h), st)));
@@ -752,43 +812,41 @@ int expand_t(LbmHandle* h, cudaStream_t st) {
   CUDA_TRY((launch_expand<T, S>(consts_of<T>(*h), s, st)));
   return LBM_OK;
 }
-int expand(LbmHandle* h, cudaStream_t st) {
+int expand(LbmHandle* h, bool in_place, cudaStream_t st) {
   return with_types(h->prec, [&](auto tag) {
-    return expand_t<typename decltype(tag)::T, typename decltype(tag)::S>(h, st);
+    return expand_t<typename decltype(tag)::T, typename decltype(tag)::S>(h, in_place, st);
   });
 }
 // From source form to stored populations, for what steps on from them.
 int ensure_populations(LbmHandle* h, cudaStream_t st) {
-  if (!h->sform) return LBM_OK;
-  const int rc = expand(h, st);
-  if (rc != LBM_OK) return rc;
-  std::swap(h->f[0], h->f[1]);
-  h->sform = false;
-  h->desc_ok = false;
-  return LBM_OK;
+  if (form_of(h) == Form::populations) return LBM_OK;
+  const int rc = expand(h, true, st);
+  return rc == LBM_OK ? clear_form(h, st) : rc;
 }
 
 template <typename T, typename S>
 int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr) {
   if (nsteps > 0) {
-    const int rc = after_reads(h, st);
+    note_capture(h, st);
+    int rc = after_reads(h, st);
+    if (rc == LBM_OK && h->tiling.tx != 0) rc = ensure_populations(h, st);  // the fused kernel reads f
     if (rc != LBM_OK) return rc;
   }
-  if (nsteps > 0 && h->tiling.tx != 0) {
-    const int rc = ensure_populations(h, st);  // the fused kernel reads f
-    if (rc != LBM_OK) return rc;
-  }
+  Form form = form_of(h);
+  if (h->tiling.tx != 0) form = Form::populations;
   for (int i = 0; i < nsteps; ++i) {
     if (ev) CUDA_TRY(cudaEventRecord(ev[2 * i], st));
     int rc;
     if constexpr (sizeof(S) == sizeof(T)) {
-      rc = is2d(h) ? launch_next2d<T>(h, st, ev ? ev[2 * i + 1] : nullptr)
-                   : launch_next<T, S>(h, h->tiling, st, ev ? ev[2 * i + 1] : nullptr);
+      rc = is2d(h) ? launch_next2d<T>(h, form, st, ev ? ev[2 * i + 1] : nullptr)
+                   : launch_next<T, S>(h, h->tiling, form, st, ev ? ev[2 * i + 1] : nullptr);
     } else {
-      rc = launch_next<T, S>(h, h->tiling, st, ev ? ev[2 * i + 1] : nullptr);
+      rc = launch_next<T, S>(h, h->tiling, form, st, ev ? ev[2 * i + 1] : nullptr);
     }
     if (rc != LBM_OK) return rc;
     h->sform = !h->raw && h->tiling.tx == 0 && wants_s(h);  // the first step writes populations
+    h->form_set = h->form_set || h->sform;
+    form = h->sform ? Form::source : Form::populations;
     h->last_raw_in = h->raw;
     h->obs_init = false;
     h->cur ^= 1;
@@ -811,10 +869,11 @@ namespace {
 template <typename T, typename S>
 int time_tiling(LbmHandle* h, const Tiling& t, int reps, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1,
                 float* ms) {
-  int rc = launch_next<T, S>(h, t, st, nullptr);  // warm-up (sets smem attributes)
+  const Form form = h->sform ? Form::source : Form::populations;
+  int rc = launch_next<T, S>(h, t, form, st, nullptr);  // warm-up (sets smem attributes)
   if (rc != LBM_OK) return rc;
   CUDA_TRY(cudaEventRecord(e0, st));
-  for (int i = 0; i < reps && rc == LBM_OK; ++i) rc = launch_next<T, S>(h, t, st, nullptr);
+  for (int i = 0; i < reps && rc == LBM_OK; ++i) rc = launch_next<T, S>(h, t, form, st, nullptr);
   if (rc != LBM_OK) return rc;
   CUDA_TRY(cudaEventRecord(e1, st));
   CUDA_TRY(cudaEventSynchronize(e1));
@@ -1179,9 +1238,12 @@ int lbm_init_fields(LbmHandle* h, const void* phi, const void* u, int src_dtype,
   });
   if (e != cudaSuccess) return fail(LBM_E_CUDA, std::string("lbm_init_fields: ") + cudaGetErrorString(e));
   if (direct) CUDA_TRY(cudaStreamSynchronize(st));
+  {
+    const int rc = clear_form(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   h->initialized = true;
   h->desc_ok = false;
-  h->sform = false;
   h->raw = true;
   h->first = true;
   h->c_last = 0;
@@ -1255,7 +1317,8 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
   if (reps <= 0) reps = 5;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   {
-    const int rc = after_reads(h, st);
+    int rc = after_reads(h, st);
+    if (rc == LBM_OK) rc = read_form(h, st);
     if (rc != LBM_OK) return rc;
   }
   const size_t ub = 3 * (size_t)h->Np * h->tsize;
@@ -1331,6 +1394,7 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
     h->desc_ok = false;
   }
   cudaMemcpyAsync(h->u, u_save, ub, cudaMemcpyDeviceToDevice, st);
+  if (rc == LBM_OK) rc = restore_form(h, st);
   cudaStreamSynchronize(st);
   cudaFree(u_save);
   cudaEventDestroy(e0);
@@ -1483,7 +1547,6 @@ int lbm_inject_droplet(LbmHandle* h, const double* center3, double radius, doubl
   h->first = true;
   h->obs_init = true;
   h->last_raw_in = true;
-  h->sform = false;
   h->desc_ok = false;
   if (core_nodes) {
     unsigned cnt = 0;
@@ -1499,19 +1562,28 @@ int lbm_get_populations(LbmHandle* h, void* f, void* g, void* stream) {
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_get_populations: not initialised");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e;
+  // a captured read-out replays on a state of either form
+  const Form form = !f ? Form::populations : form_of(h) == Form::any || (wants_s(h) && !h->raw && capturing(st))
+                                                 ? Form::any : form_of(h);
   // fin = the current state, phi_in = the latest phi, c_prev = its correction
   e = with_types(h->prec, [&](auto tag) {
     using T = typename decltype(tag)::T;
     using S = typename decltype(tag)::S;
     State<T, S> s = make_state<T, S>(*h, h->cur, h->pc);
     s.c_prev = h->c_last;
-    if constexpr (sizeof(S) == sizeof(T)) {
-      if (is2d(h)) return launch_populations2d<T>(consts_of<T>(*h), s, h->raw, h->sform, ac_of(h), (T*)f, (T*)g, st);
-    }
-    return launch_populations<T, S>(consts_of<T>(*h), s, h->raw, h->sform, (T*)f, (T*)g, st);
+    auto launch = [&](bool src, int form_if) {
+      s.form_if = form_if;
+      if constexpr (sizeof(S) == sizeof(T)) {
+        if (is2d(h)) return launch_populations2d<T>(consts_of<T>(*h), s, h->raw, src, ac_of(h), (T*)f, (T*)g, st);
+      }
+      return launch_populations<T, S>(consts_of<T>(*h), s, h->raw, src, (T*)f, (T*)g, st);
+    };
+    if (form != Form::any) return launch(form == Form::source, -1);
+    const cudaError_t r = launch(true, 1);
+    return r == cudaSuccess ? launch(false, 0) : r;
   });
   if (e != cudaSuccess) return fail(LBM_E_CUDA, std::string("lbm_get_populations: ") + cudaGetErrorString(e));
-  if (f && h->sform && !capturing(st)) {
+  if (form != Form::populations && !capturing(st)) {
     // f came from u, which the next step overwrites in place
     if (!h->read) CUDA_TRY(cudaEventCreateWithFlags(&h->read, cudaEventDisableTiming));
     if (h->read_open) CUDA_TRY(cudaStreamWaitEvent(st, h->read, 0));  // an earlier read, perhaps on another stream
@@ -1679,10 +1751,11 @@ int lbm_save_state(LbmHandle* h, void* host, int64_t bytes, void* stream) {
   if (!h->initialized) return fail(LBM_E_STATE, "lbm_save_state: call lbm_init_fields first");
   if (bytes != (int64_t)state_bytes(h)) return fail(LBM_E_ARG, "lbm_save_state: buffer size is not lbm_state_bytes");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (h->sform) {
+  {
+    int rc = read_form(h, st);
     // the blob holds populations: evaluated into the buffer the next step
     // writes, which holds no state between steps
-    const int rc = expand(h, st);
+    if (rc == LBM_OK && h->sform) rc = expand(h, false, st);
     if (rc != LBM_OK) return rc;
   }
   StateHeader hd;
@@ -1752,6 +1825,10 @@ int lbm_load_state(LbmHandle* h, const void* host, int64_t bytes, void* stream) 
     in += p.bytes;
   }
   CUDA_TRY(cudaMemcpyAsync(h->counters + 2, &hd.status, sizeof(unsigned), cudaMemcpyHostToDevice, st));
+  {
+    const int rc = clear_form(h, st);
+    if (rc != LBM_OK) return rc;
+  }
   CUDA_TRY(cudaStreamSynchronize(st));
   h->raw = hd.raw != 0;
   h->first = hd.first != 0;
@@ -1759,7 +1836,6 @@ int lbm_load_state(LbmHandle* h, const void* host, int64_t bytes, void* stream) 
   h->obs_init = hd.obs_init != 0;
   h->steps = hd.steps;
   h->initialized = true;
-  h->sform = false;
   h->desc_ok = false;
   return LBM_OK;
 }
@@ -1985,7 +2061,7 @@ cudaError_t batch_launch(LbmBatch* b, int par, bool phis_in, cudaStream_t st) {
 int batch_form(LbmBatch* b, cudaStream_t st, bool* phis_in) {
   bool all = !b->coop;
   for (LbmHandle* h : b->h)
-    if (wants_s(h)) all = all && h->sform;
+    if (wants_s(h)) all = all && form_of(h) == Form::source;
   if (!all)
     for (LbmHandle* h : b->h) {
       const int rc = ensure_populations(h, st);
@@ -2077,14 +2153,16 @@ int apart_step_t(LbmBatch* b, int nsteps, bool advance, cudaStream_t st) {
   for (int k = 0; k < nsteps && rc == LBM_OK; ++k)
     for (size_t i = 0; i < b->h.size() && rc == LBM_OK; ++i) {
       LbmHandle* h = b->h[i];
+      Form form = k == 0 && advance ? form_of(h) : h->sform ? Form::source : Form::populations;
       const int per = h->phi_per_thread, bs = h->upd_block;
       h->phi_per_thread = b->phi_per_thread;
       h->upd_block = b->upd_block;
-      rc = launch_next<T, S>(h, Tiling{}, b->lanes[b->lane_of[i]], nullptr);
+      rc = launch_next<T, S>(h, Tiling{}, form, b->lanes[b->lane_of[i]], nullptr);
       h->phi_per_thread = per;
       h->upd_block = bs;
       if (rc == LBM_OK && advance) {
         h->sform = wants_s(h);
+        h->form_set = h->form_set || h->sform;
         h->last_raw_in = h->obs_init = false;
         h->cur ^= 1;
         h->pc ^= 1;
@@ -2115,6 +2193,7 @@ void batch_advance(LbmBatch* b, int nsteps) {
     }
     h->steps += nsteps;
     if (nsteps > 0) h->sform = !b->coop && wants_s(h);
+    h->form_set = h->form_set || h->sform;
     h->last_raw_in = false;
     h->obs_init = false;
   }
@@ -2216,6 +2295,7 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
   }
   if (rest == 0) return LBM_OK;
   for (LbmHandle* h : b->h) {
+    note_capture(h, st);
     const int rc = after_reads(h, st);
     if (rc != LBM_OK) return rc;
   }
@@ -2278,7 +2358,8 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
     if (!h->initialized || h->raw || h->first)
       return fail(LBM_E_STATE, "lbm_batch_autotune: every case must have taken a step");
   for (LbmHandle* h : b->h) {
-    const int rc = after_reads(h, st);
+    int rc = after_reads(h, st);
+    if (rc == LBM_OK) rc = read_form(h, st);
     if (rc != LBM_OK) return rc;
   }
   // time batched steps that re-read the current state (u, updated in place, is restored after)
@@ -2330,6 +2411,7 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   for (size_t i = 0; i < b->h.size(); ++i) {
     const size_t ub = 3 * (size_t)b->h[i]->Np * b->h[i]->tsize;
     cudaMemcpyAsync(b->h[i]->u, usave[i], ub, cudaMemcpyDeviceToDevice, st);
+    if (rc == LBM_OK && wants_s(b->h[i])) rc = restore_form(b->h[i], st);
   }
   cudaStreamSynchronize(st);
   for (void* p : usave) cudaFree(p);

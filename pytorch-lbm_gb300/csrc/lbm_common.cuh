@@ -228,7 +228,21 @@ struct State {
   double* scal;     // [0] phi_mass_init, [1] last sum(phi)
   unsigned* status;
   int c_prev, c_cur;  // cbuf slots: factor applied to fin, factor produced this step
+  // The form of the state on the device: *form is non-zero while it is the
+  // source form (lbm_phis.cuh).  form_if 0 or 1: the kernel runs only on a state
+  // of stored populations or of the source form; -1: the host knows the form.
+  unsigned* form;
+  int form_if;
 };
+
+// What the host knows of the form.
+enum class Form { populations, source, any };
+
+// Whether this kernel is the other form's.
+template <typename T, typename S>
+__device__ __forceinline__ bool other_form(const State<T, S>& s) {
+  return s.form_if >= 0 && (*(const volatile unsigned*)s.form != 0u) != (s.form_if != 0);
+}
 
 // Droplet to inject mid-run (lbm/fe_ac_solver.py:645-732): centre, radius,
 // interface width, impact velocity; obs_init: the attributes phi, u, P are

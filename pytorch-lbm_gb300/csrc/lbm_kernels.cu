@@ -1438,6 +1438,7 @@ template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS>
 __device__ __forceinline__ void update_block(const Consts<T>& k, const State<T, S>& s, int n0) {
   const int n = n0 + threadIdx.x, P = k.ny * k.nz;
   const Pol pol = Pol::make();
+  if (SOUT && n == 0) *s.form = 1u;
   if (n0 >= P && n0 + BS <= k.N - P) {
     int ix, iy, iz;
     decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
@@ -1585,6 +1586,7 @@ template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 3 : 4) k_phi_one(const __grid_constant__ CaseDesc<T, S> d) {
   pdl_trigger();
   pdl_wait();  // f of the previous update kernel
+  if (other_form(d.s)) return;
   phi_block(d.k, d.s, blockIdx.x, gridDim.x);
 }
 template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS = kBlock>
@@ -1891,7 +1893,7 @@ __global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, 
 template <typename T, typename S, bool RAW, bool SRC = false>
 __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
+  if (n >= k.N || other_form(s)) return;
   const size_t N = (size_t)k.N;
   const uint8_t c = s.cls[n];
   int ix, iy, iz;

@@ -408,6 +408,7 @@ template <typename T, bool RAW>
 __global__ void __launch_bounds__(kBlock) k2_phi(Consts<T> k, State<T, T> s) {
   pdl_trigger();
   pdl_wait();  // f of the previous update kernel
+  if (other_form(s)) return;
   double pd = 0.0;
   unsigned long long pu = 0ull;
   bool nan = false;
@@ -450,7 +451,7 @@ __device__ __forceinline__ void f_of_source(T phi, T u0, T u1, T S0, T S1, T acT
 template <typename T>
 __global__ void __launch_bounds__(kBlock) k2_expand(Consts<T> k, State<T, T> s, double ac) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
+  if (n >= k.N || other_form(s)) return;
   T f[Q9];
   f_of_source<T>(s.phi_in[n], s.u[n], s.u[k.Np + n], s.fin[n], s.fin[k.Np + n], (T)ac, f);
 #pragma unroll
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(kMaxBlock, 3) k2_phis(Consts<T> k, State<T, T>
   __shared__ T sm[4][6][kMaxBlock];
   pdl_trigger();
   pdl_wait();  // S and u of the previous update kernel
+  if (other_form(s)) return;
   const int chunk = blockIdx.x / nwin, win = blockIdx.x - chunk * nwin;
   const int y0 = win * w_, ew = min(w_, k.ny - y0), x0 = chunk * cx, x1 = min(x0 + cx, k.nx);
   const int t = threadIdx.x, Np = k.Np;
@@ -762,6 +764,7 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
     s.gout[q * Np + n] = (g[q] - om * (g[q] - geq)) + G[q];
   }
   if (SOUT) {
+    if (n == 0) *s.form = 1u;
     s.fout[n] = S0;
     s.fout[Np + n] = S1;
   }
@@ -844,7 +847,7 @@ __device__ __forceinline__ void fetch_f9_source(T (&v)[Q9], const Consts<T>& k, 
 template <typename T, bool RAW, bool SRC = false>
 __global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T> s, double ac, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
+  if (n >= k.N || other_form(s)) return;
   const uint8_t c = s.cls[n];
   const Nb2 nb = make_nb2(k, n);
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
@@ -996,15 +999,23 @@ cudaError_t launch_expand2d(const Consts<T>& k, const State<T, T>& s, double ac,
 }
 
 // One step: k2_phi, [k2_mu, k2_gradmu], k2_update.  `mid` (may be null) is
-// recorded between the phi kernel and the rest.  sin: s.fin is in source form;
-// sout: s.fout is to be (not raw, not first).
+// recorded between the phi kernel and the rest.  in: the form of s.fin (any: the
+// phi kernels of both forms, of which the state's runs); sout: s.fout is to be
+// in source form (not raw, not first).
 template <typename T>
-cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool first, bool sin, bool sout, double ac,
+cudaError_t launch_step2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool first, Form in, bool sout, double ac,
                           cudaStream_t st, cudaEvent_t mid) {
   const int nb = d2::blocks_of(k.N), np = d2::phi_blocks_of(k.N);
-  cudaError_t e = sin ? launch_phis2d<T>(k, s, ac, st)
-                  : raw ? launch_pdl(d2::k2_phi<T, true>, np, st, k, s)
-                        : launch_pdl(d2::k2_phi<T, false>, np, st, k, s);
+  State<T, T> sp = s;
+  cudaError_t e = cudaSuccess;
+  if (in != Form::populations) {
+    if (in == Form::any) sp.form_if = 1;
+    e = launch_phis2d<T>(k, sp, ac, st);
+  }
+  if (e == cudaSuccess && in != Form::source) {
+    if (in == Form::any) sp.form_if = 0;
+    e = raw ? launch_pdl(d2::k2_phi<T, true>, np, st, k, sp) : launch_pdl(d2::k2_phi<T, false>, np, st, k, sp);
+  }
   if (e != cudaSuccess) return e;
   if (mid) {
     e = cudaEventRecord(mid, st);
@@ -1066,7 +1077,7 @@ cudaError_t launch_inject2d(const Consts<T>& k, const State<T, T>& s, bool raw, 
                                                cudaStream_t);                                                       \
   template cudaError_t launch_init2d<T, double>(const Consts<T>&, const State<T, T>&, const double*, const double*, \
                                                 cudaStream_t);                                                      \
-  template cudaError_t launch_step2d<T>(const Consts<T>&, const State<T, T>&, bool, bool, bool, bool, double,       \
+  template cudaError_t launch_step2d<T>(const Consts<T>&, const State<T, T>&, bool, bool, Form, bool, double,       \
                                         cudaStream_t, cudaEvent_t);                                                 \
   template cudaError_t launch_expand2d<T>(const Consts<T>&, const State<T, T>&, double, cudaStream_t);              \
   template cudaError_t launch_observe2d<T>(const Consts<T>&, const State<T, T>&, bool, unsigned, int, T*, T*, T*,   \

@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(kPhisNT, 2) k_phis_one(const __grid_constant__
   extern __shared__ __align__(16) float2 phis_sm[];
   pdl_trigger();
   pdl_wait();  // S and u of the previous update kernel
+  if (other_form(d.s)) return;
   phis_block<S>(d.k, d.s, d.tile, blockIdx.x, gridDim.x, phis_sm);
 }
 
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kPhisNT, 2) k_phis_batch(const CaseDesc<T, S>*
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock) k_expand(Consts<T> k, State<T, S> s) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
-  if (n >= k.N) return;
+  if (n >= k.N || other_form(s)) return;
   using IO = PopIO<T, S>;
   const size_t Np = (size_t)k.Np;
   const T* src = reinterpret_cast<const T*>(s.fin);

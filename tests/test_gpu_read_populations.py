@@ -70,6 +70,7 @@ def test_reading_f_on_another_stream_beside_a_step(grid, dtype):
         reads = []
         for st in side:
             st.wait_stream(torch.cuda.current_stream())
+            a._cache.clear()  # each stream makes its own read
             with torch.cuda.stream(st):
                 reads.append(a.f)
         a.run(1)  # not ordered after the reads by this program
