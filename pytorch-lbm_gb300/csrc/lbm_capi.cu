@@ -651,6 +651,9 @@ bool omega1_of(const LbmHandle* h) {
 int64_t units_of(const LbmHandle* h) { return h->paired ? h->N / 2 : h->N; }
 // per_thread counts nodes (a thread of the paired kernel takes per_thread / 2 pairs).
 // A grid alone that would not fill the device (608 resident blocks) at that many takes fewer.
+// A float64 grid is split alike in a batch and by its own per_thread
+// (LbmBatch::phin): its sum of phi is rounded per block, and a batch gives the
+// same bits as its cases alone.  (Float sums are exact fixed point.)
 int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
   if (alone) per_thread = (int)std::max<int64_t>(1, std::min<int64_t>(per_thread, (h->N + 608 * kBlock - 1) / (608 * kBlock)));
   const long long per = (long long)kBlock * (h->paired ? std::max(1, per_thread / 2) : per_thread);
@@ -1921,6 +1924,8 @@ struct LbmBatch {
   // with omega_f == 1, 1 linear other, 2 paired layout with omega_f == 1, 3 paired other
   int gstart[5] = {0, 0, 0, 0, 0};
   int phi_per_thread = 16;  // nodes per phi-kernel thread (half as many pairs in the paired layout)
+  std::vector<int> phin;    // phi blocks of each case
+  std::vector<int> per64;   // float64: each case's own phi_per_thread, which they follow
   int upd_block = 128;      // threads per block of the linear-layout update kernel
   bool coop = false;        // one cooperative launch per step (k_batch_coop) instead of two launches
   size_t desc = 0;          // bytes of one case descriptor
@@ -1955,8 +1960,14 @@ int batch_layout(LbmBatch* b) {
   b->b2c = nullptr;
   const int n = (int)b->h.size();
   long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0, pb_om1 = 0;
+  b->phin.assign(n, 0);
+  b->per64.clear();
   for (int i = 0; i < n; ++i) {
-    const int phin = phi_blocks_of(b->h[i], b->phi_per_thread), g = launch_group(b->h[i]);
+    const bool f64 = b->prec == LBM_F64;
+    if (f64) b->per64.push_back(b->h[i]->phi_per_thread);
+    const int phin = b->phin[i] = f64 ? phi_blocks_of(b->h[i], b->h[i]->phi_per_thread, true)
+                                      : phi_blocks_of(b->h[i], b->phi_per_thread);
+    const int g = launch_group(b->h[i]);
     pb[b->h[i]->paired ? 1 : 0] += phin;
     ub[g] += upd_blocks_of(b->h[i], b->upd_block);
     if (g == 0) pb_om1 += phin;
@@ -1976,7 +1987,7 @@ int batch_layout(LbmBatch* b) {
   for (int g = 0; g < 4; ++g) at[3 + g] = at[2 + g] + (size_t)ub[g];
   for (int i = 0; i < n; ++i) {
     size_t& a = at[b->h[i]->paired ? 1 : 0];
-    for (int k = phi_blocks_of(b->h[i], b->phi_per_thread); k > 0; --k) t[a++] = (unsigned short)i;
+    for (int k = b->phin[i]; k > 0; --k) t[a++] = (unsigned short)i;
     size_t& c = at[2 + launch_group(b->h[i])];
     for (int k = upd_blocks_of(b->h[i], b->upd_block); k > 0; --k) t[c++] = (unsigned short)i;
     if (wants_s(b->h[i]))
@@ -1995,7 +2006,7 @@ void batch_fill_t(LbmBatch* b) {
   for (int i = 0; i < n; ++i) {
     LbmHandle* h = b->h[i];
     const PhiTile tile = wants_s(h) ? phis_tile(h, n) : PhiTile{};
-    const int phin = phi_blocks_of(h, b->phi_per_thread), updn = upd_blocks_of(h, b->upd_block),
+    const int phin = b->phin[i], updn = upd_blocks_of(h, b->upd_block),
               g = launch_group(h);
     int& pbl = pb[h->paired ? 1 : 0];
     for (int par = 0; par < 2; ++par) {
@@ -2282,6 +2293,12 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
     if (!h->initialized) return fail(LBM_E_STATE, "lbm_batch_step: a case is not initialised");
     any_first |= h->raw || h->first;
   }
+  for (size_t i = 0; i < b->per64.size(); ++i)
+    if (b->per64[i] != b->h[i]->phi_per_thread) {
+      const int rc = batch_layout(b);
+      if (rc != LBM_OK) return rc;
+      break;
+    }
   int rest = nsteps;
   if (any_first && rest > 0) {
     // a case in its first step after init reads its populations in place:
