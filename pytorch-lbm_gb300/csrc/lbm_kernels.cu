@@ -2269,20 +2269,20 @@ cudaError_t launch_expand(const Consts<T>& k, const State<T, S>& s, cudaStream_t
 // (float compute only: float64 grids keep the linear layout)
 template <typename T, typename S>
 cudaError_t launch_phi_pair(const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
+  if (blocks <= 0) return cudaSuccess;
   if constexpr (sizeof(T) == 8) {
     return cudaErrorNotSupported;
   } else {
-    if (blocks <= 0) return cudaSuccess;
     return launch_pdl(k_phi_pair<T, S>, blocks, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
   }
 }
 template <typename T, typename S>
 cudaError_t launch_update_pair(const void* cases, const unsigned short* b2c, int blocks, bool omega1,
                                cudaStream_t st, bool gmu) {
+  if (blocks <= 0) return cudaSuccess;
   if constexpr (sizeof(T) == 8) {
     return cudaErrorNotSupported;
   } else {
-    if (blocks <= 0) return cudaSuccess;
     auto c = static_cast<const CaseDesc<T, S>*>(cases);
     constexpr int bs = kPairUpdBlock;
     if (gmu) {

@@ -16,7 +16,7 @@ def _lib(built_lib):
         pytest.fail("GPU tests need a CUDA device")
 
 
-@pytest.mark.parametrize("coop", [True])
+@pytest.mark.parametrize("coop", [True, False])
 def test_float64_batch_matches_cases_alone(coop):
     from lbm.batch import AllenCahnBatch
     alone, mixed = _sets(GRIDS, torch.float64)
