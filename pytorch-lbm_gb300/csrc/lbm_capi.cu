@@ -650,13 +650,18 @@ bool omega1_of(const LbmHandle* h) {
 // (Pairs of nodes in the paired layout.)
 int64_t units_of(const LbmHandle* h) { return h->paired ? h->N / 2 : h->N; }
 // per_thread counts nodes (a thread of the paired kernel takes per_thread / 2 pairs).
-// A grid alone that would not fill the device (608 resident blocks) at that many takes fewer.
+// A grid alone that would not fill the device at that many takes fewer: one wave
+// of resident blocks, 608 of the linear kernel and 456 of the paired one (80
+// registers), whose second wave at 608 would be nearly empty (128x128x96 float:
+// 110 us a step at 384 blocks, 115 at 615; 32^3: 20 us at one wave of 16 nodes
+// per thread, 13 at one node).
 // A float64 grid is split alike in a batch and by its own per_thread
 // (LbmBatch::phin): its sum of phi is rounded per block, and a batch gives the
 // same bits as its cases alone.  (Float sums are exact fixed point.)
 int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
-  if (alone) per_thread = (int)std::max<int64_t>(1, std::min<int64_t>(per_thread, (h->N + 608 * kBlock - 1) / (608 * kBlock)));
-  const long long per = (long long)kBlock * (h->paired ? std::max(1, per_thread / 2) : per_thread);
+  const int64_t wave = (h->paired ? 456 : 608) * (int64_t)kBlock;
+  if (alone) per_thread = (int)std::max<int64_t>(1, std::min<int64_t>(per_thread, (h->N + wave - 1) / wave));
+  const long long per = (long long)kBlock * (h->paired ? (alone ? (per_thread + 1) / 2 : std::max(1, per_thread / 2)) : per_thread);
   return (int)std::max<long long>(1, (units_of(h) + per - 1) / per);
 }
 
