@@ -45,7 +45,7 @@ cudaError_t launch_momentum(int, const T*, const T*, int, int, double, double, d
 template <typename T>
 cudaError_t launch_measure_static(int, int, int, const T*, const uint8_t*, double*, cudaStream_t);
 template <typename T, typename S>
-cudaError_t launch_phi_batch(const void*, const unsigned short*, int, int, cudaStream_t);
+cudaError_t launch_phi_batch(const void*, const unsigned short*, int, cudaStream_t);
 template <typename T, typename S>
 cudaError_t launch_update_batch(const void*, const unsigned short*, int, bool, bool, cudaStream_t, int);
 template <typename T, typename S>
@@ -1938,12 +1938,11 @@ struct LbmBatch {
   unsigned char* staging = nullptr;     // pinned host copy of both tables
   cudaEvent_t staged = nullptr;         // the last copy out of `staging` has run
   // block -> case: the phi grids of the linear and the paired cases, the
-  // update grids of the four groups, then the source form's phi grid of the linear
-  // cases with omega_f == 1 (float compute)
+  // update grids of the four groups, then the source form's phi grid (src)
   unsigned short* b2c = nullptr;
   int phi_blocks[2] = {0, 0}, upd_blocks[4] = {0, 0, 0, 0}, phis_blocks = 0;
-  int phi_blocks_om1 = 0;               // linear phi blocks of the omega_f == 1 cases (the first of them)
   bool graph_s = false;                 // the graph's phi pass reads S
+  bool src = false;                     // the table kernels keep the cases in source form (table_src)
   cudaStream_t cap = nullptr;           // stream used to capture the two-step graph
   // large grids (batch_apart): each case steps through its own launches on one of these streams
   std::vector<cudaStream_t> lanes;
@@ -1957,6 +1956,22 @@ namespace {
 
 int launch_group(const LbmHandle* h) { return (h->paired ? 2 : 0) + (omega1_of(h) ? 0 : 1); }
 
+// Whether the table kernels keep their cases in source form: where every case can
+// hold it (with others beside them a step has two phi passes instead of one:
+// 16 x 32^3, half of them at tau_h 0.57, 82 us a step against 67), except for many
+// small ones, whose tiles are halo for the most part, where together they fill the
+// device.  us per step, float (half), source form / populations:
+//   64 x 24^3 74 / 76 (78 / 79), 32 x 32^3 88 / 89 (93 / 92), 32 x 40^3 151 / 153 (157 / 161)
+//   128 x 24^3 147 / 138 (153 / 143), 64 x 32^3 165 / 162 (174 / 166)
+bool table_src(const LbmBatch* b) {
+  int64_t nodes = 0;
+  for (const LbmHandle* h : b->h) {
+    if (!wants_s(h)) return false;
+    nodes += h->N;
+  }
+  return nodes <= 1000000 || nodes > (int64_t)b->h.size() * 40000;
+}
+
 // Block -> case tables (device) for the current phi_per_thread; drops the graph.
 int batch_layout(LbmBatch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
@@ -1964,7 +1979,8 @@ int batch_layout(LbmBatch* b) {
   if (b->b2c) cudaFree(b->b2c);
   b->b2c = nullptr;
   const int n = (int)b->h.size();
-  long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0, pb_om1 = 0;
+  b->src = table_src(b);
+  long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0;
   b->phin.assign(n, 0);
   b->per64.clear();
   for (int i = 0; i < n; ++i) {
@@ -1975,15 +1991,13 @@ int batch_layout(LbmBatch* b) {
     const int g = launch_group(b->h[i]);
     pb[b->h[i]->paired ? 1 : 0] += phin;
     ub[g] += upd_blocks_of(b->h[i], b->upd_block);
-    if (g == 0) pb_om1 += phin;
-    if (wants_s(b->h[i])) jb += phis_tile(b->h[i], n).blocks();
+    if (b->src) jb += phis_tile(b->h[i], n).blocks();
   }
   const long long tot = pb[0] + pb[1] + ub[0] + ub[1] + ub[2] + ub[3] + jb;
   if (tot > 0x7fffffff) return fail(LBM_E_ARG, "lbm_batch: grids too large");
   for (int j = 0; j < 2; ++j) b->phi_blocks[j] = (int)pb[j];
   for (int g = 0; g < 4; ++g) b->upd_blocks[g] = (int)ub[g];
   b->phis_blocks = (int)jb;
-  b->phi_blocks_om1 = (int)pb_om1;
   std::vector<unsigned short> t((size_t)tot);
   size_t at[7];
   at[0] = 0;
@@ -1995,7 +2009,7 @@ int batch_layout(LbmBatch* b) {
     for (int k = b->phin[i]; k > 0; --k) t[a++] = (unsigned short)i;
     size_t& c = at[2 + launch_group(b->h[i])];
     for (int k = upd_blocks_of(b->h[i], b->upd_block); k > 0; --k) t[c++] = (unsigned short)i;
-    if (wants_s(b->h[i]))
+    if (b->src)
       for (int k = phis_tile(b->h[i], n).blocks(); k > 0; --k) t[at[6]++] = (unsigned short)i;
   }
   CUDA_TRY(cudaMalloc(&b->b2c, t.size() * sizeof(unsigned short)));
@@ -2010,7 +2024,7 @@ void batch_fill_t(LbmBatch* b) {
   int pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0;
   for (int i = 0; i < n; ++i) {
     LbmHandle* h = b->h[i];
-    const PhiTile tile = wants_s(h) ? phis_tile(h, n) : PhiTile{};
+    const PhiTile tile = b->src ? phis_tile(h, n) : PhiTile{};
     const int phin = b->phin[i], updn = upd_blocks_of(h, b->upd_block),
               g = launch_group(h);
     int& pbl = pb[h->paired ? 1 : 0];
@@ -2042,9 +2056,9 @@ int batch_fill(LbmBatch* b, cudaStream_t st) {
 }
 
 // One batched step reading descriptor table `par`: the phi kernels over every
-// linear-layout case (phis_in: the omega_f == 1 ones are in source
-// form and go through that form's kernel) and over every paired case, then the update kernel over each group
-// (layout x omega_f == 1 or not).  Empty launches are skipped.
+// linear-layout and every paired case (phis_in: the cases are in source form, whose
+// phi kernel runs over all of them), then the update kernel over each group (layout x
+// omega_f == 1 or not).  Empty launches are skipped.
 template <typename T, typename S>
 cudaError_t batch_launch_t(LbmBatch* b, int par, bool phis_in, cudaStream_t st) {
   const void* tab = b->table[par];
@@ -2053,14 +2067,15 @@ cudaError_t batch_launch_t(LbmBatch* b, int par, bool phis_in, cudaStream_t st) 
   const unsigned short* t = b->b2c;
   const unsigned short* upd = t + b->phi_blocks[0] + b->phi_blocks[1];
   const unsigned short* tj = upd + b->upd_blocks[0] + b->upd_blocks[1] + b->upd_blocks[2] + b->upd_blocks[3];
-  const bool j = b->phis_blocks > 0;
-  const int skip = j && phis_in ? b->phi_blocks_om1 : 0;  // the omega_f == 1 cases come first
   cudaError_t e = cudaSuccess;
-  if (j && phis_in) e = launch_phis_batch<T, S>(tab, tj, b->phis_blocks, st);
-  if (e == cudaSuccess) e = launch_phi_batch<T, S>(tab, t, skip, b->phi_blocks[0] - skip, st);
-  if (e == cudaSuccess) e = launch_phi_pair<T, S>(tab, t + b->phi_blocks[0], b->phi_blocks[1], st);
+  if (phis_in) {
+    e = launch_phis_batch<T, S>(tab, tj, b->phis_blocks, st);
+  } else {
+    e = launch_phi_batch<T, S>(tab, t, b->phi_blocks[0], st);
+    if (e == cudaSuccess) e = launch_phi_pair<T, S>(tab, t + b->phi_blocks[0], b->phi_blocks[1], st);
+  }
   for (int g = 0; g < 4 && e == cudaSuccess; ++g) {
-    e = g < 2 ? launch_update_batch<T, S>(tab, upd, b->upd_blocks[g], g == 0, j, st, b->upd_block)
+    e = g < 2 ? launch_update_batch<T, S>(tab, upd, b->upd_blocks[g], g == 0, b->src, st, b->upd_block)
               : launch_update_pair<T, S>(tab, upd, b->upd_blocks[g], g == 2, st, false);
     upd += b->upd_blocks[g];
   }
@@ -2072,12 +2087,11 @@ cudaError_t batch_launch(LbmBatch* b, int par, bool phis_in, cudaStream_t st) {
   });
 }
 
-// Makes the form of f the same for all cases that can hold S: true when all of
-// them do, else all hold populations (the cooperative step's form too).
+// Makes the form of f the same for all cases: true when all hold S and the table
+// kernels keep it, else all hold populations (the cooperative step's form too).
 int batch_form(LbmBatch* b, cudaStream_t st, bool* phis_in) {
-  bool all = !b->coop;
-  for (LbmHandle* h : b->h)
-    if (wants_s(h)) all = all && form_of(h) == Form::source;
+  bool all = b->src && !b->coop;
+  for (LbmHandle* h : b->h) all = all && form_of(h) == Form::source;
   if (!all)
     for (LbmHandle* h : b->h) {
       const int rc = ensure_populations(h, st);
@@ -2208,7 +2222,7 @@ void batch_advance(LbmBatch* b, int nsteps) {
       h->c_last ^= 1;
     }
     h->steps += nsteps;
-    if (nsteps > 0) h->sform = !b->coop && wants_s(h);
+    if (nsteps > 0) h->sform = b->src && !b->coop;
     h->form_set = h->form_set || h->sform;
     h->last_raw_in = false;
     h->obs_init = false;
@@ -2326,7 +2340,7 @@ int lbm_batch_step(LbmBatch* b, int nsteps, void* stream) {
   int rc = batch_form(b, st, &phis_in);
   if (rc == LBM_OK) rc = batch_fill(b, st);
   if (rc != LBM_OK) return rc;
-  if (!phis_in && !b->coop && b->phis_blocks > 0) {
+  if (!phis_in && !b->coop && b->src) {
     // from populations to S: one step, then the tables of the other parity
     CUDA_TRY(batch_launch(b, 0, false, st));
     batch_advance(b, 1);

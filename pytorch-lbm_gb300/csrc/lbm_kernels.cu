@@ -1560,13 +1560,12 @@ __device__ __forceinline__ void phi_block(const Consts<T>& k, const State<T, S>&
 
 template <typename T, typename S>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 3 : 4) k_phi_batch(
-    const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ blk2case, int blk0) {
-  // blk0: the first block of the table's phi part that this launch runs
+    const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ blk2case) {
   __shared__ CaseDesc<T, S> d;
-  load_desc(d, cases + blk2case[blk0 + blockIdx.x]);
+  load_desc(d, cases + blk2case[blockIdx.x]);
   pdl_trigger();
   pdl_wait();  // f of the previous update kernel
-  phi_block(d.k, d.s, blk0 + blockIdx.x - d.phi_blk0, d.phi_nblk);
+  phi_block(d.k, d.s, blockIdx.x - d.phi_blk0, d.phi_nblk);
 }
 
 // BS threads per block (the autotuners choose 128 or 256), compiled for the
@@ -1575,7 +1574,7 @@ template <typename T, typename S, bool OMEGA1, bool SOUT, int BS = kBlock>
 __global__ void __launch_bounds__(BS, UpdateOccupancy<T, S>::blocks * kBlock / BS) k_update_batch(
     const CaseDesc<T, S>* __restrict__ cases, const unsigned short* __restrict__ blk2case) {
   __shared__ CaseDesc<T, S> d;
-  load_desc(d, cases + (blk2case ? blk2case[blockIdx.x] : 0));
+  load_desc(d, cases + blk2case[blockIdx.x]);
   pdl_trigger();
   pdl_wait();  // phi of the phi kernel
   update_block<T, S, OMEGA1, false, SOUT, BS>(d.k, d.s, (blockIdx.x - d.upd_blk0) * BS);
@@ -2180,11 +2179,11 @@ cudaError_t launch_step(const Consts<T>& k, const State<T, S>& s, const Tiling& 
 }
 
 // Batched step kernels over a device case table; blocks: the grid (the part
-// of the block -> case table that starts at blk0).
+// of the block -> case table that starts at b2c).
 template <typename T, typename S>
-cudaError_t launch_phi_batch(const void* cases, const unsigned short* b2c, int blk0, int blocks, cudaStream_t st) {
+cudaError_t launch_phi_batch(const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
   if (blocks <= 0) return cudaSuccess;
-  return launch_pdl(k_phi_batch<T, S>, blocks, st, static_cast<const CaseDesc<T, S>*>(cases), b2c, blk0);
+  return launch_pdl(k_phi_batch<T, S>, blocks, st, static_cast<const CaseDesc<T, S>*>(cases), b2c);
 }
 // bs: threads per block of the update kernel, 256 or 128.  sout: S is stored in the place of f.
 template <typename T, typename S>
@@ -2528,7 +2527,7 @@ template cudaError_t launch_measure_static<double>(int, int, int, const double*,
 
 
 #define LBM_INSTANTIATE_BATCH(T, S)                                                                             \
-  template cudaError_t launch_phi_batch<T, S>(const void*, const unsigned short*, int, int, cudaStream_t);      \
+  template cudaError_t launch_phi_batch<T, S>(const void*, const unsigned short*, int, cudaStream_t);           \
   template cudaError_t launch_update_batch<T, S>(const void*, const unsigned short*, int, bool, bool,            \
                                                  cudaStream_t, int);                                             \
   template cudaError_t launch_phi_one<T, S>(const void*, cudaStream_t);                                         \
