@@ -676,13 +676,10 @@ bool wants_s(const LbmHandle* h) {
 }
 
 // Tiles of the source form's phi pass: the (y, z) split whose blocks (tile plus
-// halo within kPhisThreads nodes) waste the fewest threads, then the planes of
-// x per block (an even number: they are walked in pairs, two more at the ends)
-// that keep the device's slots busy for the shortest time, `share` cases
-// launched together sharing them.
+// halo within kPhisThreads nodes) waste the fewest threads.
 constexpr int kPhisThreads = 320, kPhisSlots = 304;  // two blocks per SM
-PhiTile phis_tile(const LbmHandle* h, int share) {
-  const int nx = (int)h->nx, ny = (int)h->ny, nz = (int)h->nz;
+PhiTile phis_split(const LbmHandle* h) {
+  const int ny = (int)h->ny, nz = (int)h->nz;
   PhiTile best{};
   double best_eff = -1.0;
   for (int ntz = 1; ntz <= nz; ++ntz) {
@@ -700,18 +697,38 @@ PhiTile phis_tile(const LbmHandle* h, int share) {
     }
     if (tz <= 8) break;
   }
-  const long long tiles = (long long)best.nty * best.ntz * std::max(1, share);
+  return best;
+}
+
+// The planes of x per block (an even number: they are walked in pairs, two more
+// at the ends) of n grids whose phi passes run in one launch: what keeps the
+// device's slots busy for the shortest time, over the blocks of all of them.
+// (Chosen for each grid as if all were of its size, a large grid among small ones
+// had a fraction of the blocks that fill the device.  us a step of table batches,
+// so / so chosen: 128^3 and 16 x 24^3 177 / 153, 96^3 and 10 x 32^3 106 / 86, 8 x 64^3
+// and 8 x 24^3 177 / 159.)
+void phis_planes(LbmHandle* const* h, int n, PhiTile* t) {
+  int most = 0;
+  for (int i = 0; i < n; ++i) {
+    t[i] = phis_split(h[i]);
+    most = std::max(most, (int)std::min<int64_t>(h[i]->nx + (h[i]->nx & 1), 64));
+  }
+  auto planes = [&](int i, int cx) { return (int)std::min<int64_t>(cx, h[i]->nx + (h[i]->nx & 1)); };
   long long best_cost = -1;
-  for (int cx = 2; cx <= std::min(nx + (nx & 1), 64); cx += 2) {
-    const int ncx = (nx + cx - 1) / cx;
-    const long long cost = (tiles * ncx + kPhisSlots - 1) / kPhisSlots * (cx + 2);
+  int best = 2;
+  for (int cx = 2; cx <= most; cx += 2) {
+    long long blocks = 0;
+    for (int i = 0; i < n; ++i) blocks += (long long)t[i].nty * t[i].ntz * ((h[i]->nx + planes(i, cx) - 1) / planes(i, cx));
+    const long long cost = (blocks + kPhisSlots - 1) / kPhisSlots * (cx + 2);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
-      best.cx = cx;
-      best.ncx = ncx;
+      best = cx;
     }
   }
-  return best;
+  for (int i = 0; i < n; ++i) {
+    t[i].cx = planes(i, best);
+    t[i].ncx = (int)((h[i]->nx + t[i].cx - 1) / t[i].cx);
+  }
 }
 
 // upd_block: threads per block of the linear-layout update kernel (the
@@ -981,7 +998,7 @@ int lbm_create(const LbmParams* params, int64_t nx, int64_t ny, int64_t nz, int 
   cudaGetDevice(&h->device);
   const size_t T = h->tsize;
   h->tiling = make_tiling(nx, ny, nz, 0, 0, 0, precision);
-  if (nz > 1) h->tile = phis_tile(h, 1);
+  if (nz > 1) phis_planes(&h, 1, &h->tile);
   const Sizes z = sizes_of(nx, ny, nz, precision);
   cudaError_t e = cudaSuccess;
   auto A = [&](void** p, size_t bytes) {
@@ -1943,6 +1960,7 @@ struct LbmBatch {
   int phi_blocks[2] = {0, 0}, upd_blocks[4] = {0, 0, 0, 0}, phis_blocks = 0;
   bool graph_s = false;                 // the graph's phi pass reads S
   bool src = false;                     // the table kernels keep the cases in source form (table_src)
+  std::vector<PhiTile> tiles;           // src: of each case
   cudaStream_t cap = nullptr;           // stream used to capture the two-step graph
   // large grids (batch_apart): each case steps through its own launches on one of these streams
   std::vector<cudaStream_t> lanes;
@@ -1980,6 +1998,8 @@ int batch_layout(LbmBatch* b) {
   b->b2c = nullptr;
   const int n = (int)b->h.size();
   b->src = table_src(b);
+  b->tiles.assign(n, PhiTile{});
+  if (b->src) phis_planes(b->h.data(), n, b->tiles.data());
   long long pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0;
   b->phin.assign(n, 0);
   b->per64.clear();
@@ -1991,7 +2011,7 @@ int batch_layout(LbmBatch* b) {
     const int g = launch_group(b->h[i]);
     pb[b->h[i]->paired ? 1 : 0] += phin;
     ub[g] += upd_blocks_of(b->h[i], b->upd_block);
-    if (b->src) jb += phis_tile(b->h[i], n).blocks();
+    jb += b->tiles[i].blocks();
   }
   const long long tot = pb[0] + pb[1] + ub[0] + ub[1] + ub[2] + ub[3] + jb;
   if (tot > 0x7fffffff) return fail(LBM_E_ARG, "lbm_batch: grids too large");
@@ -2009,8 +2029,7 @@ int batch_layout(LbmBatch* b) {
     for (int k = b->phin[i]; k > 0; --k) t[a++] = (unsigned short)i;
     size_t& c = at[2 + launch_group(b->h[i])];
     for (int k = upd_blocks_of(b->h[i], b->upd_block); k > 0; --k) t[c++] = (unsigned short)i;
-    if (b->src)
-      for (int k = phis_tile(b->h[i], n).blocks(); k > 0; --k) t[at[6]++] = (unsigned short)i;
+    for (int k = b->tiles[i].blocks(); k > 0; --k) t[at[6]++] = (unsigned short)i;
   }
   CUDA_TRY(cudaMalloc(&b->b2c, t.size() * sizeof(unsigned short)));
   CUDA_TRY(cudaMemcpy(b->b2c, t.data(), t.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
@@ -2024,7 +2043,7 @@ void batch_fill_t(LbmBatch* b) {
   int pb[2] = {0, 0}, ub[4] = {0, 0, 0, 0}, jb = 0;
   for (int i = 0; i < n; ++i) {
     LbmHandle* h = b->h[i];
-    const PhiTile tile = b->src ? phis_tile(h, n) : PhiTile{};
+    const PhiTile& tile = b->tiles[i];
     const int phin = b->phin[i], updn = upd_blocks_of(h, b->upd_block),
               g = launch_group(h);
     int& pbl = pb[h->paired ? 1 : 0];
