@@ -1978,16 +1978,19 @@ int launch_group(const LbmHandle* h) { return (h->paired ? 2 : 0) + (omega1_of(h
 // hold it (with others beside them a step has two phi passes instead of one:
 // 16 x 32^3, half of them at tau_h 0.57, 82 us a step against 67), except for many
 // small ones, whose tiles are halo for the most part, where together they fill the
-// device.  us per step, float (half), source form / populations:
-//   64 x 24^3 74 / 76 (78 / 79), 32 x 32^3 88 / 89 (93 / 92), 32 x 40^3 151 / 153 (157 / 161)
-//   128 x 24^3 147 / 138 (153 / 143), 64 x 32^3 165 / 162 (174 / 166)
+// device; float ones only as long as their populations stay in L2 between the
+// kernels.  us per step, float (half), source form / populations:
+//   64 x 24^3 74 / 76 (78 / 79), 32 x 32^3 87 / 88 (92 / 90), 32 x 40^3 151 / 153 (157 / 161)
+//   128 x 24^3 146 / 139 (152 / 140), 64 x 32^3 165 / 160 (173 / 161)
+//   256 x 24^3 277 / 287 (290 / 274), 128 x 32^3 329 / 335 (340 / 314)
 bool table_src(const LbmBatch* b) {
   int64_t nodes = 0;
   for (const LbmHandle* h : b->h) {
     if (!wants_s(h)) return false;
     nodes += h->N;
   }
-  return nodes <= 1000000 || nodes > (int64_t)b->h.size() * 40000;
+  if (nodes > (int64_t)b->h.size() * 40000) return true;
+  return nodes <= 1000000 || (b->prec == LBM_F32 && nodes > 3000000);
 }
 
 // Block -> case tables (device) for the current phi_per_thread; drops the graph.
