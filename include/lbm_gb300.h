@@ -379,8 +379,8 @@ int lbm_footprint(int64_t nx, int64_t ny, int64_t nz, int precision, int64_t* by
  * Batches: many independent grids (handles) that advance together, one launch
  * of each step kernel per time step for all of them (a block finds its case
  * in a block -> case table), replayed from a captured two-step CUDA graph.
- * Cases of a mean of about 48^3 nodes and more (float or half storage, linear
- * layout) go through their own launches on a few streams of the batch instead,
+ * Cases of a mean of about 48^3 nodes and more, none below about 40^3 (float or
+ * half storage, linear layout), go through their own launches on a few streams of the batch instead,
  * ordered after the work of the caller's stream and before what follows there.
  * Each case's arithmetic and reductions are its own, so its results are
  * bit-identical to stepping it alone.  The handles stay usable on their own

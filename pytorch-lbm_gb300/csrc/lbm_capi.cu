@@ -2149,20 +2149,24 @@ int batch_graph(LbmBatch* b, bool phis_in) {
 // constants and pointers as constant-bank operands instead of a shared-memory
 // descriptor, and one case's phi pass (bound by its instructions) runs beside
 // another's update (bound by memory); but each case costs two launches a step.
-// us per step of a batch, table kernels / 1, 2, 4, 8 streams:
-//   8 x 48^3      float 75 / 141, 83, 75, 73      half  88 / 162, 92, 81, 80
-//   8 x 80x80x64  float 245 / 309, 217, 212, 216  half 266 / 355, 242, 223, 224
-//   6 x 128x128x96 float 634 / 614, 552, 562, 571 half 661 / 663, 556, 561, 563
-//   2 x 192x192x128 float 597 / 551, 532          half 611 / 539, 502
-// Below a mean of 48^3 nodes the launches bound it.  (Linear layouts in 32-bit
-// compute; the cooperative form is one launch by request.)
-constexpr int64_t kApartNodes = 110000;
+// us per step of a batch, float (half), table kernels / 4 streams:
+//   8 x 47^3 67 / 67 (72 / 71), 8 x 64^3 144 / 139 (148 / 144), 4 x 96^3 239 / 209 (246 / 204)
+//   128^3 and 4 x 40^3 156 / 150, 96^3 and 6 x 40^3 89 / 86, 192^3 and 10 x 40^3 486 / 464 (490 / 434)
+//   128^3 and 12 x 32^3 173 / 182, 96^3 and 10 x 32^3 86 / 110, 128^3 and 16 x 24^3 153 / 201 (162 / 202),
+//   2 x 128^3 and 30 x 24^3 309 / 434 (322 / 432), 192^3 and 40 x 24^3 469 / 601 (470 / 577)
+// (1, 2, 8 streams when they were chosen: 8 x 48^3 141, 83, 73 against 75 on 4.)
+// Below a mean of 48^3 nodes the launches bound it, and a small case beside large
+// ones waits with each of its launches for their blocks: every case has to be of
+// some size.  (Linear layouts in 32-bit compute; the cooperative form is one
+// launch by request.)
+constexpr int64_t kApartNodes = 110000;      // mean
+constexpr int64_t kApartSmallest = 60000;
 constexpr int kApartLanes = 4;
 bool batch_apart(const LbmBatch* b) {
   if (b->coop || b->prec == LBM_F64) return false;
   int64_t nodes = 0;
   for (const LbmHandle* h : b->h) {
-    if (h->paired) return false;
+    if (h->paired || h->N < kApartSmallest) return false;
     nodes += h->N;
   }
   return nodes >= (int64_t)b->h.size() * kApartNodes;

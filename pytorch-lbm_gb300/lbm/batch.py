@@ -3,9 +3,10 @@
 ``AllenCahnBatch(solvers)`` advances many ``AllenCahnSolver`` cases together:
 each time step is one launch of each step kernel for all cases (the blocks
 of one launch are spread over the cases by a block -> case table on the
-device), replayed from a captured two-step CUDA graph; cases of about 48^3
-nodes and more go through their own launches on a few streams instead, where
-one case's phi pass runs beside another's update.  Every case keeps its
+device), replayed from a captured two-step CUDA graph; cases of a mean of
+about 48^3 nodes and more, none below about 40^3, go through their own launches
+on a few streams instead, where one case's phi pass runs beside another's
+update.  Every case keeps its
 own arithmetic, reductions and mass correction, so its fields are
 bit-identical to stepping it alone; the solvers remain usable on their own
 between batch calls (fields, ``measure()``).

@@ -25,6 +25,7 @@ SETS = {
     "tau alone": ([(24, 24, 20), (30, 25, 33)], [0.57, 0.6]),
     "many small": ([(32, 32, 32)] * 31, [None] * 31),  # 1.02e6 nodes of a mean below 40,000
     "very many small": ([(32, 32, 32)] * 92, [None] * 92),  # 3.01e6: float in source form again
+    "one too small": ([(96, 96, 64), (96, 64, 64), (24, 24, 24)], [None] * 3),  # of a mean for the streams
     "sizes apart": ([(96, 64, 32), (24, 24, 24), (17, 40, 21)], [None] * 3),
 }
 
