@@ -668,11 +668,16 @@ int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
 // Whether the two-kernel step of a grid leaves f in source form: tau_f == 1, float
 // compute, linear layout.  (float64 keeps the populations: its step is bound by
 // the float64 pipe, and the source form evaluates f again on each tile's halo.)
-// 2-D: not in the gradient-of-mu modes, whose update re-reads f, and not below
-// 32 columns, where a block's window would be mostly its two ends.
+// 2-D: not in the gradient-of-mu modes, whose update re-reads f, not where the
+// populations stay in L2 between the kernels and the phi pass is bound by latency,
+// and not below 256 columns, where its blocks have too few threads for one
+// barrier a row.  us per step, source form / populations:
+//   256x256 14.2 / 10.1, 512x512 18.8 / 16.9, 640x1024 27.8 / 27.2, 2800x256 30.2 / 30.8,
+//   896x896 31.8 / 33.4, 1536x1024 56.7 / 62.6, 2048x2048 129 / 150, 4x262144 38.9 / 40.3
+//   4096x192 34.6 / 33.4, 16384x128 92 / 87, 16384x64 55 / 47
 bool wants_s(const LbmHandle* h) {
   if (h->prec == LBM_F64 || h->paired || !omega1_of(h)) return false;
-  return h->nz > 1 || (!h->mu && h->ny >= 32);
+  return h->nz > 1 || (!h->mu && h->ny >= 256 && h->N >= 700000);
 }
 
 // Tiles of the source form's phi pass: the (y, z) split whose blocks (tile plus
