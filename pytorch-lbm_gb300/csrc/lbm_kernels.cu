@@ -1888,10 +1888,9 @@ __global__ void __launch_bounds__(kBlock) k_observe(Consts<T> k, State<T, S> s, 
 }
 
 // Current populations in the reference layout: s.fin/s.gin hold the last
-// step's output, s.phi_in that step's phi and s.c_prev its correction.  SRC:
-// s.fin holds S; the 19 pulled values are evaluated from their nodes' phi, u
-// and S, so that a read-out writes nothing of the state.
-template <typename T, typename S, bool RAW, bool SRC = false>
+// step's output, s.phi_in that step's phi and s.c_prev its correction.  (f of a
+// state in source form: k_read_source.)
+template <typename T, typename S, bool RAW>
 __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N || other_form(s)) return;
@@ -1903,8 +1902,7 @@ __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S>
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q];
   if (f_o) {
-    if constexpr (SRC) fetch_f_source<S>(v, k, s, n, nb, c, eps);
-    else fetch_f<T, S, RAW, false, true>(v, k, s, n, N, nb, c, eps);
+    fetch_f<T, S, RAW, false, true>(v, k, s, n, N, nb, c, eps);
 #pragma unroll
     for (int q = 0; q < Q; ++q) f_o[(size_t)q * N + n] = v[q];
   }
@@ -2404,8 +2402,13 @@ cudaError_t launch_populations(const Consts<T>& k, const State<T, S>& s, bool ra
     if constexpr (sizeof(T) == 8) {
       return cudaErrorNotSupported;
     } else {
-      k_populations<T, S, false, true><<<grid, kBlock, 0, st>>>(k, s, f, g);
-      return cudaGetLastError();
+      if (k.N < kReadOne) {
+        k_read_source<T, S, true><<<special_blocks(k.N) + grid, kBlock, 0, st>>>(k, s, f, g);
+        return cudaGetLastError();
+      }
+      k_read_source<T, S, false><<<grid, kBlock, 0, st>>>(k, s, f, g);
+      const cudaError_t e = cudaGetLastError();
+      return e == cudaSuccess ? launch_pdl(k_read_special<T, S>, special_blocks(k.N), st, k, s, f) : e;
     }
   }
   if (raw) k_populations<T, S, true><<<grid, kBlock, 0, st>>>(k, s, f, g);

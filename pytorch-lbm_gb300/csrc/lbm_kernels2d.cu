@@ -820,8 +820,8 @@ __global__ void __launch_bounds__(kBlock) k2_observe(Consts<T> k, State<T, T> s,
   }
 }
 
-// fetch_f9 of a state in source form (s.fin holds S): each slot that node n
-// reads, evaluated at the slot's node.
+// fetch_f9 of a fluid node of a state in source form (s.fin holds S): each slot
+// that node n reads, evaluated at the slot's node.
 template <typename T>
 __device__ __forceinline__ void fetch_f9_source(T (&v)[Q9], const Consts<T>& k, const State<T, T>& s, int n, const Nb2& nb,
                                                 uint8_t c, T eps, T acT) {
@@ -835,17 +835,93 @@ __device__ __forceinline__ void fetch_f9_source(T (&v)[Q9], const Consts<T>& k, 
 #pragma unroll
   for (int q = 0; q < Q9; ++q) {
     const int m = nb.at(n, -ex(q), -ey(q));
-    if (c & kSolid) v[q] = slot(opp(q), n);
-    else if (c & kPartial) v[q] = one_m * slot(q, m) + eps * slot(opp(q), n);
-    else v[q] = slot(q, m);
+    v[q] = slot(q, m);
+    if (c & kPartial) v[q] = one_m * v[q] + eps * slot(opp(q), n);
     v[q] = v[q] * corr;
   }
   relax9(v, k, s, n, c, corr);
 }
 
-// Current populations in the reference layout [9][N].  SRC: s.fin holds S.
-template <typename T, bool RAW, bool SRC = false>
-__global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T> s, double ac, T* f_o, T* g_o) {
+// Whether node n of class c does more than pull its f: solid and partial nodes, and
+// top-surface ones whose corrected phi lies in the boundary-phi relaxation's range.
+template <typename T>
+__device__ __forceinline__ bool special_reader(const Consts<T>& k, const State<T, T>& s, int n, uint8_t c, T corr) {
+  if (c & (kSolid | kPartial)) return true;
+  if (!(k.relax_on && (c & kTop))) return false;
+  const T pb = clamp01(s.phi_in[n] * corr);
+  return pb > T(0.15) && pb < T(0.85);
+}
+
+// f and g (may be null) of a state in source form, in two kernels.
+// k2_read_source: a thread evaluates its node's f and writes each value, corrected,
+// to the slot of the node that pulls it, and pulls its g.  k2_read_special makes f of the
+// special readers, over what the first wrote there: each block collects those of
+// kSpecialRun nodes, and does all but its stores before the first kernel has ended.
+constexpr int kSpecialRun = 8 * kBlock;
+
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k2_read_source(Consts<T> k, State<T, T> s, double ac, T* f_o, T* g_o) {
+  pdl_trigger();
+  const int n = blockIdx.x * kBlock + threadIdx.x;
+  if (n >= k.N || other_form(s)) return;
+  const Nb2 nb = make_nb2(k, n);
+  const T corr = s.cbuf[s.c_prev];
+  T f[Q9];
+  f_of_source<T>(s.phi_in[n], s.u[n], s.u[k.Np + n], s.fin[n], s.fin[k.Np + n], (T)ac, f);
+#pragma unroll
+  for (int q = 0; q < Q9; ++q) f_o[q * k.N + nb.at(n, ex(q), ey(q))] = f[q] * corr;
+  if (g_o) {
+    const uint8_t c = s.cls[n];
+    fetch9<T, false>(f, s.gin, k.Np, n, nb, c, (c & kPartial) ? s.eps[n] : T(0), T(1));
+#pragma unroll
+    for (int q = 0; q < Q9; ++q) g_o[q * k.N + n] = f[q];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k2_read_special(Consts<T> k, State<T, T> s, double ac, T* f_o) {
+  __shared__ unsigned short list[kSpecialRun];
+  __shared__ int count;
+  const int n0 = blockIdx.x * kSpecialRun, i0 = 8 * threadIdx.x;
+  const T corr = s.cbuf[s.c_prev];
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  // eight classes per thread in one load (the array is padded with zeros to a multiple of 32)
+  if (n0 + i0 < k.N && !other_form(s)) {
+    const uint2 w = *reinterpret_cast<const uint2*>(s.cls + n0 + i0);
+    for (int i = 0; i < 8; ++i) {
+      const uint8_t c = (uint8_t)((i < 4 ? w.x : w.y) >> (8 * (i & 3)));
+      if (n0 + i0 + i < k.N && special_reader(k, s, n0 + i0 + i, c, corr))
+        list[atomicAdd(&count, 1)] = (unsigned short)(i0 + i);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < count || i < kBlock; i += kBlock) {
+    T v[Q9], f[Q9];
+    int n = 0;
+    if (i < count) {
+      n = n0 + list[i];
+      const uint8_t c = s.cls[n];
+      if (c & kSolid) {
+        // the node's own opposite slots
+        f_of_source<T>(s.phi_in[n], s.u[n], s.u[k.Np + n], s.fin[n], s.fin[k.Np + n], (T)ac, f);
+#pragma unroll
+        for (int q = 0; q < Q9; ++q) v[opp(q)] = f[q] * corr;
+      } else {
+        fetch_f9_source<T>(v, k, s, n, make_nb2(k, n), c, (c & kPartial) ? s.eps[n] : T(0), (T)ac);
+      }
+    }
+    if (i < kBlock) pdl_wait();  // all threads of the block, once
+    if (i < count) {
+#pragma unroll
+      for (int q = 0; q < Q9; ++q) f_o[q * k.N + n] = v[q];
+    }
+  }
+}
+
+// Current populations in the reference layout [9][N].
+template <typename T, bool RAW>
+__global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T> s, T* f_o, T* g_o) {
   const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N || other_form(s)) return;
   const uint8_t c = s.cls[n];
@@ -853,8 +929,7 @@ __global__ void __launch_bounds__(kBlock) k2_populations(Consts<T> k, State<T, T
   const T eps = (c & kPartial) ? s.eps[n] : T(0);
   T v[Q9];
   if (f_o) {
-    if constexpr (SRC) fetch_f9_source<T>(v, k, s, n, nb, c, eps, (T)ac);
-    else fetch_f9<T, RAW>(v, k, s, n, nb, c, eps);
+    fetch_f9<T, RAW>(v, k, s, n, nb, c, eps);
 #pragma unroll
     for (int q = 0; q < Q9; ++q) f_o[q * k.N + n] = v[q];
   }
@@ -1057,9 +1132,16 @@ template <typename T>
 cudaError_t launch_populations2d(const Consts<T>& k, const State<T, T>& s, bool raw, bool src, double ac, T* f, T* g,
                                  cudaStream_t st) {
   const int nb = d2::blocks_of(k.N);
-  if (src) d2::k2_populations<T, false, true><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
-  else if (raw) d2::k2_populations<T, true><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
-  else d2::k2_populations<T, false><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
+  if (src) {
+    d2::k2_read_source<T><<<nb, kBlock, 0, st>>>(k, s, ac, f, g);
+    const cudaError_t e = cudaGetLastError();
+    const int special = (k.N + d2::kSpecialRun - 1) / d2::kSpecialRun;
+    return e == cudaSuccess ? launch_pdl(d2::k2_read_special<T>, special, st, k, s, ac, f) : e;
+  } else if (raw) {
+    d2::k2_populations<T, true><<<nb, kBlock, 0, st>>>(k, s, f, g);
+  } else {
+    d2::k2_populations<T, false><<<nb, kBlock, 0, st>>>(k, s, f, g);
+  }
   return cudaGetLastError();
 }
 

@@ -101,8 +101,8 @@ __device__ __forceinline__ void feval_all(const Consts<float>& k, float phi, con
   }
 }
 
-// fetch_f of a state in source form (s.fin holds S): the value of each slot
-// that node n reads, evaluated at the slot's node.  Linear layout.
+// fetch_f of a fluid node of a state in source form (s.fin holds S): the value of
+// each slot that node n reads, evaluated at the slot's node.  Linear layout.
 template <typename S>
 __device__ __forceinline__ void fetch_f_source(float (&v)[Q], const Consts<float>& k, const State<float, S>& s, int n,
                                                const Nbr& nb, uint8_t c, float eps) {
@@ -121,13 +121,9 @@ __device__ __forceinline__ void fetch_f_source(float (&v)[Q], const Consts<float
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const unsigned m = (unsigned)nb.at(n, -ex(q), -ey(q), -ez(q));
-    if (c & (kSolid | kPartial)) {
-      // the node's own opposite slot: its reader is x - e_q
-      const float o = slot(opp(q), (unsigned)n, DEV ? s.phi_in[m] : 0.0f);
-      v[q] = (c & kSolid) ? o : fma_(one_m, slot(q, m, ref_self), mul_rn(eps, o));
-    } else {
-      v[q] = slot(q, m, ref_self);
-    }
+    v[q] = slot(q, m, ref_self);
+    // blended with the node's own opposite slot, whose reader is x - e_q
+    if (c & kPartial) v[q] = fma_(one_m, v[q], mul_rn(eps, slot(opp(q), (unsigned)n, DEV ? s.phi_in[m] : 0.0f)));
     v[q] = mul_rn(v[q], corr);
   }
   relax_f<float, S, false>(v, k, s, n, c, corr);
@@ -308,6 +304,133 @@ __global__ void __launch_bounds__(kPhisNT, 2) k_phis_batch(const CaseDesc<T, S>*
   pdl_trigger();
   pdl_wait();
   phis_block<S>(d.k, d.s, d.tile, blockIdx.x - d.phs_blk0, d.tile.blocks(), phis_sm);
+}
+
+// Whether node n of class c does more than pull its f: solid and partial nodes, and
+// top-surface ones whose corrected phi lies in the boundary-phi relaxation's range.
+template <typename T, typename S>
+__device__ __forceinline__ bool special_reader(const Consts<T>& k, const State<T, S>& s, unsigned n, uint8_t c, T corr) {
+  if (c & (kSolid | kPartial)) return true;
+  if (!(k.relax_on && (c & kTop))) return false;
+  const T pb = clamp01(mul_rn(s.phi_in[n], corr));
+  return pb > T(0.15) && pb < T(0.85);
+}
+
+// f and g (may be null) of a state in source form as the reference holds them
+// between steps, without writing anything of the state.  A thread evaluates its
+// node's f once and writes each value, corrected, to the slot of the node that
+// pulls it, and pulls its g.  f of the special readers is made by blocks that each
+// collect those of kSpecialRun nodes (a wall puts one or two into most warps): below
+// kReadOne nodes the first special_blocks(N) of the launch, and a node's class is
+// looked up before a value is written to it; above (the lookup of 18 classes per node costs
+// 35 us at 128x128x96) a second kernel, over what the first wrote there, which does all
+// but its stores before the first has ended.
+// us for f and g, float (half): 128x128x96 85 (86), and every node evaluating the 19
+// values that it reads 112 (130), k_expand and reading what it wrote 94; read-outs
+// of stored populations take 78 (76), but the next step then reads them.  A step and
+// a read-out of f and g: 232 (231) against 261 (279) on stored populations; at 24^3 in
+// one kernel 22 (25) against 26 (29).
+constexpr int kSpecialRun = 8 * kBlock;
+constexpr int kReadOne = 500000;
+__host__ __device__ constexpr int special_blocks(int N) { return (N + kSpecialRun - 1) / kSpecialRun; }
+
+// (WAIT: the values of the block's first kBlock special nodes are made before pdl_wait.)
+template <bool WAIT, typename T, typename S>
+__device__ __forceinline__ void read_special(const Consts<T>& k, const State<T, S>& s, int n0, T* f_o) {
+  __shared__ unsigned short list[kSpecialRun];
+  __shared__ int count;
+  const T corr = s.cbuf[s.c_prev];
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  // eight classes per thread in one load (the array is padded with zeros to a multiple of 32)
+  const int i0 = 8 * threadIdx.x;
+  if (n0 + i0 < k.N) {
+    const uint2 w = *reinterpret_cast<const uint2*>(s.cls + n0 + i0);
+    for (int i = 0; i < 8; ++i) {
+      const uint8_t c = (uint8_t)((i < 4 ? w.x : w.y) >> (8 * (i & 3)));
+      if (n0 + i0 + i < k.N && special_reader(k, s, (unsigned)(n0 + i0 + i), c, corr))
+        list[atomicAdd(&count, 1)] = (unsigned short)(i0 + i);
+    }
+  }
+  __syncthreads();
+  const unsigned N = (unsigned)k.N, Np = (unsigned)k.Np;
+  for (int i = threadIdx.x; i < count || (WAIT && i < kBlock); i += kBlock) {
+    T v[Q];
+    int n = 0;
+    if (i < count) {
+      n = n0 + list[i];
+      const uint8_t c = s.cls[n];
+      int ix, iy, iz;
+      decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+      const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
+      if (c & kSolid) {
+        // the node's own opposite slots, whose readers are its neighbours
+        const T* src = reinterpret_cast<const T*>(s.fin);
+        const T u[3] = {s.u[n], s.u[Np + n], s.u[2 * Np + n]}, sv[3] = {src[n], src[Np + n], src[2 * Np + n]};
+        T f[Q];
+        feval_all<S>(k, s.phi_in[n], u, sv, f);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          if (PopIO<T, S>::kDev) f[q] = stored_f<S>(k, q, f[q], s.phi_in[nb.at(n, ex(q), ey(q), ez(q))]);
+          v[opp(q)] = mul_rn(f[q], corr);
+        }
+      } else {
+        fetch_f_source<S>(v, k, s, n, nb, c, (c & kPartial) ? s.eps[n] : T(0));
+      }
+    }
+    if (WAIT && i < kBlock) pdl_wait();  // all threads of the block, once
+    if (i < count) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) f_o[q * N + n] = v[q];
+    }
+  }
+}
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) k_read_special(Consts<T> k, State<T, S> s, T* f_o) {
+  if (other_form(s)) {
+    pdl_wait();
+    return;
+  }
+  read_special<true>(k, s, blockIdx.x * kSpecialRun, f_o);
+}
+
+// ONE: with the special readers.
+template <typename T, typename S, bool ONE>
+__global__ void __launch_bounds__(kBlock) k_read_source(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
+  if (!ONE) pdl_trigger();
+  if (other_form(s)) return;
+  const int special = ONE ? special_blocks(k.N) : 0;
+  if (ONE && (int)blockIdx.x < special) {
+    read_special<false>(k, s, blockIdx.x * kSpecialRun, f_o);
+    return;
+  }
+  const int n = (blockIdx.x - special) * kBlock + threadIdx.x;
+  if (n >= k.N) return;
+  const unsigned N = (unsigned)k.N, Np = (unsigned)k.Np;
+  int ix, iy, iz;
+  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
+  {
+    const T* src = reinterpret_cast<const T*>(s.fin);
+    const T corr = s.cbuf[s.c_prev];
+    const T u[3] = {s.u[n], s.u[Np + n], s.u[2 * Np + n]}, sv[3] = {src[n], src[Np + n], src[2 * Np + n]};
+    T f[Q];
+    feval_all<S>(k, s.phi_in[n], u, sv, f);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const unsigned m = (unsigned)nb.at(n, ex(q), ey(q), ez(q));
+      const T v = PopIO<T, S>::kDev ? stored_f<S>(k, q, f[q], s.phi_in[m]) : f[q];
+      if (!ONE || !special_reader(k, s, m, s.cls[m], corr)) f_o[q * N + m] = mul_rn(v, corr);
+    }
+  }
+  if (g_o) {
+    const uint8_t c = s.cls[n];
+    T v[Q];
+    fetch_pop<T, S, false, false, false>(v, k, s.gin, s.phi_in, n, (size_t)N, nb, c, (c & kPartial) ? s.eps[n] : T(0), T(1));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) g_o[q * N + n] = v[q];
+  }
 }
 
 // The populations of a state in source form: s.fin holds S, s.phi_in the phi
