@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "lbm_common.cuh"
+#include "lbm_div.h"
 #include "lbm_launch.cuh"
 
 namespace lbm {
@@ -216,21 +217,6 @@ __device__ __forceinline__ T edot(int q, T a0, T a1) {
   return T(0);
 }
 
-// x / d, correctly rounded, from r = 1 / d correctly rounded: q = x r, then
-// q + r (x - d q) with the remainder exact in a fused multiply-add (Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34(1), 1990).  Three operations where the division's general
-// form takes about ten; several quotients by one d share its reciprocal.  The
-// same values as x / d except where the remainder underflows (|x| below ~1e-31
-// in float) and for infinite x (NaN).
-template <typename T>
-struct Div {
-  T d, r;
-  __device__ __forceinline__ T operator()(T x) const {
-    const T q = x * r;
-    return fma(fma(-d, q, x), r, q);
-  }
-};
 __device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
 __device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
 template <typename T>
@@ -713,15 +699,16 @@ __global__ void __launch_bounds__(kBlock) k2_update(Consts<T> k, State<T, T> s, 
     S0 = S0 + (k.mob * (mx - gx)) * k.guo;
     S1 = S1 + (k.mob * (my - gy)) * k.guo;
   } else {
-    // |grad| clamped to 1e-10: below 1e-21 (most of the gas) its square needs no root
+    // |grad| clamped to 1e-10: below 1e-21 (most of the gas) its square needs no root.
+    // (phi and its ghost values are bounded, so are these quotients.)
     const T g2 = gx * gx + gy * gy;
     Div<T> by_gm{T(1e-10), T(1) / T(1e-10)};
     if (!(g2 < T(1e-21))) {
       const T gm = sqrt(g2);
       by_gm = by(gm < T(1e-10) ? T(1e-10) : gm);
     }
-    const T lam = Div<T>{k.W, k.inv_W}((T(4) * phi) * (T(1) - phi));
-    T sx = ((k.cs2 * lam) * by_gm(gx)) * k.ac_scale, sy = ((k.cs2 * lam) * by_gm(gy)) * k.ac_scale;
+    const T lam = Div<T>{k.W, k.inv_W}.bounded((T(4) * phi) * (T(1) - phi));
+    T sx = ((k.cs2 * lam) * by_gm.bounded(gx)) * k.ac_scale, sy = ((k.cs2 * lam) * by_gm.bounded(gy)) * k.ac_scale;
     if (k.wetting) {
       const T red = T(1) - k.sharpen_reduce * k.ww[c >> kWwShift];
       sx = sx * red;
