@@ -404,7 +404,8 @@ int lbm_batch_size(LbmBatch* b, int* ncases);
 
 /* Autotuner of the batched step's launch shape: the phi kernel's nodes per
  * thread (1, 2, 4, 8, 12, 16, 24 or 32: its block count per case) and the
- * update kernel's threads per block (128 or 256).  Times `reps` batched
+ * update kernel's threads per block (128 or 256); only the latter where the
+ * nodes per thread reach no kernel (every case in source form, float64).  Times `reps` batched
  * steps that re-read the current state for each candidate pair and keeps the
  * fastest; the state is left unchanged.  Every case must have taken a step.
  * Synchronises `stream`; allocates temporary copies of u.  Outputs (may be

@@ -1388,11 +1388,12 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
                             : fail(LBM_E_CUDA, std::string("lbm_autotune: ") + cudaGetErrorString(e));
       if (rc != LBM_OK) break;
     }
-    // the two-kernel step: also its phi kernel's nodes per thread and the
-    // update kernel's threads per block (256 only for the gradient-of-mu modes
-    // and the paired layout, whose update kernel has a fixed block)
+    // the two-kernel step: also its phi kernel's nodes per thread (of the pass
+    // over stored populations) and the update kernel's threads per block (256
+    // only for the gradient-of-mu modes and the paired layout, whose update
+    // kernel has a fixed block)
     const std::vector<int> pers =
-        t.tx == 0 ? std::vector<int>{4, 8, 12, 16, 24, 32} : std::vector<int>{h->phi_per_thread};
+        t.tx == 0 && !wants_s(h) ? std::vector<int>{4, 8, 12, 16, 24, 32} : std::vector<int>{h->phi_per_thread};
     const std::vector<int> bss =
         (t.tx == 0 && !h->mu && !h->paired) ? std::vector<int>{128, kBlock} : std::vector<int>{h->upd_block};
     for (int bs : bss) {
@@ -1424,7 +1425,8 @@ int lbm_autotune(LbmHandle* h, int reps, void* stream, int* best_txyz3, float* b
     h->desc_ok = false;
   }
   cudaMemcpyAsync(h->u, u_save, ub, cudaMemcpyDeviceToDevice, st);
-  if (rc == LBM_OK) rc = restore_form(h, st);
+  const int rf = restore_form(h, st);
+  if (rc == LBM_OK) rc = rf;
   cudaStreamSynchronize(st);
   cudaFree(u_save);
   cudaEventDestroy(e0);
@@ -2417,6 +2419,18 @@ int lbm_batch_size(LbmBatch* b, int* ncases) {
   return LBM_OK;
 }
 
+namespace {
+// Whether the nodes per thread of the batch's phi pass count: not where every case
+// steps in source form, nor in float64 (a case's own split).
+bool per_counts(const LbmBatch* b) {
+  if (b->prec == LBM_F64) return false;
+  if (!steps_apart(b)) return b->coop || !b->src;
+  for (const LbmHandle* h : b->h)
+    if (!wants_s(h)) return true;
+  return false;
+}
+}  // namespace
+
 int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread, float* best_ms) {
   if (!b) return fail(LBM_E_ARG, "lbm_batch_autotune: null batch");
   if (reps <= 0) reps = 5;
@@ -2443,8 +2457,10 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   const bool apart = steps_apart(b);
   int best = b->phi_per_thread, best_bs = b->upd_block, rc = batch_form(b, st, &phis_in);
   float best_t = 1e30f;
+  const std::vector<int> pers = per_counts(b) ? std::vector<int>{1, 2, 4, 8, 12, 16, 24, 32}
+                                              : std::vector<int>{b->phi_per_thread};
   for (int bs : {128, kBlock})
-  for (int per : {1, 2, 4, 8, 12, 16, 24, 32}) {
+  for (int per : pers) {
     if (rc != LBM_OK) break;
     if (b->coop && bs != kBlock) continue;  // the cooperative step runs 256-thread update blocks
     b->phi_per_thread = per;
@@ -2478,7 +2494,8 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
   for (size_t i = 0; i < b->h.size(); ++i) {
     const size_t ub = 3 * (size_t)b->h[i]->Np * b->h[i]->tsize;
     cudaMemcpyAsync(b->h[i]->u, usave[i], ub, cudaMemcpyDeviceToDevice, st);
-    if (rc == LBM_OK && wants_s(b->h[i])) rc = restore_form(b->h[i], st);
+    const int rf = wants_s(b->h[i]) ? restore_form(b->h[i], st) : LBM_OK;
+    if (rc == LBM_OK) rc = rf;
   }
   cudaStreamSynchronize(st);
   for (void* p : usave) cudaFree(p);

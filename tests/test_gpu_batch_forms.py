@@ -51,3 +51,20 @@ def test_table_batch_matches_cases_alone(name, dtype):
     b.run(4)
     _same(alone, mixed)
     b.close()
+
+
+def test_autotuners_leave_alone_what_reaches_no_kernel():
+    """The nodes per thread of the phi pass over stored populations, in source form."""
+    from lbm.batch import AllenCahnBatch
+    s = _solver(0, (24, 24, 20), torch.float32)
+    s.run(3)
+    s.set_launch_shape(11, 128)
+    s.autotune(reps=1)
+    assert s.launch_shape()[0] == 11
+    cases = [_solver(i, (24, 24, 20), torch.float32) for i in range(3)]
+    b = AllenCahnBatch(cases)
+    b.run(3)
+    per = b.launch_shape()[0]
+    for _ in range(4):
+        assert b.autotune(reps=1)[0] == per
+    b.close()
