@@ -19,8 +19,7 @@ namespace lbm {
 // |x / d| above 2^-126), within an ulp below that.  Where the remainder is not a
 // number (x, d or the quotient infinite, d zero) the value is x r: as x / d, an
 // infinity or zero, or NaN where that is.  (The division itself outside of the
-// first range, by a test of x and q: 1024x1024 float 40 -> 73 us a step; this
-// selection 40 -> 42.)
+// first range, by a test of x and q: 1024x1024 float 40 -> 73 us a step.)
 template <typename T>
 struct Div {
   T d, r;
@@ -34,5 +33,35 @@ struct Div {
     return std::fma(std::fma(-d, q, x), r, q);
   }
 };
+
+// x / d by a constant d = cs2 or 2 cs2 (cs2 = 1/3 in T): x times the double-length
+// reciprocal hi + lo, hi rounded towards zero and lo > 0 (so an infinite x gives
+// that infinity), in two operations: x hi + rnd(x lo), rounded once.  Its error is
+// within 0.5 + 2^-p of an ulp (p the type's bits): the correctly rounded quotient for
+// every float mantissa but one (0x1.555554p0, a tie but for 2^-24 of an ulp, one ulp
+// off); below 2^-100 (float) within an ulp.  (Div's form with its selection in these
+// places: 1024x1024 float 40 -> 42 us a step.)
+template <typename T>
+struct ByCs2;
+template <>
+struct ByCs2<float> {
+  static constexpr float d = 0x1.555556p-2f, hi = 0x1.7ffffep+1f, lo = 0x1.4p-23f;
+};
+template <>
+struct ByCs2<double> {
+  static constexpr double d = 0x1.5555555555555p-2, hi = 0x1.8p+1, lo = 0x1.8p-53;
+};
+static_assert(ByCs2<float>::d == (float)(1.0 / 3.0) && ByCs2<double>::d == 1.0 / 3.0, "cs2");
+template <typename T>
+struct DivConst {
+  T hi, lo;
+  __host__ __device__ __forceinline__ T operator()(T x) const { return std::fma(x, hi, x * lo); }
+};
+template <typename T>
+__host__ __device__ __forceinline__ DivConst<T> by_cs2() { return DivConst<T>{ByCs2<T>::hi, ByCs2<T>::lo}; }
+template <typename T>
+__host__ __device__ __forceinline__ DivConst<T> by_two_cs2() {
+  return DivConst<T>{T(0.5) * ByCs2<T>::hi, T(0.5) * ByCs2<T>::lo};
+}
 
 }  // namespace lbm

@@ -221,18 +221,13 @@ __device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
 __device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
 template <typename T>
 __device__ __forceinline__ Div<T> by(T d) { return Div<T>{d, rcp_rn(d)}; }
-template <typename T>
-__device__ __forceinline__ Div<T> by_cs2() { return Div<T>{cs2<T>(), T(1) / cs2<T>()}; }
-template <typename T>
-__device__ __forceinline__ Div<T> by_two_cs2() { return Div<T>{T(2) * cs2<T>(), T(1) / (T(2) * cs2<T>())}; }
-
 // t[q] = (c e_q . (a0, a1)) / d for every q, with one division per opposite
 // pair (q, opp q): e_opp(q) . a = -(e_q . a) exactly, and (c (-x)) / d =
 // -((c x) / d) in IEEE arithmetic, so the opposite's value is the negation.
 // c and d depend on the weight class (cw: per q); the rest value is 0.
 // Same values as the per-q expression of the reference.
-template <typename T, typename CW>
-__device__ __forceinline__ void pair_div(T (&t)[Q9], T a0, T a1, CW cw, const Div<T>& d) {
+template <typename T, typename CW, typename D>
+__device__ __forceinline__ void pair_div(T (&t)[Q9], T a0, T a1, CW cw, const D& d) {
   t[0] = T(0);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

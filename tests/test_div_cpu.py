@@ -1,5 +1,6 @@
 """The quotients of the 2-D step (csrc/lbm_div.h) against the division, compiled for the host: the same value for
-zeros, infinities, NaN and overflow and wherever the remainder is representable, within an ulp below that."""
+zeros, infinities, NaN and overflow and wherever the remainder is representable, within an ulp below that.  Quotients by
+cs2: every float mantissa (one of them, next to a tie, an ulp off), many double ones."""
 import os
 import shutil
 import subprocess
@@ -41,8 +42,39 @@ template <typename T> int run(int lo, int hi, int emin) {
   }
   return bad;
 }
+template <typename T> bool cs2_special() {
+  using L = std::numeric_limits<T>;
+  const T inf = L::infinity(), d = lbm::ByCs2<T>::d;
+  const T xs[] = {0, -(T)0, 1, -1, inf, -inf, L::quiet_NaN(), L::max(), -L::max()};
+  bool ok = true;
+  for (T x : xs) ok = ok && same(lbm::by_cs2<T>()(x), x / d) && same(lbm::by_two_cs2<T>()(x), x / (2 * d));
+  for (int i = 0; i < 100000; ++i) {
+    const T x = value<T>(L::min_exponent - (int)(rnd() % 20)), t = x / d;
+    ok = ok && std::fabs(lbm::by_cs2<T>()(x) - t) <= std::nextafter(std::fabs(t), inf) - std::fabs(t);
+  }
+  return ok;
+}
+int cs2() {
+  int bad = 0, off = 0;
+  for (uint32_t m = 0; m < (1u << 23); ++m) {
+    const uint32_t b = 0x3f800000u | m;
+    float x;
+    std::memcpy(&x, &b, 4);
+    for (int two = 0; two < 2; ++two) {
+      const float t = x / (lbm::ByCs2<float>::d * (two ? 2 : 1));
+      const float e = two ? lbm::by_two_cs2<float>()(x) : lbm::by_cs2<float>()(x);
+      if (e != t) (std::fabs(e - t) <= std::nextafter(t, 9.0f) - t && x == 0x1.555554p0f ? off : bad)++;
+    }
+  }
+  for (int i = 0; i < 20000000; ++i) {
+    const double x = value<double>((int)(rnd() % 200) - 100);
+    if (lbm::by_cs2<double>()(x) != x / lbm::ByCs2<double>::d) ++bad;
+  }
+  if (bad || off != 2 || !cs2_special<float>() || !cs2_special<double>()) std::printf("cs2: bad %d off %d\n", bad, off), ++bad;
+  return bad;
+}
 int main() {
-  const int bad = run<float>(-100, 90, -149) + run<double>(-900, 900, -1074);
+  const int bad = cs2() + run<float>(-100, 90, -149) + run<double>(-900, 900, -1074);
   std::printf("%d\n", bad);
   return bad != 0;
 }
