@@ -1955,7 +1955,7 @@ struct LbmBatch {
   int phi_per_thread = 16;  // nodes per phi-kernel thread (half as many pairs in the paired layout)
   std::vector<int> phin;    // phi blocks of each case
   std::vector<int> per64;   // float64: each case's own phi_per_thread, which they follow
-  int upd_block = 128;      // threads per block of the linear-layout update kernel
+  int upd_block = 128;      // threads per block of the linear-layout update kernel of the two launches
   bool coop = false;        // one cooperative launch per step (k_batch_coop) instead of two launches
   size_t desc = 0;          // bytes of one case descriptor
   void* table[2] = {nullptr, nullptr};  // device descriptors: [0] this step, [1] the next
@@ -2000,6 +2000,9 @@ bool table_src(const LbmBatch* b) {
   return nodes <= 1000000 || (b->prec == LBM_F32 && nodes > 3000000);
 }
 
+// Threads per block of the update work: the cooperative form has its own.
+int upd_block_in(const LbmBatch* b) { return b->coop ? kBlock : b->upd_block; }
+
 // Block -> case tables (device) for the current phi_per_thread; drops the graph.
 int batch_layout(LbmBatch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
@@ -2020,7 +2023,7 @@ int batch_layout(LbmBatch* b) {
                                       : phi_blocks_of(b->h[i], b->phi_per_thread);
     const int g = launch_group(b->h[i]);
     pb[b->h[i]->paired ? 1 : 0] += phin;
-    ub[g] += upd_blocks_of(b->h[i], b->upd_block);
+    ub[g] += upd_blocks_of(b->h[i], upd_block_in(b));
     jb += b->tiles[i].blocks();
   }
   const long long tot = pb[0] + pb[1] + ub[0] + ub[1] + ub[2] + ub[3] + jb;
@@ -2038,7 +2041,7 @@ int batch_layout(LbmBatch* b) {
     size_t& a = at[b->h[i]->paired ? 1 : 0];
     for (int k = b->phin[i]; k > 0; --k) t[a++] = (unsigned short)i;
     size_t& c = at[2 + launch_group(b->h[i])];
-    for (int k = upd_blocks_of(b->h[i], b->upd_block); k > 0; --k) t[c++] = (unsigned short)i;
+    for (int k = upd_blocks_of(b->h[i], upd_block_in(b)); k > 0; --k) t[c++] = (unsigned short)i;
     for (int k = b->tiles[i].blocks(); k > 0; --k) t[at[6]++] = (unsigned short)i;
   }
   CUDA_TRY(cudaMalloc(&b->b2c, t.size() * sizeof(unsigned short)));
@@ -2054,7 +2057,7 @@ void batch_fill_t(LbmBatch* b) {
   for (int i = 0; i < n; ++i) {
     LbmHandle* h = b->h[i];
     const PhiTile& tile = b->tiles[i];
-    const int phin = b->phin[i], updn = upd_blocks_of(h, b->upd_block),
+    const int phin = b->phin[i], updn = upd_blocks_of(h, upd_block_in(b)),
               g = launch_group(h);
     int& pbl = pb[h->paired ? 1 : 0];
     for (int par = 0; par < 2; ++par) {
@@ -2402,14 +2405,13 @@ int lbm_batch_set_cooperative(LbmBatch* b, int on) {
         return fail(LBM_E_UNSUPPORTED, "lbm_batch_set_cooperative: the single-launch step serves linear-layout cases");
   }
   b->coop = on != 0;
-  if (b->coop) b->upd_block = kBlock;
   return batch_layout(b);
 }
 
 int lbm_batch_get_launch(LbmBatch* b, int* phi_nodes_per_thread, int* update_block) {
   if (!b) return fail(LBM_E_ARG, "lbm_batch_get_launch: null batch");
   if (phi_nodes_per_thread) *phi_nodes_per_thread = b->phi_per_thread;
-  if (update_block) *update_block = b->upd_block;
+  if (update_block) *update_block = upd_block_in(b);
   return LBM_OK;
 }
 
@@ -2464,7 +2466,7 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
     if (rc != LBM_OK) break;
     if (b->coop && bs != kBlock) continue;  // the cooperative step runs 256-thread update blocks
     b->phi_per_thread = per;
-    b->upd_block = bs;
+    if (!b->coop) b->upd_block = bs;
     rc = batch_layout(b);
     if (rc == LBM_OK && !apart) rc = batch_fill(b, st);
     if (rc != LBM_OK) break;
@@ -2488,7 +2490,7 @@ int lbm_batch_autotune(LbmBatch* b, int reps, void* stream, int* best_per_thread
     if (ms < best_t) {
       best_t = ms;
       best = per;
-      best_bs = bs;
+      if (!b->coop) best_bs = bs;
     }
   }
   for (size_t i = 0; i < b->h.size(); ++i) {

@@ -68,3 +68,18 @@ def test_autotuners_leave_alone_what_reaches_no_kernel():
     for _ in range(4):
         assert b.autotune(reps=1)[0] == per
     b.close()
+
+
+def test_cooperative_form_leaves_the_update_block_of_the_two_launches():
+    from lbm.batch import AllenCahnBatch
+    cases = [_solver(i, (24, 24, 20), torch.float32) for i in range(2)]
+    b = AllenCahnBatch(cases)
+    before = b.launch_shape()
+    b.set_cooperative(True)
+    assert b.launch_shape()[1] == 256
+    b.run(2)
+    b.autotune(reps=1)
+    b.set_cooperative(False)
+    assert b.launch_shape()[1] == before[1]
+    b.run(2)
+    b.close()
