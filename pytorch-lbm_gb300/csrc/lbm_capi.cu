@@ -119,7 +119,6 @@ static int fail(int code, const std::string& msg) {
 
 constexpr size_t kDescBytes = 4096;  // room for one case descriptor in host memory
 constexpr int kMeasureBlocks = 1024;
-constexpr int kMeasVals = 11;
 
 struct LbmHandle {
   LbmParams prm;
@@ -659,7 +658,7 @@ int64_t units_of(const LbmHandle* h) { return h->paired ? h->N / 2 : h->N; }
 // (LbmBatch::phin): its sum of phi is rounded per block, and a batch gives the
 // same bits as its cases alone.  (Float sums are exact fixed point.)
 int phi_blocks_of(const LbmHandle* h, int per_thread, bool alone = false) {
-  const int64_t wave = (h->paired ? 456 : 608) * (int64_t)kBlock;
+  const int64_t wave = (int64_t)(h->paired ? 3 : 4) * kSms * kBlock;
   if (alone) per_thread = (int)std::max<int64_t>(1, std::min<int64_t>(per_thread, (h->N + wave - 1) / wave));
   const long long per = (long long)kBlock * (h->paired ? (alone ? (per_thread + 1) / 2 : std::max(1, per_thread / 2)) : per_thread);
   return (int)std::max<long long>(1, (units_of(h) + per - 1) / per);
@@ -681,18 +680,18 @@ bool wants_s(const LbmHandle* h) {
 }
 
 // Tiles of the source form's phi pass: the (y, z) split whose blocks (tile plus
-// halo within kPhisThreads nodes) waste the fewest threads.
-constexpr int kPhisThreads = 320, kPhisSlots = 304;  // two blocks per SM
+// halo within kPhisNT nodes) waste the fewest threads.
+constexpr int kPhisSlots = kPhisPerSm * kSms;
 PhiTile phis_split(const LbmHandle* h) {
   const int ny = (int)h->ny, nz = (int)h->nz;
   PhiTile best{};
   double best_eff = -1.0;
   for (int ntz = 1; ntz <= nz; ++ntz) {
     const int tz = (nz + ntz - 1) / ntz;
-    if (tz + 2 > kPhisThreads / 3) continue;
-    const int rows = kPhisThreads / (tz + 2) - 2;
+    if (tz + 2 > kPhisNT / 3) continue;
+    const int rows = kPhisNT / (tz + 2) - 2;
     const int nty = (ny + rows - 1) / rows, ty = (ny + nty - 1) / nty, ntz_ = (nz + tz - 1) / tz;
-    const double eff = (double)ny * nz / ((double)nty * ntz_ * kPhisThreads);
+    const double eff = (double)ny * nz / ((double)nty * ntz_ * kPhisNT);
     if (eff > best_eff * 1.01) {
       best_eff = eff;
       best.ty = ty;

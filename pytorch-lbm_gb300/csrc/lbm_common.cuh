@@ -56,6 +56,12 @@ struct Lat {
   __host__ __device__ static constexpr T inv_w(int q) { return T(1) / w(q); }     // 1 / w_q
 };
 
+// Shared by the work splits (host) and the kernels they are for.
+constexpr int kSms = 152;     // SMs of the part the splits fill; any number gives the same float results
+constexpr int kPhisNT = 320;  // threads per block of the source form's phi pass: nodes of a tile and its halo
+constexpr int kPhisPerSm = 2; // its resident blocks per SM
+constexpr int kMeasVals = 11; // doubles of room per block's partial of the diagnostics
+
 // Node class byte.
 constexpr uint8_t kSolid = 1;     // solid node (bounce-back)
 constexpr uint8_t kBoundary = 2;  // fluid node with a solid D3Q19 neighbour (wetting)

@@ -1922,7 +1922,6 @@ __global__ void __launch_bounds__(kBlock) k_populations(Consts<T> k, State<T, S>
 // reduced on it (128x128x96: 67 us with all eleven values in float64, 42 us
 // with the merges between warps and blocks there, 21 us without).
 // ---------------------------------------------------------------------------
-constexpr int kMeasVals = 11;  // doubles of room per block's partial
 
 template <typename T>
 struct Meas {

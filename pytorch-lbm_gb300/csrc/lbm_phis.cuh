@@ -27,7 +27,6 @@
 
 namespace lbm {
 
-constexpr int kPhisNT = 320;  // threads per block: nodes of the tile and its halo
 // rows of float pairs in shared memory: the 4 e_x = +1 velocities of two pairs
 // of planes, the 8 e_x = 0 and the 4 e_x = -1 ones of one (the column's own 0,
 // 1, 2 stay in registers)
@@ -287,7 +286,7 @@ __device__ __forceinline__ void phis_block(const Consts<float>& k, const State<f
 }
 
 template <typename T, typename S>
-__global__ void __launch_bounds__(kPhisNT, 2) k_phis_one(const __grid_constant__ CaseDesc<T, S> d) {
+__global__ void __launch_bounds__(kPhisNT, kPhisPerSm) k_phis_one(const __grid_constant__ CaseDesc<T, S> d) {
   extern __shared__ __align__(16) float2 phis_sm[];
   pdl_trigger();
   pdl_wait();  // S and u of the previous update kernel
@@ -296,7 +295,7 @@ __global__ void __launch_bounds__(kPhisNT, 2) k_phis_one(const __grid_constant__
 }
 
 template <typename T, typename S>
-__global__ void __launch_bounds__(kPhisNT, 2) k_phis_batch(const CaseDesc<T, S>* __restrict__ cases,
+__global__ void __launch_bounds__(kPhisNT, kPhisPerSm) k_phis_batch(const CaseDesc<T, S>* __restrict__ cases,
                                                            const unsigned short* __restrict__ blk2case) {
   extern __shared__ __align__(16) float2 phis_sm[];
   __shared__ CaseDesc<T, S> d;
