@@ -170,7 +170,10 @@ struct Consts {
   T w[Q];      // lattice weights (float32 table, widened)
   T wc[Q];     // w_i / cs2                      (stencil weights)
   T w2c[Q];    // 2 w_i / cs2                    (laplacian weights)
-  T wac[Q];    // (1 - 1/(2 tau_f)) w_i          (Allen-Cahn source)
+  // (1 - 1/(2 tau_f)) w_i (Allen-Cahn source).  No kernel reads it; without it the
+  // fields below move and the table kernels spill more (float update on stored
+  // populations 4 -> 32 bytes, half in source form 4 -> 24).
+  T wac[Q];
   T wac3[Q];   // wac_i / cs2
   T inv_w[Q];  // 1 / w_i (deviation storage)
   T cs2, two_cs2, inv_cs2, inv_two_cs2, inv_W;

@@ -171,21 +171,6 @@ struct PopIO<float, __half> {
   }
 };
 
-// sqrt(x) for the magnitudes of the step, taken only where it can matter:
-// below 1e-21 (sqrt < 3.2e-11) every caller clamps the magnitude to 1e-10 or
-// compares it with 1e-6, so 0 is returned there.  A zero gradient (most of the
-// domain away from the interface) then never enters the square root's
-// special-case path.  Same results as sqrt(x) after the callers' clamp or
-// comparison; NaN still propagates.
-// GUARD selects it; the float32 update keeps the plain sqrt (measured on the
-// 150x150x107 case: the guard makes the half form 0.1791 -> 0.1759 ms per
-// step but the float32 form 0.1699 -> 0.1790, its register allocation shifting).
-template <bool GUARD, typename T>
-__device__ __forceinline__ T sqrt_mag(T x) {
-  if constexpr (GUARD) return (x >= T(1e-21) || x != x) ? sqrt(x) : T(0);
-  else return sqrt(x);
-}
-
 // Separately rounded multiply and add (never contracted into an FMA).  The
 // isotropic gradient is accumulated with these so that mirror-symmetric
 // neighbour pairs cancel to exactly zero, as in the reference: the
@@ -197,8 +182,6 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float rcp(float a) { return 1.0f / a; }
-__device__ __forceinline__ double rcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
 __device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
 __device__ __forceinline__ float sqrt_rn(float a) { return __fsqrt_rn(a); }
@@ -433,23 +416,6 @@ __device__ __forceinline__ T phi_value(const Consts<T>& k, const State<T, S>& s,
   return phi_of<T, S, MAP>(k, s, n, c, v, s.cbuf[s.c_prev],
                            (k.relax_on && (c & kTop)) ? ld_state(s.phi_in + (MAP ? sidx(k, n) : (unsigned)n)) : T(0));
 }
-
-// Lattice constants as the paired step kernels read them: compile-time immediates
-// (IMM) or the grid's constant table.  Both hold the same values (the table is
-// checked against the immediates when it is built); which is faster depends
-// on the kernel's register allocation (measured on the 150x150x107 case:
-// immediates for the half-storage form, 0.1829 -> 0.1797 ms per step; the
-// table for float storage, 0.1746 -> 0.1698).
-template <typename T, bool IMM>
-struct LatK {
-  const Consts<T>& k;
-  __device__ __forceinline__ T w(int q) const { return IMM ? Lat<T>::w(q) : k.w[q]; }
-  __device__ __forceinline__ T wc(int q) const { return IMM ? Lat<T>::wc(q) : k.wc[q]; }
-  __device__ __forceinline__ T w2c(int q) const { return IMM ? Lat<T>::w2c(q) : k.w2c[q]; }
-  __device__ __forceinline__ T cs2() const { return IMM ? Lat<T>::cs2() : k.cs2; }
-  __device__ __forceinline__ T inv_cs2() const { return IMM ? Lat<T>::inv_cs2() : k.inv_cs2; }
-  __device__ __forceinline__ T inv_two_cs2() const { return IMM ? Lat<T>::inv_two_cs2() : k.inv_two_cs2; }
-};
 
 // First population of each opposite pair (q, opp q) of D3Q19.
 __host__ __device__ constexpr int pair_first(int i) {
@@ -1120,7 +1086,7 @@ __device__ __forceinline__ bool grid_phi_total(TileSum<T>& ts, double* partials,
     unsigned long long* up = reinterpret_cast<unsigned long long*>(partials);
     if (threadIdx.x == 0) {
       unsigned long long r = 0ull;
-for (int i = 0; i < nw; ++i) r += s_warp[i];
+      for (int i = 0; i < nw; ++i) r += s_warp[i];
       up[blk] = nan ? kSumNaN : r;
       __threadfence();
       s_last = (atomicAdd(counter, 1u) == (unsigned)nblk - 1);
@@ -1142,7 +1108,7 @@ for (int i = 0; i < nw; ++i) r += s_warp[i];
     __syncthreads();
     if (threadIdx.x == 0) {
       unsigned long long r = 0ull;
-for (int i = 0; i < nw; ++i) r += s_warp[i];
+      for (int i = 0; i < nw; ++i) r += s_warp[i];
       *total = any_nan ? __longlong_as_double(0x7ff8000000000000ll) : (double)r / kFix;
       *counter = 0u;
     }

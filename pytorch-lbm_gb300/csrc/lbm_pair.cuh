@@ -22,6 +22,39 @@
 
 namespace lbm {
 
+// sqrt(x) for the magnitudes of the step, taken only where it can matter:
+// below 1e-21 (sqrt < 3.2e-11) every caller clamps the magnitude to 1e-10 or
+// compares it with 1e-6, so 0 is returned there.  A zero gradient (most of the
+// domain away from the interface) then never enters the square root's
+// special-case path.  Same results as sqrt(x) after the callers' clamp or
+// comparison; NaN still propagates.
+// GUARD selects it: in the half form.
+template <bool GUARD, typename T>
+__device__ __forceinline__ T sqrt_mag(T x) {
+  if constexpr (GUARD) return (x >= T(1e-21) || x != x) ? sqrt(x) : T(0);
+  else return sqrt(x);
+}
+
+__device__ __forceinline__ float rcp(float a) { return 1.0f / a; }
+__device__ __forceinline__ double rcp(double a) { return 1.0 / a; }
+
+// Lattice constants as the paired step kernels read them: compile-time immediates
+// (IMM) or the grid's constant table.  Both hold the same values (the table is
+// checked against the immediates when it is built); which is faster depends
+// on the kernel's register allocation (measured on the 150x150x107 case:
+// immediates for the half-storage form, 0.1829 -> 0.1797 ms per step; the
+// table for float storage, 0.1746 -> 0.1698).
+template <typename T, bool IMM>
+struct LatK {
+  const Consts<T>& k;
+  __device__ __forceinline__ T w(int q) const { return IMM ? Lat<T>::w(q) : k.w[q]; }
+  __device__ __forceinline__ T wc(int q) const { return IMM ? Lat<T>::wc(q) : k.wc[q]; }
+  __device__ __forceinline__ T w2c(int q) const { return IMM ? Lat<T>::w2c(q) : k.w2c[q]; }
+  __device__ __forceinline__ T cs2() const { return IMM ? Lat<T>::cs2() : k.cs2; }
+  __device__ __forceinline__ T inv_cs2() const { return IMM ? Lat<T>::inv_cs2() : k.inv_cs2; }
+  __device__ __forceinline__ T inv_two_cs2() const { return IMM ? Lat<T>::inv_two_cs2() : k.inv_two_cs2; }
+};
+
 template <typename T>
 struct VecOf;
 template <>
