@@ -22,7 +22,8 @@ One "step" is one lattice time step of the whole grid.  Reported:
   roofline   the dominant kernel (k_update): algorithmic bytes per launch /
              its CUDA-event duration (from a separate pass with events between
              the kernels), against the measured HBM copy peak; step_roofline:
-             the whole step's bytes (224 B/node) over the timed region.
+             the whole step's bytes (224 B/node in source form) over the
+             timed region.
   cpu_baseline  the numpy oracle (oracle/ac_oracle.py) on a bounded sample of
              the same workload, one host core; the reference's own PyTorch
              CPU figure, measured where the reference is installed, beside it.
@@ -47,29 +48,37 @@ sys.path.insert(0, ROOT)
 
 import numpy as np  # noqa: E402
 
-# Algorithmic bytes per node and step, float32 state.  The two-kernel step
-# keeps the source vector S in place of f (tau_f == 1): g (19), u (3), S (3)
-# and the previous phi (1), each read once and written once:
-# 2 x 4 x (19 + 3 + 3 + 1) = 208 B, and 4 x 4 more because the phi kernel and
-# the update kernel both read u and the previous phi.  Half-precision population
-# storage: 2 x 2 x 19 + 2 x 4 x 7 + 16 = 148 B.  The fused kernel keeps f and g:
-# 2 x 4 x (38 + 3 + 1) = 336 B, or 184 B.
-B_ALG_STEP = {"fp32": 224, "fp16": 148}
-B_ALG_STEP_FUSED = {"fp32": 336, "fp16": 184}
-# Per kernel (each adds the node-class byte it reads):
-#   k_phi     previous phi (4), u (12), S (12) read, phi written (4)
-#   k_update  g (76 | 38), u (12) and previous phi (4) read; g (76 | 38), u (12)
-#             and S (12) written; the phi stencil comes from L2
-#   k_step    the fused kernel: the whole step
-B_ALG_KERNEL = {"fp32": {"k_phi": 33, "k_update": 193, "k_step": 337},
-                "fp16": {"k_phi": 33, "k_update": 117, "k_step": 185}}
-# 2-D (D2Q9) grids, float32: S (2) in place of f, g (9), u (2), previous phi (1),
-# read and written once: 2 x 4 x 14 = 112 B, and 4 x 3 more for u and the
-# previous phi read by both kernels.  k2_phis reads the previous phi (4), u (8),
-# S (8) and the class byte and writes phi (4); k2_update reads g (36), u (8), the
-# previous phi (4) and the class byte and writes g (36), u (8) and S (8).
-B_ALG_STEP_2D = 124
-B_ALG_KERNEL_2D = {"k2_phi": 25, "k2_update": 101}
+def alg_bytes(precision, two_d=False, fused=False, source=True, gmu=False):
+    """Algorithmic bytes per node of (the step, its phi kernel, the rest of it: the update kernel and, in the
+    gradient-of-mu modes, the two kernels of mu before it).  Each kernel's include the node-class byte it reads; the phi
+    stencil comes from L2.
+
+    source  the state is phi, u and the interface source S (one value per dimension) between steps, else f stands in
+            the place of S.  The phi kernel reads the previous phi, u and S (or f; in half storage also the previous phi)
+            and writes phi; the update kernel reads g, u and the previous phi and writes g, u and S (or f).
+    fused   one kernel for the step, stored populations.
+    gmu     mu (phi read, mu written), its gradient (mu read, gradient written), both read by the update kernel;
+            the 2-D update also reads f again."""
+    dim, q = (2, 9) if two_d else (3, 19)
+    pop = (2 if precision == "fp16" else 4) * q
+    vec = 4 * dim
+    state = vec if source else pop
+    phi = 4 + 1 + state + (4 + vec if source else 4 if precision == "fp16" else 0)
+    upd = 1 + 2 * pop + 2 * vec + 4 + state
+    if fused:
+        return 4 * pop + 2 * vec + 2 * 4, None, 4 * pop + 2 * vec + 2 * 4 + 1
+    step = phi + upd - 2
+    if gmu:
+        extra = 4 + 4 + 4 + vec + 4 + vec + (pop if two_d else 0)
+        step += extra
+        upd += extra + 2
+    return step, phi, upd
+
+
+def source_form(two_d, ny, n, paired, gmu):
+    """Whether the library keeps a float or half state with tau_f == 1 in source form (wants_s in lbm_capi.cu)."""
+    return (not gmu and ny >= 256 and n >= 700000) if two_d else not paired
+
 
 WORKLOADS = {
     "ridge150": dict(grid=(150, 150, 107), substrate=("ridge", 1.0, 22.5), center=(75, 75, 80),
@@ -397,10 +406,11 @@ def run_ours(args, rank, world, device):
     if rank == 0:
         peak, peak_kind = peaks()
         f16 = args.precision == "fp16"
-        b_step = B_ALG_STEP_2D if two_d else (B_ALG_STEP if two_kernel else B_ALG_STEP_FUSED)[args.precision]
+        gmu = args.mode in ("cahn-hilliard", "mu-drive")
+        b_step, b_phi, b_ker = alg_bytes(args.precision, two_d, not two_kernel,
+                                         source_form(two_d, cfg.ny, n, layout == "paired", gmu), gmu)
         # the dominant kernel of the step: k_update (two-kernel step) or k_step (fused)
         kname = ("k2_update" if two_d else "k_update") if two_kernel else "k_step"
-        b_ker = B_ALG_KERNEL_2D[kname] if two_d else B_ALG_KERNEL[args.precision][kname]
         ker_s = upd_ms / K / 1e3
         achieved = b_ker * n / ker_s / 1e9
         traffic_pn = profiled_traffic(kname + ("_f16" if f16 else ""))
@@ -408,7 +418,6 @@ def run_ours(args, rank, world, device):
         kernels = {}
         if two_kernel:
             pname = "k2_phi" if two_d else "k_phi"
-            b_phi = B_ALG_KERNEL_2D[pname] if two_d else B_ALG_KERNEL[args.precision][pname]
             kernels = {pname: {"ms_per_launch": phi_ms / K, "bytes_per_node": b_phi,
                                "achieved_gbs": b_phi * n / (phi_ms / K / 1e3) / 1e9},
                        kname: {"ms_per_launch": upd_ms / K, "bytes_per_node": b_ker,
@@ -465,7 +474,7 @@ def run_ours(args, rank, world, device):
                               "frac": step_bw / peak, "mlups_roofline": peak * 1e3 / b_step},
             "kernels": kernels,
             # two kernels per step (four with the mu and grad-mu passes of the grad-mu modes)
-            "gpu_launches": ((4 if args.mode in ("cahn-hilliard", "mu-drive") else 2) * K) if two_kernel else K,
+            "gpu_launches": ((4 if gmu else 2) * K) if two_kernel else K,
             "cpu_baseline": cpu,
             "fp64_error": fp64,
             "clocks": clk.summary(),
