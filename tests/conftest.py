@@ -1,3 +1,4 @@
+import gc
 import os
 import sys
 
@@ -20,3 +21,11 @@ def built_lib():
     from lbm import _build, _native
     _build.build()
     return _native.lib()
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _collect_solvers():
+    """A solver and its wetting tables refer to each other: what a module's tests left gives its device arrays back at
+    the module's end, not in the middle of a later module that watches memory."""
+    yield
+    gc.collect()
