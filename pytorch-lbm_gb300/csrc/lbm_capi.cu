@@ -582,6 +582,12 @@ int clear_form(LbmHandle* h, cudaStream_t st) {
   h->form_set = h->sform = false;
   return LBM_OK;
 }
+// The device's word after a step of a grid alone on `st` whose input had the form `in` and that wrote S.
+int mark_form(LbmHandle* h, Form in, cudaStream_t st) {
+  if (in != Form::source && !is2d(h)) CUDA_TRY(cudaMemsetAsync(h->counters + 5, 1, sizeof(unsigned), st));
+  h->form_set = true;
+  return LBM_OK;
+}
 // What the host knows of the form (exactly that of f: not any), after kernels that wrote S without advancing the state.
 int restore_form(LbmHandle* h, cudaStream_t st) {
   CUDA_TRY(cudaMemsetAsync(h->counters + 5, h->sform ? 1 : 0, sizeof(unsigned), st));
@@ -874,7 +880,10 @@ int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr
     }
     if (rc != LBM_OK) return rc;
     h->sform = !h->raw && h->tiling.tx == 0 && wants_s(h);  // the first step writes populations
-    h->form_set = h->form_set || h->sform;
+    if (h->sform) {
+      rc = mark_form(h, form, st);
+      if (rc != LBM_OK) return rc;
+    }
     form = h->sform ? Form::source : Form::populations;
     h->last_raw_in = h->raw;
     h->obs_init = false;
@@ -2227,7 +2236,7 @@ int apart_step_t(LbmBatch* b, int nsteps, bool advance, cudaStream_t st) {
       h->upd_block = bs;
       if (rc == LBM_OK && advance) {
         h->sform = wants_s(h);
-        h->form_set = h->form_set || h->sform;
+        if (h->sform) rc = mark_form(h, form, b->lanes[b->lane_of[i]]);
         h->last_raw_in = h->obs_init = false;
         h->cur ^= 1;
         h->pc ^= 1;

@@ -1400,11 +1400,12 @@ __device__ __forceinline__ void update_one(const Consts<T>& k, const State<T, S>
 // addressing (NodeIn: 1,063 -> 890 instructions per warp and 136 -> 131 us with
 // stored populations on the 150x150x107 case), the blocks on the first and last
 // planes, whose x neighbours wrap around, the general one.
-template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS>
+// MARK: the device's word of the form is set with S.
+template <typename T, typename S, bool OMEGA1, bool GMU, bool SOUT, int BS, bool MARK = false>
 __device__ __forceinline__ void update_block(const Consts<T>& k, const State<T, S>& s, int n0) {
   const int n = n0 + threadIdx.x, P = k.ny * k.nz;
   const Pol pol = Pol::make();
-  if (SOUT && n == 0) *s.form = 1u;
+  if (SOUT && MARK && n == 0) *s.form = 1u;
   if (n0 >= P && n0 + BS <= k.N - P) {
     int ix, iy, iz;
     decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
@@ -1543,7 +1544,7 @@ __global__ void __launch_bounds__(BS, UpdateOccupancy<T, S>::blocks * kBlock / B
   load_desc(d, cases + blk2case[blockIdx.x]);
   pdl_trigger();
   pdl_wait();  // phi of the phi kernel
-  update_block<T, S, OMEGA1, false, SOUT, BS>(d.k, d.s, (blockIdx.x - d.upd_blk0) * BS);
+  update_block<T, S, OMEGA1, false, SOUT, BS, true>(d.k, d.s, (blockIdx.x - d.upd_blk0) * BS);
 }
 
 // The step kernels of one grid alone: the descriptor is a kernel parameter, so
