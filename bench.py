@@ -413,7 +413,8 @@ def run_ours(args, rank, world, device):
         kname = ("k2_update" if two_d else "k_update") if two_kernel else "k_step"
         ker_s = upd_ms / K / 1e3
         achieved = b_ker * n / ker_s / 1e9
-        traffic_pn = profiled_traffic(kname + ("_f16" if f16 else ""))
+        # the committed captures are of the default forms
+        traffic_pn = (None if gmu or layout == "paired" else profiled_traffic(kname + ("_f16" if f16 else "")))
         step_bw = b_step * n / (tot_ms / K / 1e3) / 1e9
         kernels = {}
         if two_kernel:

@@ -775,8 +775,7 @@ int fill_desc(LbmHandle* h, cudaStream_t st) {
 // after init and the fused kernel through launch_step; every other
 // two-kernel step through the kernels of a grid alone (linear layout), or the
 // paired kernels on the handle's one-case table.  in: the form of f (any: the phi
-// kernels of both forms, of which the state's runs; measured about 2 us more than
-// one of them).  `mid` (may be null) is recorded between the two kernels
+// kernels of both forms, of which the state's runs).  `mid` (may be null) is recorded between the two kernels
 // (before the fused kernel).
 template <typename T, typename S>
 int launch_next(LbmHandle* h, const Tiling& t, Form in, cudaStream_t st, cudaEvent_t mid) {

@@ -238,10 +238,11 @@ struct State {
   unsigned* status;
   int c_prev, c_cur;  // cbuf slots: factor applied to fin, factor produced this step
   // The form of the state on the device: *form is non-zero while it is the
-  // source form (lbm_phis.cuh).  Set by the host behind the first step of a grid alone
-  // that writes S (the store in its update kernel cost 2 % of the step), by the
-  // update kernels of batches and of 2-D grids.  form_if 0 or 1: the kernel runs only on a state
-  // of stored populations or of the source form; -1: the host knows the form.
+  // source form (lbm_phis.cuh).  Set by the host behind the first step of a grid
+  // alone that writes S (the store in its update kernel cost 2 % of the step), by
+  // the update kernels of batches and of 2-D grids.  form_if 0 or 1: the kernel
+  // runs only on a state of stored populations or of the source form; -1: the host
+  // knows the form.
   unsigned* form;
   int form_if;
 };
@@ -263,7 +264,7 @@ struct InjectParams {
   int obs_init;
 };
 
-// Work split of the phi pass over a state that holds J (lbm_phij.cuh): a
+// Work split of the phi pass over a state in source form (lbm_phis.cuh): a
 // block walks cx planes in x over a ty x tz tile of the (y, z) plane.
 struct PhiTile {
   int ty, tz, cx;      // tile extents, planes per block

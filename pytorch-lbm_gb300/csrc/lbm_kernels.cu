@@ -26,9 +26,10 @@
 //
 // Source form.  With tau_f == 1 (float compute, linear layout) the update stores
 // the interface source S in the place of f's 19 populations, and the phi pass
-// evaluates them again from phi, u and S (lbm_phis.cuh): 197 + 33 bytes per node
-// and step (float) instead of 257 + 81.  Whatever reads f gets it back with
-// k_expand.  Measured with the block-uniform addressing below on the 150x150x107
+// evaluates them again from phi, u and S (lbm_phis.cuh): 193 + 33 bytes per node
+// and step (float) instead of 257 + 81.  Read-outs of f evaluate it too
+// (k_read_source); what steps on from populations gets them with k_expand.
+// Measured with the block-uniform addressing below on the 150x150x107
 // case: 171.9 -> 144.4 us per step, 256x256x192 909 -> 702 us, 384x384x256 in
 // half storage 2288 -> 1849 us, 80x80x65 44.5 -> 31.0 us.
 //
@@ -1416,9 +1417,9 @@ __device__ __forceinline__ void update_block(const Consts<T>& k, const State<T, 
   }
 }
 
-// One thread per node, linear order.  What bounds it: 197 bytes per node (source
-// form) took 80 us on the 150x150x107 case in a kernel of the same loads and
-// stores without the arithmetic; with it 102.5 us (float), half of the warps'
+// One thread per node, linear order.  What bounds it: 193 bytes per node and this
+// step's phi from L2 (source form) took 80 us on the 150x150x107 case in a kernel
+// of the same loads and stores without the arithmetic; with it 102.5 us (float), half of the warps'
 // time waiting for loads, half of the issue slots used.  (Measured slower there: a
 // persistent grid-stride form, 108 -> 112 us; all loads first with 80 to 96
 // registers, 105 -> 115 us; forms that stage the next node's g, u and previous
@@ -2198,7 +2199,7 @@ cudaError_t launch_update_one(const void* desc, bool omega1, bool sout, cudaStre
   return launch_update_one_t<T, S, false, kBlock>(d, omega1, sout, st);
 }
 // The phi pass of a state that holds S (float compute only), and the
-// populations back from J: s.fout = the populations of the state s.fin.
+// populations back from S: s.fout = the populations of the state s.fin.
 template <typename T, typename S>
 cudaError_t launch_phis_batch(const void* cases, const unsigned short* b2c, int blocks, cudaStream_t st) {
   if constexpr (sizeof(T) == 8) {

@@ -13,8 +13,8 @@
 //              node, then its isotropic gradient;
 //   k2_update  stencils, wetting, forces, velocity, both BGK collisions.
 // Besides: k2_init (init_fields), k2_expand (populations of a state in source
-// form), k2_inject (inject_droplet), k2_observe and
-// k2_populations (attribute read-out).
+// form), k2_inject (inject_droplet), k2_observe, k2_populations, k2_read_source and
+// k2_read_special (attribute read-out).
 // These kernels keep the reference's operation order (divisions, per-
 // population non-equilibrium stress) instead of the restructured moment and
 // collision algebra of the 3-D kernels, and are compiled without FMA
