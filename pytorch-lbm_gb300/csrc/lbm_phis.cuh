@@ -324,10 +324,10 @@ __device__ __forceinline__ bool special_reader(const Consts<T>& k, const State<T
 // looked up before a value is written to it; above (the lookup of 18 classes per node costs
 // 35 us at 128x128x96) a second kernel, over what the first wrote there, which does all
 // but its stores before the first has ended.
-// us for f and g, float (half): 128x128x96 85 (86), and every node evaluating the 19
+// us for f and g, float (half): 128x128x96 84 (86), and every node evaluating the 19
 // values that it reads 112 (130), k_expand and reading what it wrote 94; read-outs
 // of stored populations take 78 (76), but the next step then reads them.  A step and
-// a read-out of f and g: 232 (231) against 261 (279) on stored populations; at 24^3 in
+// a read-out of f and g: 227 (230) against 261 (279) on stored populations; at 24^3 in
 // one kernel 22 (25) against 26 (29).
 constexpr int kSpecialRun = 8 * kBlock;
 constexpr int kReadOne = 500000;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kBlock) k_read_special(Consts<T> k, State<T, S
 
 // ONE: with the special readers.
 template <typename T, typename S, bool ONE>
-__global__ void __launch_bounds__(kBlock) k_read_source(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
+__global__ void __launch_bounds__(kBlock, 4) k_read_source(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
   if (!ONE) pdl_trigger();
   if (other_form(s)) return;
   const int special = ONE ? special_blocks(k.N) : 0;
