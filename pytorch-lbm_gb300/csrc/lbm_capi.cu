@@ -582,12 +582,6 @@ int clear_form(LbmHandle* h, cudaStream_t st) {
   h->form_set = h->sform = false;
   return LBM_OK;
 }
-// The device's word after a step of a grid alone on `st` whose input had the form `in` and that wrote S.
-int mark_form(LbmHandle* h, Form in, cudaStream_t st) {
-  if (in != Form::source && !is2d(h)) CUDA_TRY(cudaMemsetAsync(h->counters + 5, 1, sizeof(unsigned), st));
-  h->form_set = true;
-  return LBM_OK;
-}
 // What the host knows of the form (exactly that of f: not any), after kernels that wrote S without advancing the state.
 int restore_form(LbmHandle* h, cudaStream_t st) {
   CUDA_TRY(cudaMemsetAsync(h->counters + 5, h->sform ? 1 : 0, sizeof(unsigned), st));
@@ -795,19 +789,20 @@ int launch_next(LbmHandle* h, const Tiling& t, Form in, cudaStream_t st, cudaEve
       CUDA_TRY((launch_phi_pair<T, S>(d, nullptr, phi_blocks_of(h, h->phi_per_thread, true), st)));
     } else {
       if (case_desc_bytes<T, S>() > kDescBytes) return fail(LBM_E_ARG, "lbm_step: internal error: descriptor size");
-      auto fill = [&](int form_if) {
+      auto fill = [&](int form_if, bool set = false) {
         s.form_if = form_if;
+        s.form_set = set ? 1 : 0;  // of the phi pass over populations before S is written
         fill_case_desc<T, S>(one, consts_of<T>(*h), s, 0, phi_blocks_of(h, h->phi_per_thread, true), 0,
                              upd_blocks_of(h, h->upd_block), 0, h->tile);
       };
       if (in == Form::any) {
         fill(1);
         CUDA_TRY((launch_phis_one<T, S>(d, st)));
-        fill(0);
+        fill(0, true);
         CUDA_TRY((launch_phi_one<T, S>(d, st)));
         fill(-1);
       } else {
-        fill(-1);
+        fill(-1, in == Form::populations && wants_s(h));
         if (in == Form::source) CUDA_TRY((launch_phis_one<T, S>(d, st)));
         else CUDA_TRY((launch_phi_one<T, S>(d, st)));
       }
@@ -879,10 +874,7 @@ int do_step(LbmHandle* h, int nsteps, cudaStream_t st, cudaEvent_t* ev = nullptr
     }
     if (rc != LBM_OK) return rc;
     h->sform = !h->raw && h->tiling.tx == 0 && wants_s(h);  // the first step writes populations
-    if (h->sform) {
-      rc = mark_form(h, form, st);
-      if (rc != LBM_OK) return rc;
-    }
+    h->form_set = h->form_set || h->sform;
     form = h->sform ? Form::source : Form::populations;
     h->last_raw_in = h->raw;
     h->obs_init = false;
@@ -2235,7 +2227,7 @@ int apart_step_t(LbmBatch* b, int nsteps, bool advance, cudaStream_t st) {
       h->upd_block = bs;
       if (rc == LBM_OK && advance) {
         h->sform = wants_s(h);
-        if (h->sform) rc = mark_form(h, form, b->lanes[b->lane_of[i]]);
+        h->form_set = h->form_set || h->sform;
         h->last_raw_in = h->obs_init = false;
         h->cur ^= 1;
         h->pc ^= 1;

@@ -238,13 +238,14 @@ struct State {
   unsigned* status;
   int c_prev, c_cur;  // cbuf slots: factor applied to fin, factor produced this step
   // The form of the state on the device: *form is non-zero while it is the
-  // source form (lbm_phis.cuh).  Set by the host behind the first step of a grid
-  // alone that writes S (the store in its update kernel cost 2 % of the step), by
-  // the update kernels of batches and of 2-D grids.  form_if 0 or 1: the kernel
-  // runs only on a state of stored populations or of the source form; -1: the host
-  // knows the form.
+  // source form (lbm_phis.cuh).  Set in the step that goes over to it: by the
+  // update kernels of batches and of 2-D grids, of a grid alone by the last block of
+  // the phi pass over its stored populations (form_set; every block has looked at
+  // the word by then, and the store in the update kernel cost 2 % of the step).
+  // form_if 0 or 1: the kernel runs only on a state of stored populations or of the
+  // source form; -1: the host knows the form.
   unsigned* form;
-  int form_if;
+  int form_if, form_set;
 };
 
 // What the host knows of the form.

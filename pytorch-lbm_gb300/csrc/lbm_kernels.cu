@@ -1368,6 +1368,7 @@ __device__ __forceinline__ void phi_finish(const State<T, S>& s, TileSum<T>& par
     if (!(total == total) || total - total != 0.0) atomicOr(s.status, 1u);
     s.cbuf[s.c_cur] = corr;
     s.scal[1] = total;
+    if (s.form_set) *s.form = 1u;
   }
 }
 
