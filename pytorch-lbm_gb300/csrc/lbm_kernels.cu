@@ -2370,13 +2370,14 @@ cudaError_t launch_populations(const Consts<T>& k, const State<T, S>& s, bool ra
     if constexpr (sizeof(T) == 8) {
       return cudaErrorNotSupported;
     } else {
-      if (k.N < kReadOne) {
-        k_read_source<T, S, true><<<special_blocks(k.N) + grid, kBlock, 0, st>>>(k, s, f, g);
+      if (k.N < kReadSmall) {
+        k_read_small<T, S><<<grid, kBlock, 0, st>>>(k, s, f, g);
         return cudaGetLastError();
       }
-      k_read_source<T, S, false><<<grid, kBlock, 0, st>>>(k, s, f, g);
+      k_read_source<T, S><<<grid, kBlock, 0, st>>>(k, s, f, g);
       const cudaError_t e = cudaGetLastError();
-      return e == cudaSuccess ? launch_pdl(k_read_special<T, S>, special_blocks(k.N), st, k, s, f) : e;
+      const int special = (k.N + kSpecialRun - 1) / kSpecialRun;
+      return e == cudaSuccess ? launch_pdl(k_read_special<T, S>, special, st, k, s, f) : e;
     }
   }
   if (raw) k_populations<T, S, true><<<grid, kBlock, 0, st>>>(k, s, f, g);

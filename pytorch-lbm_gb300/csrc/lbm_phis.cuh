@@ -315,27 +315,47 @@ __device__ __forceinline__ bool special_reader(const Consts<T>& k, const State<T
   return pb > T(0.15) && pb < T(0.85);
 }
 
-// f and g (may be null) of a state in source form as the reference holds them
-// between steps, without writing anything of the state.  A thread evaluates its
-// node's f once and writes each value, corrected, to the slot of the node that
-// pulls it, and pulls its g.  f of the special readers is made by blocks that each
-// collect those of kSpecialRun nodes (a wall puts one or two into most warps): below
-// kReadOne nodes the first special_blocks(N) of the launch, and a node's class is
-// looked up before a value is written to it; above (the lookup of 18 classes per node costs
-// 35 us at 128x128x96) a second kernel, over what the first wrote there, which does all
-// but its stores before the first has ended.
-// us for f and g, float (half): 128x128x96 84 (86), and every node evaluating the 19
-// values that it reads 112 (130), k_expand and reading what it wrote 94; read-outs
-// of stored populations take 78 (76), but the next step then reads them.  A step and
-// a read-out of f and g: 227 (230) against 261 (279) on stored populations; at 24^3 in
-// one kernel 22 (25) against 26 (29).
-constexpr int kSpecialRun = 8 * kBlock;
-constexpr int kReadOne = 500000;
-__host__ __device__ constexpr int special_blocks(int N) { return (N + kSpecialRun - 1) / kSpecialRun; }
+// f of solid node n of a state in source form: its own opposite slots, whose readers
+// are its neighbours.
+template <typename T, typename S>
+__device__ __forceinline__ void solid_f_source(T (&v)[Q], const Consts<T>& k, const State<T, S>& s, int n, const Nbr& nb,
+                                               T corr) {
+  const unsigned Np = (unsigned)k.Np;
+  const T* src = reinterpret_cast<const T*>(s.fin);
+  const T u[3] = {s.u[n], s.u[Np + n], s.u[2 * Np + n]}, sv[3] = {src[n], src[Np + n], src[2 * Np + n]};
+  T f[Q];
+  feval_all<S>(k, s.phi_in[n], u, sv, f);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    if (PopIO<T, S>::kDev) f[q] = stored_f<S>(k, q, f[q], s.phi_in[nb.at(n, ex(q), ey(q), ez(q))]);
+    v[opp(q)] = mul_rn(f[q], corr);
+  }
+}
 
-// (WAIT: the values of the block's first kBlock special nodes are made before pdl_wait.)
-template <bool WAIT, typename T, typename S>
-__device__ __forceinline__ void read_special(const Consts<T>& k, const State<T, S>& s, int n0, T* f_o) {
+// f and g (may be null) of a state in source form as the reference holds them
+// between steps, without writing anything of the state.  Below kReadSmall nodes
+// every node evaluates the 19 values that it reads (k_read_small).  Above, a thread
+// evaluates its node's f once and writes each value, corrected, to the slot of the
+// node that pulls it, and pulls its g (k_read_source); f of the special readers follows
+// from k_read_special, over what the first kernel wrote there: its blocks collect those of
+// kSpecialRun nodes each (a wall puts one or two into most warps; a lookup of 18
+// classes per node instead costs 35 us at 128x128x96) and do all but their stores
+// before the first kernel has ended.
+// us for f and g, float (half): 128x128x96 84 (86), by k_read_small 112 (130),
+// k_expand and reading what it wrote 94; read-outs of stored populations take 78 (76),
+// but the next step then reads them.  A step and a read-out of f and g there: 227 (230)
+// against 261 (279) on stored populations; by k_read_small / the two kernels 24^3 20.4 /
+// 22.7 (20.4 / 26.5), 48^3 26.7 / 28.7 (28.7 / 30.8), 60^3 39.1 / 37.7 (41.4 / 41.1).
+constexpr int kSpecialRun = 8 * kBlock;
+constexpr int kReadSmall = 200000;
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) k_read_special(Consts<T> k, State<T, S> s, T* f_o) {
+  if (other_form(s)) {
+    pdl_wait();
+    return;
+  }
+  const int n0 = blockIdx.x * kSpecialRun;
   __shared__ unsigned short list[kSpecialRun];
   __shared__ int count;
   const T corr = s.cbuf[s.c_prev];
@@ -352,8 +372,8 @@ __device__ __forceinline__ void read_special(const Consts<T>& k, const State<T, 
     }
   }
   __syncthreads();
-  const unsigned N = (unsigned)k.N, Np = (unsigned)k.Np;
-  for (int i = threadIdx.x; i < count || (WAIT && i < kBlock); i += kBlock) {
+  const unsigned N = (unsigned)k.N;
+  for (int i = threadIdx.x; i < count || i < kBlock; i += kBlock) {
     T v[Q];
     int n = 0;
     if (i < count) {
@@ -363,21 +383,12 @@ __device__ __forceinline__ void read_special(const Consts<T>& k, const State<T, 
       decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
       const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
       if (c & kSolid) {
-        // the node's own opposite slots, whose readers are its neighbours
-        const T* src = reinterpret_cast<const T*>(s.fin);
-        const T u[3] = {s.u[n], s.u[Np + n], s.u[2 * Np + n]}, sv[3] = {src[n], src[Np + n], src[2 * Np + n]};
-        T f[Q];
-        feval_all<S>(k, s.phi_in[n], u, sv, f);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          if (PopIO<T, S>::kDev) f[q] = stored_f<S>(k, q, f[q], s.phi_in[nb.at(n, ex(q), ey(q), ez(q))]);
-          v[opp(q)] = mul_rn(f[q], corr);
-        }
+        solid_f_source(v, k, s, n, nb, corr);
       } else {
         fetch_f_source<S>(v, k, s, n, nb, c, (c & kPartial) ? s.eps[n] : T(0));
       }
     }
-    if (WAIT && i < kBlock) pdl_wait();  // all threads of the block, once
+    if (i < kBlock) pdl_wait();  // all threads of the block, once
     if (i < count) {
 #pragma unroll
       for (int q = 0; q < Q; ++q) f_o[q * N + n] = v[q];
@@ -386,25 +397,10 @@ __device__ __forceinline__ void read_special(const Consts<T>& k, const State<T, 
 }
 
 template <typename T, typename S>
-__global__ void __launch_bounds__(kBlock) k_read_special(Consts<T> k, State<T, S> s, T* f_o) {
-  if (other_form(s)) {
-    pdl_wait();
-    return;
-  }
-  read_special<true>(k, s, blockIdx.x * kSpecialRun, f_o);
-}
-
-// ONE: with the special readers.
-template <typename T, typename S, bool ONE>
 __global__ void __launch_bounds__(kBlock, 4) k_read_source(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
-  if (!ONE) pdl_trigger();
+  pdl_trigger();
   if (other_form(s)) return;
-  const int special = ONE ? special_blocks(k.N) : 0;
-  if (ONE && (int)blockIdx.x < special) {
-    read_special<false>(k, s, blockIdx.x * kSpecialRun, f_o);
-    return;
-  }
-  const int n = (blockIdx.x - special) * kBlock + threadIdx.x;
+  const int n = blockIdx.x * kBlock + threadIdx.x;
   if (n >= k.N) return;
   const unsigned N = (unsigned)k.N, Np = (unsigned)k.Np;
   int ix, iy, iz;
@@ -420,13 +416,35 @@ __global__ void __launch_bounds__(kBlock, 4) k_read_source(Consts<T> k, State<T,
     for (int q = 0; q < Q; ++q) {
       const unsigned m = (unsigned)nb.at(n, ex(q), ey(q), ez(q));
       const T v = PopIO<T, S>::kDev ? stored_f<S>(k, q, f[q], s.phi_in[m]) : f[q];
-      if (!ONE || !special_reader(k, s, m, s.cls[m], corr)) f_o[q * N + m] = mul_rn(v, corr);
+      f_o[q * N + m] = mul_rn(v, corr);
     }
   }
   if (g_o) {
     const uint8_t c = s.cls[n];
     T v[Q];
     fetch_pop<T, S, false, false, false>(v, k, s.gin, s.phi_in, n, (size_t)N, nb, c, (c & kPartial) ? s.eps[n] : T(0), T(1));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) g_o[q * N + n] = v[q];
+  }
+}
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(kBlock) k_read_small(Consts<T> k, State<T, S> s, T* f_o, T* g_o) {
+  const int n = blockIdx.x * kBlock + threadIdx.x;
+  if (n >= k.N || other_form(s)) return;
+  const unsigned N = (unsigned)k.N;
+  const uint8_t c = s.cls[n];
+  int ix, iy, iz;
+  decode(k.dz, k.dy, n, k.nz, k.ny, ix, iy, iz);
+  const Nbr nb = make_nbr_xyz(ix, iy, iz, k.nx, k.ny, k.nz);
+  const T eps = (c & kPartial) ? s.eps[n] : T(0);
+  T v[Q];
+  if (c & kSolid) solid_f_source(v, k, s, n, nb, s.cbuf[s.c_prev]);
+  else fetch_f_source<S>(v, k, s, n, nb, c, eps);
+#pragma unroll
+  for (int q = 0; q < Q; ++q) f_o[q * N + n] = v[q];
+  if (g_o) {
+    fetch_pop<T, S, false, false, false>(v, k, s.gin, s.phi_in, n, (size_t)N, nb, c, eps, T(1));
 #pragma unroll
     for (int q = 0; q < Q; ++q) g_o[q * N + n] = v[q];
   }

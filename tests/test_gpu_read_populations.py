@@ -43,7 +43,9 @@ def _same(a, b):
 
 
 CASES = [((2, 2, 2), torch.float32), ((7, 17, 18), torch.float32), ((40, 31, 27), torch.float16),
-         ((5, 9, 107), torch.float16), ((101, 97, 53), torch.float32), ((101, 97, 53), torch.float16), ((33, 40), torch.float32), ((6, 383), torch.float32)]
+         ((5, 9, 107), torch.float16), ((59, 58, 58), torch.float32), ((59, 58, 59), torch.float32),
+         ((101, 97, 53), torch.float32), ((101, 97, 53), torch.float16), ((33, 40), torch.float32),
+         ((6, 383), torch.float32)]
 
 
 @pytest.mark.parametrize("grid,dtype", CASES)
