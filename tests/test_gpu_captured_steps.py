@@ -1,7 +1,7 @@
 """Steps captured into a CUDA graph and replayed, against the same steps made by calls: whatever form the state had when
 they were captured (stored populations right after the first step, else the source form), and whatever was done to it
 between the replays: more steps, a read of f, a checkpoint restored, the fused kernel, the autotuner, new initial fields.
-Batches of larger grids likewise."""
+Batches of larger grids likewise, and captured read-outs of f and g."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -118,6 +118,28 @@ def test_replays_after_new_initial_fields(grid, dtype):
     for s in (a, b):
         s.run(3)
     _same(a, b)
+
+
+@pytest.mark.parametrize("grid,dtype", [((14, 17, 18), torch.float32), ((101, 97, 53), torch.float32),
+                                        ((101, 97, 53), torch.float16), ((1831, 383), torch.float32)])
+def test_replays_of_a_read_out(grid, dtype):
+    a, b = _solver(grid, dtype), _solver(grid, dtype)
+    for s in (a, b):
+        s.run(3)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        f, pg = a.f, a.g
+    for stored in (False, True, False):
+        if stored:
+            a.load_state_dict(a.state_dict())  # populations from here to the next step
+        else:
+            for s in (a, b):
+                s.run(2)
+        f.fill_(float("nan"))
+        g.replay()
+        assert _equal(f, b.f) and _equal(pg, b.g)
+        assert bool(torch.isfinite(f).all())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
